@@ -61,6 +61,8 @@ struct Level {
     LevelDesc L;
     double* ddw64 = nullptr;
     float* ddw32 = nullptr;
+    double* div64 = nullptr;   // divergence of general moduli (null: not used, or no memory for it)
+    float* div32 = nullptr;
     double* diag64 = nullptr;
     double* dinv64 = nullptr;
     float* dinv32 = nullptr;
@@ -357,6 +359,19 @@ agb_status check_level(agb_op op, int level)
     return AGB_OK;
 }
 
+// A level's divergence field, made from its moduli.  A field that finds no
+// memory is left out: the rows then read the moduli of the neighbours.
+template <typename T> void make_div(agb_op op, Level& lv, const T* ddw, T** div)
+{
+    if (!stencil_uses_div(op->sym, sizeof(T) == 4, lv.L)) return;
+    if (!*div && op->alloc(div, 18 * (size_t)lv.L.S) != AGB_OK) {
+        cudaGetLastError();
+        *div = nullptr;
+        return;
+    }
+    launch_div_moduli<T>(op->st, lv.L, ddw, *div);
+}
+
 agb_status ensure_f32(agb_op op)
 {
     if (op->f32_ready) return AGB_OK;
@@ -373,6 +388,7 @@ agb_status ensure_f32(agb_op op)
         }
         launch_convert<float, double>(op->st, lv.L, op->nc, lv.ddw64, lv.ddw32, 1.0);
         launch_recip<float>(op->st, lv.L, 3, lv.diag64, lv.dinv32);
+        make_div<float>(op, lv, lv.ddw32, &lv.div32);
     }
     // prepare() assembled the dense coarsest operator; the FP32 cycles take its inverse
     if (op->bottom_inv32)
@@ -415,13 +431,13 @@ agb_status prepare_mixed(agb_op op)
         launch_average_ddw<float>(op->st, op->lev[l - 1].L, op->lev[l].L, op->lev[l - 1].ddw32, op->lev[l].ddw32,
                                   op->nc);
     for (auto& lv : op->lev) {
-        launch_diagonal<float>(op->st, op->sym, lv.L, op->bc, lv.ddw32, lv.dinv32);
-        launch_recip_inplace(op->st, lv.L, 3, lv.dinv32);
+        launch_diagonal<float, float>(op->st, op->sym, lv.L, op->bc, lv.ddw32, nullptr, lv.dinv32);
+        make_div<float>(op, lv, lv.ddw32, &lv.div32);
     }
+    make_div<double>(op, op->lev[0], op->lev[0].ddw64, &op->lev[0].div64);   // the FP64 residuals
     Level& bl = op->lev[nl - 1];
     if (nl > 1) launch_convert<double, float>(op->st, bl.L, op->nc, bl.ddw32, bl.ddw64, 1.0);
-    launch_diagonal<double>(op->st, op->sym, bl.L, op->bc, bl.ddw64, bl.diag64);
-    launch_recip<double>(op->st, bl.L, 3, bl.diag64, bl.dinv64);
+    launch_diagonal<double, double>(op->st, op->sym, bl.L, op->bc, bl.ddw64, bl.diag64, bl.dinv64);
     if (op->bottom_A)
         launch_bottom_assemble(op->st, op->sym, bl.L, op->bc, op->uniform, bl.ddw64, op->bottom_A);
     if (op->bottom_inv32) launch_bottom_invert(op->st, bl.L, op->bottom_A, op->bottom_inv32, op->bottom_inv_ok);
@@ -448,8 +464,8 @@ agb_status prepare(agb_op op)
     for (size_t l = 1; l < op->lev.size(); l++)
         launch_average_ddw<double>(op->st, op->lev[l - 1].L, op->lev[l].L, op->lev[l - 1].ddw64, op->lev[l].ddw64, op->nc);
     for (auto& lv : op->lev) {
-        launch_diagonal<double>(op->st, op->sym, lv.L, op->bc, lv.ddw64, lv.diag64);
-        launch_recip<double>(op->st, lv.L, 3, lv.diag64, lv.dinv64);
+        launch_diagonal<double, double>(op->st, op->sym, lv.L, op->bc, lv.ddw64, lv.diag64, lv.dinv64);
+        make_div<double>(op, lv, lv.ddw64, &lv.div64);
     }
     if (op->bottom_A)
         launch_bottom_assemble(op->st, op->sym, op->lev.back().L, op->bc, op->uniform, op->lev.back().ddw64,
@@ -472,6 +488,7 @@ template <> struct Arr<double> {
     static double* tmp(Level& l) { return l.tmp64; }
     static const double* ddw(Level& l) { return l.ddw64; }
     static const double* dinv(Level& l) { return l.dinv64; }
+    static const double* div(Level& l) { return l.div64; }
     static void swap_res_rescor(Level& l) { std::swap(l.res64, l.rescor64); }
     static void swap_cor_hold(Level& l) { std::swap(l.cor64, l.hold64); }
 };
@@ -483,6 +500,7 @@ template <> struct Arr<float> {
     static float* tmp(Level& l) { return l.tmp32; }
     static const float* ddw(Level& l) { return l.ddw32; }
     static const float* dinv(Level& l) { return l.dinv32; }
+    static const float* div(Level& l) { return l.div32; }
     static void swap_res_rescor(Level& l) { std::swap(l.res32, l.rescor32); }
     static void swap_cor_hold(Level& l) { std::swap(l.cor32, l.hold32); }
 };
@@ -497,9 +515,9 @@ template <typename T> struct Engine {
     void sweep2(int l, T* x, const T* b)
     {
         Level& v = lv(l);
-        launch_stencil<T>(op->st, op->sym, MODE_JACOBI, v.L, op->bc, op->uniform, A::ddw(v), x, b, A::dinv(v),
+        launch_stencil<T>(op->st, op->sym, MODE_JACOBI, v.L, op->bc, op->uniform, A::ddw(v), A::div(v), x, b, A::dinv(v),
                           A::tmp(v), (T)op->omega, nullptr);
-        launch_stencil<T>(op->st, op->sym, MODE_JACOBI, v.L, op->bc, op->uniform, A::ddw(v), A::tmp(v), b,
+        launch_stencil<T>(op->st, op->sym, MODE_JACOBI, v.L, op->bc, op->uniform, A::ddw(v), A::div(v), A::tmp(v), b,
                           A::dinv(v), x, (T)op->omega, nullptr);
     }
     void smooth(int l, T* x, const T* b, int nsmooth)
@@ -516,14 +534,14 @@ template <typename T> struct Engine {
             return;
         }
         launch_jacobi_zero<T>(op->st, v.L, 3, A::tmp(v), b, A::dinv(v), (T)op->omega);
-        launch_stencil<T>(op->st, op->sym, MODE_JACOBI, v.L, op->bc, op->uniform, A::ddw(v), A::tmp(v), b,
+        launch_stencil<T>(op->st, op->sym, MODE_JACOBI, v.L, op->bc, op->uniform, A::ddw(v), A::div(v), A::tmp(v), b,
                           A::dinv(v), x, (T)op->omega, nullptr);
         for (int s = 1; s < nsmooth; s++) sweep2(l, x, b);
     }
     void residual(int l, const T* x, const T* b, T* r, void* slot)
     {
         Level& v = lv(l);
-        launch_stencil<T>(op->st, op->sym, MODE_RESID, v.L, op->bc, op->uniform, A::ddw(v), x, b, nullptr, r, (T)0,
+        launch_stencil<T>(op->st, op->sym, MODE_RESID, v.L, op->bc, op->uniform, A::ddw(v), A::div(v), x, b, nullptr, r, (T)0,
                           slot);
     }
     // The solve's fine-level residual and its max norm (into a zeroed slot).
@@ -859,7 +877,7 @@ agb_status inner_gcr32(agb_solver s, double inner_tol, double* inorm_out, int* c
         float* z = s->kZ[k];
         float* w = s->kW[k];
         CK(cudaMemcpyAsync(z, v0.cor32, bytes, cudaMemcpyDeviceToDevice, st));
-        launch_stencil<float>(st, op->sym, MODE_APPLY, L, op->bc, op->uniform, v0.ddw32, z, nullptr, nullptr, w, 0.0f,
+        launch_stencil<float>(st, op->sym, MODE_APPLY, L, op->bc, op->uniform, v0.ddw32, v0.div32, z, nullptr, nullptr, w, 0.0f,
                               nullptr);
         if (sing) launch_remove_mean<float>(st, L, w, op->d_slots + 11);
         CK(cudaMemsetAsync(s->kdots, 0, sizeof(double) * (GCR_MAX + 2), st));
@@ -894,7 +912,7 @@ agb_status inner_gcr32(agb_solver s, double inner_tol, double* inorm_out, int* c
             float* zl = s->kZ[k];
             float* wl = s->kW[k];
             TRY(learned_direction(s->net, st, op->sym, L, s->kr, v0.ddw32, zl));
-            launch_stencil<float>(st, op->sym, MODE_APPLY, L, op->bc, op->uniform, v0.ddw32, zl, nullptr, nullptr, wl,
+            launch_stencil<float>(st, op->sym, MODE_APPLY, L, op->bc, op->uniform, v0.ddw32, v0.div32, zl, nullptr, nullptr, wl,
                                   0.0f, nullptr);
             CK(cudaMemsetAsync(s->kdots, 0, sizeof(double) * (GCR_MAX + 4), st));
             if (k > 0) {
@@ -1223,7 +1241,7 @@ agb_status agb_op_fapply(agb_op op, int level, double* f, const double* u, int m
     TRY(prepare(op));
     Level& v = op->lev[level];
     TRY((upload<double, double>(op, v.L, 3, false, u, mem, v.hold64)));
-    launch_stencil<double>(op->st, op->sym, MODE_APPLY, v.L, op->bc, op->uniform, v.ddw64, v.hold64, nullptr, nullptr,
+    launch_stencil<double>(op->st, op->sym, MODE_APPLY, v.L, op->bc, op->uniform, v.ddw64, v.div64, v.hold64, nullptr, nullptr,
                            v.tmp64, 0.0, nullptr);
     CK(cudaGetLastError());
     TRY((download<double, double>(op, v.L, 3, false, v.tmp64, f, mem)));
@@ -1238,7 +1256,7 @@ agb_status agb_op_fapply_f32(agb_op op, int level, float* f, const float* u, int
     TRY(ensure_f32(op));
     Level& v = op->lev[level];
     TRY((upload<float, float>(op, v.L, 3, false, u, mem, v.hold32)));
-    launch_stencil<float>(op->st, op->sym, MODE_APPLY, v.L, op->bc, op->uniform, v.ddw32, v.hold32, nullptr, nullptr,
+    launch_stencil<float>(op->st, op->sym, MODE_APPLY, v.L, op->bc, op->uniform, v.ddw32, v.div32, v.hold32, nullptr, nullptr,
                           v.tmp32, 0.0f, nullptr);
     CK(cudaGetLastError());
     TRY((download<float, float>(op, v.L, 3, false, v.tmp32, f, mem)));
@@ -1298,7 +1316,7 @@ agb_status agb_op_residual(agb_op op, int level, double* r, const double* x, con
     Level& v = op->lev[level];
     TRY((upload<double, double>(op, v.L, 3, false, x, mem, v.hold64)));
     TRY((upload<double, double>(op, v.L, 3, false, b, mem, v.rescor64)));
-    launch_stencil<double>(op->st, op->sym, MODE_RESID, v.L, op->bc, op->uniform, v.ddw64, v.hold64, v.rescor64,
+    launch_stencil<double>(op->st, op->sym, MODE_RESID, v.L, op->bc, op->uniform, v.ddw64, v.div64, v.hold64, v.rescor64,
                            nullptr, v.tmp64, 0.0, nullptr);
     CK(cudaGetLastError());
     TRY((download<double, double>(op, v.L, 3, false, v.tmp64, r, mem)));
@@ -1656,10 +1674,10 @@ agb_status agb_op_time_sweep(agb_op op, int level, int precision, int mode, int 
     if (precision == AGB_PREC_MIXED) TRY(ensure_f32(op));
     auto one = [&]() {
         if (precision == AGB_PREC_MIXED)
-            launch_stencil<float>(op->st, op->sym, mode, v.L, op->bc, op->uniform, v.ddw32, v.cor32, v.res32, v.dinv32,
+            launch_stencil<float>(op->st, op->sym, mode, v.L, op->bc, op->uniform, v.ddw32, v.div32, v.cor32, v.res32, v.dinv32,
                                   v.tmp32, (float)op->omega, mode == MODE_RESID ? (void*)(op->d_slots + 3) : nullptr);
         else
-            launch_stencil<double>(op->st, op->sym, mode, v.L, op->bc, op->uniform, v.ddw64, v.cor64, v.res64, v.dinv64,
+            launch_stencil<double>(op->st, op->sym, mode, v.L, op->bc, op->uniform, v.ddw64, v.div64, v.cor64, v.res64, v.dinv64,
                                    v.tmp64, op->omega, mode == MODE_RESID ? (void*)(op->d_slots + 3) : nullptr);
     };
     one();

@@ -189,9 +189,17 @@ bool batch_shape_ok(int shape, int sym, const int per[3]);
 // Launchers (kernels_*.cu).  All work is queued on `st`; none synchronizes.
 template <typename T>
 void launch_stencil(cudaStream_t st, int sym, int mode, const LevelDesc& L, const BCTable& bc, bool uniform,
-                    const T* ddw, const T* x, const T* b, const T* diag, T* out, T omega, void* norm_slot);
+                    const T* ddw, const T* div, const T* x, const T* b, const T* diag, T* out, T omega,
+                    void* norm_slot);
+// Divergence of general moduli (18 planes, kernels_stencil.cu) for the levels
+// whose rows read it; a null `div` makes launch_stencil read the moduli of the
+// neighbours instead.
+bool stencil_uses_div(int sym, bool fp32, const LevelDesc& L);
 template <typename T>
-void launch_diagonal(cudaStream_t st, int sym, const LevelDesc& L, const BCTable& bc, const T* ddw, T* diag);
+void launch_div_moduli(cudaStream_t st, const LevelDesc& L, const T* ddw, T* div);
+// diag = D (may be null), dinv = 1/D
+template <typename T, typename TI>
+void launch_diagonal(cudaStream_t st, int sym, const LevelDesc& L, const BCTable& bc, const T* ddw, T* diag, TI* dinv);
 template <typename T>
 void launch_restriction(cudaStream_t st, const LevelDesc& Lf, const LevelDesc& Lc, const T* fine, T* crse,
                         int ncomp);
@@ -224,8 +232,6 @@ template <typename TD, typename TS>
 void launch_export(cudaStream_t st, const LevelDesc& L, int ncomp, const TS* src, TD* dst, bool aos, int k0, int kc,
                    bool chunk);
 void launch_axpy_mixed(cudaStream_t st, const LevelDesc& L, int ncomp, double* y, const float* x, double a);
-// d <- 1/d (FP32, in place; zeros stay zero)
-void launch_recip_inplace(cudaStream_t st, const LevelDesc& L, int ncomp, float* d);
 // Inner FP32 GCR (kernels_transfer.cu): up to GCR_MAX stored directions.
 constexpr int GCR_MAX = 16;
 struct GcrVecs {

@@ -70,7 +70,7 @@ template <typename T> __device__ __forceinline__ Geo<T> geo_of(const BProb& p)
         g.h2[d] = (T)p.h2[d];
         g.hm[d] = (T)p.hm[d];
     }
-    g.cube = 0;   // the batched kernels keep the general row form
+    g.cube = p.h1[0] == p.h1[1] && p.h1[1] == p.h1[2];
     return g;
 }
 
@@ -624,15 +624,22 @@ __global__ void __launch_bounds__(256) k_batch_diag(const BProb* __restrict__ pr
             mx[d] = !L.per[d] && pos[d] == L.n[d];
         }
         const long long p = L.idx(i, j, k);
-        double c[NCoef<SYM>::value];
-        for (int m = 0; m < NCoef<SYM>::value; m++) c[m] = ddw[P.co + m * L.S + p];
-        const DiagGeo<double> dg = make_diag_geo<double>(L);
+        DiagGeo<double> dg;
+        for (int d = 0; d < 3; d++) {
+            dg.h2m[d] = -2.0 * P.h2[d];
+            dg.i1[d] = P.i1[d];
+        }
+        auto cf = [&](int m) { return __ldg(ddw + P.co + m * L.S + p); };
+        double dd[3];
+        if (mn[0] | mx[0] | mn[1] | mx[1] | mn[2] | mx[2]) diag_boundary<double, SYM>(cf, dg, bc, mn, mx, dd);
+        else diag_interior<double, SYM>(cf, dg, dd);
+#pragma unroll
         for (int q = 0; q < 3; q++) {
-            const double d = diag_entry<double, SYM>(c, L, dg, bc, mn, mx, q);
+            const double d = dd[q], inv = d != 0.0 ? 1.0 / d : 0.0;
             const long long o = P.vo + q * L.S + p;
             diag[o] = d;
-            dinv64[o] = d != 0.0 ? 1.0 / d : 0.0;
-            if (dinv32) dinv32[o] = d != 0.0 ? (float)(1.0 / d) : 0.0f;
+            dinv64[o] = inv;
+            if (dinv32) dinv32[o] = (float)inv;
         }
     }
 }

@@ -277,13 +277,6 @@ __global__ void k_axpy_mixed(long long n, double* __restrict__ y, const float* _
         y[e] += a * (double)x[e];
 }
 
-// d <- 1/d in place (0 stays 0: padding)
-__global__ void k_recip_inplace(long long n, float* __restrict__ d)
-{
-    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x)
-        d[e] = d[e] != 0.0f ? 1.0f / d[e] : 0.0f;
-}
-
 template <typename TD>
 __global__ void k_recip(long long n, const double* __restrict__ d, TD* __restrict__ r)
 {
@@ -590,13 +583,6 @@ void launch_gcr_step(cudaStream_t st, long long n, const double* dots, float* w,
     count_launch();
 }
 
-void launch_recip_inplace(cudaStream_t st, const LevelDesc& L, int ncomp, float* d)
-{
-    const long long n = (long long)ncomp * L.S;
-    k_recip_inplace<<<blocks_1d(n), 256, 0, st>>>(n, d);
-    count_launch();
-}
-
 void launch_axpy_mixed(cudaStream_t st, const LevelDesc& L, int ncomp, double* y, const float* x, double a)
 {
     const long long n = (long long)ncomp * L.S;
@@ -618,7 +604,6 @@ void launch_recip(cudaStream_t st, const LevelDesc& L, int ncomp, const double* 
     template void launch_zero<T>(cudaStream_t, const LevelDesc&, int, T*);                                   \
     template void launch_jacobi_zero<T>(cudaStream_t, const LevelDesc&, int, T*, const T*, const T*, T);     \
     template void launch_norm_inf<T>(cudaStream_t, const LevelDesc&, int, const T*, void*);                  \
-    template void launch_recip<T>(cudaStream_t, const LevelDesc&, int, const double*, T*);                   \
     template void launch_remove_mean<T>(cudaStream_t, const LevelDesc&, T*, double*, void*);                 \
     template void launch_import<T, double>(cudaStream_t, const LevelDesc&, int, const double*, T*, bool, int, int, bool); \
     template void launch_import<T, float>(cudaStream_t, const LevelDesc&, int, const float*, T*, bool, int, int, bool);   \
@@ -627,6 +612,7 @@ void launch_recip(cudaStream_t st, const LevelDesc& L, int ncomp, const double* 
 INST(double)
 INST(float)
 #undef INST
+template void launch_recip<float>(cudaStream_t, const LevelDesc&, int, const double*, float*);
 template void launch_convert<float, double>(cudaStream_t, const LevelDesc&, int, const double*, float*, double);
 template void launch_convert<double, float>(cudaStream_t, const LevelDesc&, int, const float*, double*, double);
 template void launch_convert<double, double>(cudaStream_t, const LevelDesc&, int, const double*, double*, double);
