@@ -123,8 +123,11 @@ struct agb_op_s {
     double* h_slots = nullptr;   // pinned mirror
     double* bottom_work = nullptr;
     double* bottom_A = nullptr;   // dense coarsest-level operator (small bottom levels)
-    float* bottom_inv32 = nullptr;   // its inverse for the FP32 cycles (exact coarsest solve)
-    int* bottom_inv_ok = nullptr;    // device flag: the inverse exists
+    bool bottom_exact = false;    // the cycles take the exact coarsest solve (AGB_BOTTOM_EXACT)
+    double* bottom_inv64 = nullptr;   // its inverse for the FP64 cycles
+    float* bottom_inv32 = nullptr;    // and for the FP32 cycles
+    double* bottom_iwork = nullptr;   // work of the panel elimination
+    int* bottom_inv_ok = nullptr;     // device flag: the inverse exists
     int* d_ret = nullptr;
     char* stage = nullptr;       // bounded staging buffer for pageable host copies
     size_t stage_bytes = 0;
@@ -158,6 +161,7 @@ struct agb_solver_s {
     long long replayed = 0;                  // kernels executed through graph replays
     // inner FP32 GCR of the mixed solve (params.krylov > 0): directions, their
     // images, the inner residual, device scalars, the preconditioner's graph
+    bool exact_bottom = false;   // this solve's cycles take the inverse (set by prepare_bottom, the same on every solve)
     std::vector<float*> kZ, kW;
     float* kr = nullptr;
     double* kdots = nullptr;
@@ -390,9 +394,6 @@ agb_status ensure_f32(agb_op op)
         launch_recip<float>(op->st, lv.L, 3, lv.diag64, lv.dinv32);
         make_div<float>(op, lv, lv.ddw32, &lv.div32);
     }
-    // prepare() assembled the dense coarsest operator; the FP32 cycles take its inverse
-    if (op->bottom_inv32)
-        launch_bottom_invert(op->st, op->lev.back().L, op->bottom_A, op->bottom_inv32, op->bottom_inv_ok);
     CK(cudaGetLastError());
     op->f32_ready = true;
     return AGB_OK;
@@ -438,12 +439,44 @@ agb_status prepare_mixed(agb_op op)
     Level& bl = op->lev[nl - 1];
     if (nl > 1) launch_convert<double, float>(op->st, bl.L, op->nc, bl.ddw32, bl.ddw64, 1.0);
     launch_diagonal<double, double>(op->st, op->sym, bl.L, op->bc, bl.ddw64, bl.diag64, bl.dinv64);
-    if (op->bottom_A)
+    if (bottom_dense_fits(bl.L) && op->bottom_A)
         launch_bottom_assemble(op->st, op->sym, bl.L, op->bc, op->uniform, bl.ddw64, op->bottom_A);
-    if (op->bottom_inv32) launch_bottom_invert(op->st, bl.L, op->bottom_A, op->bottom_inv32, op->bottom_inv_ok);
     CK(cudaGetLastError());
     op->prepared = false;
     op->f32_ready = true;
+    return AGB_OK;
+}
+
+// The inverse of the coarsest operator for the solver's cycles, made on every
+// solve from the operator that prepare() or prepare_mixed() assembled (a level
+// above the dense BiCGStab's size is assembled here).  Buffers that find no
+// memory leave the inverse out, and the cycles keep the BiCGStab bottom.
+// An FP64 solve that asks for a fixed number of iterations, or whose box has
+// one level only (the bottom solve to bottom_tol is then the whole cycle), keeps
+// MLMG's BiCGStab iterates.
+agb_status prepare_bottom(agb_solver s, bool fp32)
+{
+    agb_op op = s->op;
+    Level& bl = op->lev.back();
+    s->exact_bottom = false;
+    if (!op->bottom_exact || !bottom_exact_fits(bl.L)) return AGB_OK;
+    if (!fp32 && s->p.fixed_iter > 0) return AGB_OK;
+    if (op->lev.size() == 1 && !(fp32 && bottom_dense_fits(bl.L))) return AGB_OK;
+    const size_t n2 = bottom_dense_bytes(bl.L) / sizeof(double), nw = bottom_invert_work_bytes(bl.L) / sizeof(double);
+    const bool dense = bottom_dense_fits(bl.L);
+    if ((!op->bottom_A && op->alloc(&op->bottom_A, n2) != AGB_OK) ||
+        (!op->bottom_iwork && nw && op->alloc(&op->bottom_iwork, nw + 1) != AGB_OK) ||
+        (!op->bottom_inv_ok && op->alloc(&op->bottom_inv_ok, 1) != AGB_OK) ||
+        (fp32 && !op->bottom_inv32 && op->alloc(&op->bottom_inv32, n2) != AGB_OK) ||
+        (!fp32 && !op->bottom_inv64 && op->alloc(&op->bottom_inv64, n2) != AGB_OK)) {
+        cudaGetLastError();
+        return AGB_OK;
+    }
+    if (!dense) launch_bottom_assemble(op->st, op->sym, bl.L, op->bc, op->uniform, bl.ddw64, op->bottom_A);
+    launch_bottom_invert(op->st, bl.L, op->bottom_A, fp32 ? nullptr : op->bottom_inv64,
+                         fp32 ? op->bottom_inv32 : nullptr, op->bottom_iwork, op->bottom_inv_ok);
+    CK(cudaGetLastError());
+    s->exact_bottom = true;
     return AGB_OK;
 }
 
@@ -452,7 +485,9 @@ agb_status prepare_for_solve(agb_solver s)
 {
     agb_op op = s->op;
     op->prepared = false;
-    return s->p.precision == AGB_PREC_MIXED ? prepare_mixed(op) : prepare(op);
+    const bool mixed = s->p.precision == AGB_PREC_MIXED;
+    TRY(mixed ? prepare_mixed(op) : prepare(op));
+    return prepare_bottom(s, mixed);
 }
 
 // averageDownCoeffs + Diagonal(true) for every level (Operator.cpp:253-260)
@@ -467,7 +502,7 @@ agb_status prepare(agb_op op)
         launch_diagonal<double, double>(op->st, op->sym, lv.L, op->bc, lv.ddw64, lv.diag64, lv.dinv64);
         make_div<double>(op, lv, lv.ddw64, &lv.div64);
     }
-    if (op->bottom_A)
+    if (bottom_dense_fits(op->lev.back().L) && op->bottom_A)
         launch_bottom_assemble(op->st, op->sym, op->lev.back().L, op->bc, op->uniform, op->lev.back().ddw64,
                                op->bottom_A);
     CK(cudaGetLastError());
@@ -489,6 +524,7 @@ template <> struct Arr<double> {
     static const double* ddw(Level& l) { return l.ddw64; }
     static const double* dinv(Level& l) { return l.dinv64; }
     static const double* div(Level& l) { return l.div64; }
+    static const double* inv(agb_op op) { return op->bottom_inv64; }
     static void swap_res_rescor(Level& l) { std::swap(l.res64, l.rescor64); }
     static void swap_cor_hold(Level& l) { std::swap(l.cor64, l.hold64); }
 };
@@ -501,6 +537,7 @@ template <> struct Arr<float> {
     static const float* ddw(Level& l) { return l.ddw32; }
     static const float* dinv(Level& l) { return l.dinv32; }
     static const float* div(Level& l) { return l.div32; }
+    static const float* inv(agb_op op) { return op->bottom_inv32; }
     static void swap_res_rescor(Level& l) { std::swap(l.res32, l.rescor32); }
     static void swap_cor_hold(Level& l) { std::swap(l.cor32, l.hold32); }
 };
@@ -508,6 +545,7 @@ template <> struct Arr<float> {
 template <typename T> struct Engine {
     agb_op op;
     const agb_solver_params& p;
+    bool exact_bottom = false;
     typedef Arr<T> A;
     Level& lv(int l) { return op->lev[l]; }
     int bot() const { return (int)op->lev.size() - 1; }
@@ -561,19 +599,16 @@ template <typename T> struct Engine {
     void bottom()
     {
         Level& v = lv(bot());
-        if (op->bottom_A) {
-            // the FP32 cycles of the mixed solve take the exact coarsest solve
-            // when prepare_mixed made the inverse; the FP64 cycles keep MLMG's
-            // BiCGStab bottom
-            const bool exact = sizeof(T) == 4 && op->bottom_inv32 && op->f32_ready;
+        const T* inv = exact_bottom ? A::inv(op) : nullptr;
+        if (bottom_dense_fits(v.L) && op->bottom_A) {
             launch_bottom_dense<T>(op->st, v.L, op->bottom_A, v.diag64, A::cor(v), A::res(v), p.bottom_max_iter,
                                    p.bottom_tol_rel, p.bottom_tol_abs, op->d_ret, p.bottom_smooth, p.final_smooth,
-                                   op->omega, exact ? op->bottom_inv32 : nullptr, exact ? op->bottom_inv_ok : nullptr);
+                                   op->omega, inv, op->bottom_inv_ok);
             return;
         }
         launch_bottom<T>(op->st, op->sym, v.L, op->bc, op->uniform, v.ddw64, v.diag64, A::cor(v), A::res(v),
                          op->bottom_work, p.bottom_max_iter, p.bottom_tol_rel, p.bottom_tol_abs, op->d_ret,
-                         p.bottom_smooth, p.final_smooth, op->omega);
+                         p.bottom_smooth, p.final_smooth, op->omega, inv, op->bottom_inv_ok);
     }
     // MLMG::mgVcycle(amrlev = 0, mglev_top)
     void vcycle(int top)
@@ -643,7 +678,7 @@ double slot_as_float(const double* slots, int i)
 void iter64_body(agb_solver s, int iter)
 {
     agb_op op = s->op;
-    Engine<double> E{op, s->p};
+    Engine<double> E{op, s->p, s->exact_bottom};
     Level& v0 = op->lev[0];
     E.cycle(iter);
     launch_axpy<double>(op->st, v0.L, 3, s->x64, v0.cor64, 1.0);
@@ -656,7 +691,7 @@ void iter64_body(agb_solver s, int iter)
 void iter32_body(agb_solver s, int iter)
 {
     agb_op op = s->op;
-    Engine<float> E{op, s->p};
+    Engine<float> E{op, s->p, s->exact_bottom};
     Level& v0 = op->lev[0];
     E.cycle(iter);
     launch_axpy<float>(op->st, v0.L, 3, s->sol32, v0.cor32, 1.0f);
@@ -735,7 +770,7 @@ agb_status run_iter32(agb_solver s, int iter)
 agb_status residual64(agb_solver s, double* norm)
 {
     agb_op op = s->op;
-    Engine<double> E{op, s->p};
+    Engine<double> E{op, s->p, s->exact_bottom};
     Level& v0 = op->lev[0];
     CK(cudaMemsetAsync(op->d_slots, 0, sizeof(double), op->st));
     E.fine_residual(s->x64, s->b64, v0.res64, op->d_slots);
@@ -811,7 +846,7 @@ agb_status solve_plain(agb_solver s, double tol_rel, double tol_abs, agb_solve_r
 void precond32_body(agb_solver s)
 {
     agb_op op = s->op;
-    Engine<float> E{op, s->p};
+    Engine<float> E{op, s->p, s->exact_bottom};
     Level& v0 = op->lev[0];
     cudaMemcpyAsync(v0.res32, s->kr, sizeof(float) * 3 * (size_t)v0.L.S, cudaMemcpyDeviceToDevice, op->st);
     E.cycle(0);
@@ -1132,12 +1167,8 @@ agb_status agb_op_create(const int n_cells[3], const double dx[3], const int per
     if (bottom_dense_fits(op->lev.back().L) && use_dense_bottom()) {
         if ((s = op->alloc(&op->bottom_A, bottom_dense_bytes(op->lev.back().L) / sizeof(double))) != AGB_OK)
             return bail(s);
-        if (use_exact_bottom()) {
-            if ((s = op->alloc(&op->bottom_inv32, bottom_dense_bytes(op->lev.back().L) / sizeof(double))) != AGB_OK)
-                return bail(s);
-            if ((s = op->alloc(&op->bottom_inv_ok, 1)) != AGB_OK) return bail(s);
-        }
     }
+    op->bottom_exact = use_dense_bottom() && use_exact_bottom();
     op->stage_bytes = 64u << 20;
     if ((s = op->alloc(&op->stage, op->stage_bytes)) != AGB_OK) return bail(s);
     if (cudaMallocHost(&op->h_slots, 16 * sizeof(double)) != cudaSuccess)

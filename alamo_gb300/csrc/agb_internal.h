@@ -281,25 +281,30 @@ bool launch_stencil_tma(cudaStream_t st, int sym, int mode, const LevelDesc& L, 
 int tma_error_take();   // 1 if a TMA kernel's bounded wait ran out since the last call
 void init_tma_attributes();
 
-// Dense coarsest level (at most 128 unknowns): A assembled once per solve,
-// BiCGStab + smoothing of launch_bottom on it in one CTA; or, with inv and
-// *inv_ok set (launch_bottom_invert), the exact product cor = A^-1 res.
+// Coarsest level.  Up to 128 unknowns: A assembled once per solve, BiCGStab +
+// smoothing of launch_bottom on it in one CTA; up to 1536 unknowns also its
+// inverse (launch_bottom_invert): with inv and *inv_ok set, launch_bottom_dense
+// and launch_bottom are the exact product cor = A^-1 res.
 bool bottom_dense_fits(const LevelDesc& L);
+bool bottom_exact_fits(const LevelDesc& L);
 bool use_dense_bottom();
 bool use_exact_bottom();
 size_t bottom_dense_bytes(const LevelDesc& L);
+size_t bottom_invert_work_bytes(const LevelDesc& L);
 void launch_bottom_assemble(cudaStream_t st, int sym, const LevelDesc& L, const BCTable& bc, bool uniform,
                             const double* ddw64, double* A);
-void launch_bottom_invert(cudaStream_t st, const LevelDesc& L, const double* A, float* inv, int* ok);
+void launch_bottom_invert(cudaStream_t st, const LevelDesc& L, const double* A, double* inv64, float* inv32,
+                          double* work, int* ok);
 template <typename T>
 void launch_bottom_dense(cudaStream_t st, const LevelDesc& L, const double* A, const double* diag64, T* cor,
                          const T* res, int maxiter, double tol_rel, double tol_abs, int* ret_slot, int nub, int nuf,
-                         double omega, const float* inv = nullptr, const int* inv_ok = nullptr);
+                         double omega, const T* inv = nullptr, const int* inv_ok = nullptr);
 void init_bottom_attributes();
 template <typename T>
 void launch_bottom(cudaStream_t st, int sym, const LevelDesc& L, const BCTable& bc, bool uniform,
                    const double* ddw64, const double* diag64, T* cor, const T* res, double* work, int maxiter,
-                   double tol_rel, double tol_abs, int* ret_slot, int nub, int nuf, double omega);
+                   double tol_rel, double tol_abs, int* ret_slot, int nub, int nuf, double omega,
+                   const T* inv = nullptr, const int* inv_ok = nullptr);
 
 void launch_newton_rhs(cudaStream_t st, int sym, const LevelDesc& L, const BCTable& bc, const double* ddw,
                        const double* F0, const double* u, const double* b, double* rhs, double* dw_work);

@@ -1,6 +1,7 @@
-// kernels_bottom.cu -- coarsest-level solve in one CTA, FP64.
+// kernels_bottom.cu -- coarsest-level solve: the exact product with the inverse
+// of the level's operator where that is small enough, else BiCGStab in one CTA.
 //
-// Restates AMReX MLMG's bottom step as Alamo configures it
+// BiCGStab restates AMReX MLMG's bottom step as Alamo configures it
 // (Solver/Nonlocal/Linear.H:258 selects BiCGStab):
 //   cor = 0; BiCGStab on the diagonally scaled system (MLCGSolver::solve_bicgstab
 //   with Operator<Node>::normalize = divide by the diagonal, Operator.cpp:156-165);
@@ -144,15 +145,48 @@ __device__ void cta_mean3(const LevelDesc& L, const double* v, double* red, doub
              c_ < 3; c_++)                                                                               \
             for (long long q = c_ * L.S + L.idx(i_, j_, k_), once_ = 0; once_ < 1; once_++)
 
+// cor = A^-1 res with the inverse row-major: one row a warp, the right-hand
+// side in shared memory.  Every CTA of the grid takes its rows.
+template <typename T>
+__device__ __forceinline__ void exact_product(const LevelDesc& L, const T* __restrict__ inv, T* __restrict__ cor,
+                                              const T* __restrict__ res, T* __restrict__ xs, int* ret_slot)
+{
+    const int cnt = (int)L.count(), nu = 3 * cnt;
+    for (int q = threadIdx.x; q < nu; q += blockDim.x) xs[q] = __ldcg(res + dense_to_padded(L, q, cnt));
+    __syncthreads();
+    const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+    for (int row = blockIdx.x * nw + (threadIdx.x >> 5); row < nu; row += gridDim.x * nw) {
+        const T* a = inv + (long long)row * nu;
+        T y0 = 0, y1 = 0;
+        int j = lane;
+        for (; j + 32 < nu; j += 64) {
+            y0 += a[j] * xs[j];
+            y1 += a[j + 32] * xs[j + 32];
+        }
+        if (j < nu) y0 += a[j] * xs[j];
+        y0 += y1;
+        for (int o = 16; o > 0; o >>= 1) y0 += __shfl_xor_sync(0xffffffffu, y0, o);
+        if (lane == 0) cor[dense_to_padded(L, row, cnt)] = y0;
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0 && ret_slot) *ret_slot = 0;
+}
+
 template <typename T, int SYM>
 __global__ void __launch_bounds__(BOT_THREADS) k_bottom(LevelDesc L, BCTable bc, Geo<double> g, int uniform,
                                                         const double* __restrict__ ddw,
                                                         const double* __restrict__ diag, T* __restrict__ cor,
                                                         const T* __restrict__ res, double* __restrict__ work,
                                                         int maxiter, double eps_rel, double eps_abs, int nub,
-                                                        int nuf, double omega, int* ret_slot)
+                                                        int nuf, double omega, int* ret_slot,
+                                                        const T* __restrict__ inv, const int* __restrict__ inv_ok)
 {
     __shared__ double red[33];
+    if (inv && *inv_ok) {
+        extern __shared__ __align__(16) unsigned char bsm_raw[];
+        exact_product<T>(L, inv, cor, res, reinterpret_cast<T*>(bsm_raw), ret_slot);
+        return;
+    }
+    if (blockIdx.x) return;   // the BiCGStab solve is one CTA's
     const long long n3 = 3 * L.S, cnt = L.count();
     double *r = work, *rh = work + n3, *p = work + 2 * n3, *v = work + 3 * n3, *s = work + 4 * n3,
            *t = work + 5 * n3, *sol = work + 6 * n3, *b = work + 7 * n3;
@@ -304,7 +338,8 @@ __global__ void k_bottom_assemble(LevelDesc L, BCTable bc, Geo<double> g, int un
     acc.S = L.S;
     acc.base = L.idx(i, j, k);
     acc.comp = col / cnt;
-    acc.unit = L.idx(ce % L.nn[0], (ce / L.nn[0]) % L.nn[1], ce / (L.nn[0] * L.nn[1]));
+    const int cpos[3] = {ce % L.nn[0], (ce / L.nn[0]) % L.nn[1], ce / (L.nn[0] * L.nn[1])};
+    acc.unit = L.idx(cpos[0], cpos[1], cpos[2]);
     const long long st[3] = {1, (long long)L.P, (long long)L.P * L.nn[1]};
     const int pos[3] = {i, j, k};
     int mn[3], mx[3];
@@ -321,9 +356,16 @@ __global__ void k_bottom_assemble(LevelDesc L, BCTable bc, Geo<double> g, int un
             if (pos[d] == L.n[d] - 1) acc.o[d][2] = -st[d] * (L.n[d] - 1);
         }
     }
-    double f[3];
-    if (bnd) boundary_row<double, SYM>(acc, g, bc, mn, mx, f);
-    else interior_row<double, SYM>(acc, g, uniform != 0, f);
+    bool near = true;   // a row reaches the 26 neighbours (periodic images included) only
+    for (int d = 0; d < 3; d++) {
+        const int a = abs(cpos[d] - pos[d]);
+        near = near && (a <= 1 || (L.per[d] && a == L.n[d] - 1));
+    }
+    double f[3] = {0, 0, 0};
+    if (near) {
+        if (bnd) boundary_row<double, SYM>(acc, g, bc, mn, mx, f);
+        else interior_row<double, SYM>(acc, g, uniform != 0, f);
+    }
     for (int c = 0; c < 3; c++) A[(long long)col * nu + c * cnt + e] = f[c];
 }
 
@@ -333,39 +375,25 @@ template <typename R> __device__ __forceinline__ void dense_load(R* A, const dou
     for (int q = threadIdx.x; q < nu * nu; q += blockDim.x) A[q] = (R)Ag[q];
 }
 
-// With `inv` set and *inv_ok (an exact inverse exists, k_bottom_invert), the
-// bottom is the product cor = A^-1 res instead of the BiCGStab solve.
+// With `inv` set and *inv_ok (an exact inverse exists, launch_bottom_invert),
+// the bottom is the product cor = A^-1 res instead of the BiCGStab solve.
 template <typename T, typename R>
 __global__ void __launch_bounds__(DENSE_MAX) k_bottom_dense(LevelDesc L, const double* __restrict__ Ag,
                                                             const double* __restrict__ diag, T* __restrict__ cor,
                                                             const T* __restrict__ res, int maxiter, double eps_rel_d,
                                                             double eps_abs_d, int nub, int nuf, double omega_d,
-                                                            int* ret_slot, const float* __restrict__ inv,
+                                                            int* ret_slot, const T* __restrict__ inv,
                                                             const int* __restrict__ inv_ok)
 {
     pdl_entry();
     extern __shared__ __align__(16) unsigned char dsm_raw[];
     __shared__ R red[2 * 3 * 32];
-    const int cnt = (int)L.count(), nu = 3 * cnt;
+    const int nu = 3 * (int)L.count();
     if (inv && *inv_ok) {
-        float* xs = reinterpret_cast<float*>(dsm_raw);
-        const int q = threadIdx.x;
-        const long long pq = q < nu ? dense_to_padded(L, q, cnt) : 0;
-        if (q < nu) xs[q] = (float)__ldcg(res + pq);
-        __syncthreads();
-        if (q < nu) {
-            float y0 = 0.0f, y1 = 0.0f;
-            int j = 0;
-            for (; j + 1 < nu; j += 2) {
-                y0 = fmaf(inv[(long long)j * nu + q], xs[j], y0);
-                y1 = fmaf(inv[(long long)(j + 1) * nu + q], xs[j + 1], y1);
-            }
-            if (j < nu) y0 = fmaf(inv[(long long)j * nu + q], xs[j], y0);
-            cor[pq] = (T)(y0 + y1);
-        }
-        if (threadIdx.x == 0 && ret_slot) *ret_slot = 0;
+        exact_product<T>(L, inv, cor, res, reinterpret_cast<T*>(dsm_raw), ret_slot);
         return;
     }
+    if (blockIdx.x) return;   // the BiCGStab solve is one CTA's
     R* A = reinterpret_cast<R*>(dsm_raw);
     dense_load<R>(A, Ag, nu);
     __syncthreads();
@@ -376,16 +404,32 @@ __global__ void __launch_bounds__(DENSE_MAX) k_bottom_dense(LevelDesc L, const d
 bool bottom_dense_fits(const LevelDesc& L) { return 3 * L.count() <= DENSE_MAX; }
 
 // ---------------------------------------------------------------------------
-// Exact coarsest solve for the FP32 cycles of the mixed solve.  Once per solve
-// the dense operator (FP64, column-major) is inverted by Gauss-Jordan
-// elimination with partial pivoting in one CTA, the matrix in shared memory
-// (row-major), and stored in FP32 column-major (inv[j * nu + r] = A^-1(r, j))
-// so that thread r of the product reads a coalesced column per j.  A fully
-// periodic level (singular), or a pivot at or below 1e-13 of the largest
+// Exact coarsest solve.  Once per solve the dense operator (FP64,
+// column-major) is inverted by Gauss-Jordan elimination with partial pivoting
+// in FP64 and stored row-major in FP64 (FP64 cycles) and FP32 (FP32 cycles).  A
+// fully periodic level (singular), or a pivot at or below 1e-13 of the largest
 // |entry|, clears *ok and the cycles keep the BiCGStab bottom.
+//
+// BiCGStab runs in one CTA, whose SM has two FP64 lanes per clock and whose
+// reductions are barriers: 37 us (isotropic) to 248 us a call on 81 unknowns,
+// 2.7 ms on the 588 of a 6 x 6 x 3-cell level, six calls and more a cycle.
+// The product takes 4 to 6 us and the inversion is paid once per solve (0.3 ms
+// for 81 unknowns, a few ms for 588): the FP64 solve of a 65^3 polycrystal (81
+// unknowns) went from 176 to 113 ms, the mixed solve of a 96 x 96 x 48-cell
+// one (588) from 391 to 34 ms.  Above EXACT_MAX the inversion (cubic in the
+// unknowns) and its two copies of the matrix cost more than they save.
+//
+// Up to DENSE_MAX unknowns the matrix fits the shared memory of one CTA
+// (k_bottom_invert).  Up to EXACT_MAX it is eliminated eight columns at a
+// time: k_inv_panel (one CTA, a row or two of the panel in each thread's
+// registers) runs the eight steps with their row interchanges and leaves the
+// panel's transformation T; k_inv_update applies it to every other column,
+// new(r, c) = (r in panel ? 0 : old(perm r, c)) + sum_q T(r, q) old(perm(k + q), c),
+// from one copy of the matrix into another, so that its tiles are independent.
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(1024) k_bottom_invert(LevelDesc L, const double* __restrict__ Ag,
-                                                       float* __restrict__ inv, int* __restrict__ ok)
+                                                       double* __restrict__ inv64, float* __restrict__ inv32,
+                                                       int* __restrict__ ok)
 {
     extern __shared__ __align__(16) unsigned char inv_raw[];
     double* M = reinterpret_cast<double*>(inv_raw);   // nu x nu, row-major
@@ -479,10 +523,205 @@ __global__ void __launch_bounds__(1024) k_bottom_invert(LevelDesc L, const doubl
         __syncthreads();
     }
     for (int t = tid; t < nu * nu; t += nt) {
-        const int j = t / nu, r = t - j * nu;
-        inv[t] = (float)M[r * nu + j];
+        if (inv64) inv64[t] = M[t];
+        if (inv32) inv32[t] = (float)M[t];
     }
     if (tid == 0) *ok = 1;
+}
+
+constexpr int INV_NB = 8;           // panel width
+constexpr int EXACT_MAX = 1536;     // unknowns
+
+// M = A row-major, perm state reset; the largest |entry| into *amax (bits)
+__global__ void __launch_bounds__(256) k_inv_begin(int nu, const double* __restrict__ A, double* __restrict__ M,
+                                                   unsigned long long* amax)
+{
+    __shared__ double t[32][33];
+    const int x = threadIdx.x & 31, y = threadIdx.x >> 5;
+    const int r0 = blockIdx.x * 32, c0 = blockIdx.y * 32;
+    double a = 0;
+    for (int q = y; q < 32; q += 8)   // column c0 + q, rows r0 + x
+        if (c0 + q < nu && r0 + x < nu) {
+            const double v = A[(long long)(c0 + q) * nu + r0 + x];
+            t[q][x] = v;
+            a = fmax(a, fabs(v));
+        }
+    __syncthreads();
+    for (int q = y; q < 32; q += 8)
+        if (r0 + q < nu && c0 + x < nu) M[(long long)(r0 + q) * nu + c0 + x] = t[x][q];
+    for (int o = 16; o > 0; o >>= 1) a = fmax(a, __shfl_xor_sync(0xffffffffu, a, o));
+    if (x == 0) atomicMax(amax, (unsigned long long)__double_as_longlong(a));
+}
+
+// Gauss-Jordan on columns k .. k + w of M (w <= INV_NB): T (nu x INV_NB), the
+// source row of every row after the interchanges (perm), the pivots (piv).
+template <int INV_ROWS>   // rows a thread holds: blocks of 1024 (one row) or 768 (two) threads at most
+__global__ void __launch_bounds__(INV_ROWS == 1 ? 1024 : 768) k_inv_panel(int nu, int k, const double* __restrict__ M,
+                                                    double* __restrict__ T, int* __restrict__ perm,
+                                                    int* __restrict__ piv, const unsigned long long* amax, int* ok)
+{
+    __shared__ double best_s[32], prow[INV_NB + 1], srow[INV_NB];
+    __shared__ int row_s[32], src_s[2];
+    if (!*ok) return;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
+    const int w = min(INV_NB, nu - k);
+    const double tol = 1e-13 * __longlong_as_double((long long)*amax);
+    double a[INV_ROWS][INV_NB];
+    int src[INV_ROWS];
+#pragma unroll
+    for (int q = 0; q < INV_ROWS; q++) {
+        const int r = tid + q * blockDim.x;
+        src[q] = r;
+#pragma unroll
+        for (int c = 0; c < INV_NB; c++) a[q][c] = r < nu && c < w ? M[(long long)r * nu + k + c] : 0.0;
+    }
+#pragma unroll
+    for (int s = 0; s < INV_NB; s++) {
+        if (s >= w) break;
+        // pivot: the largest |a| of column s in rows >= k + s (ties to the lower row)
+        double best = -1.0;
+        int br = k + s;
+#pragma unroll
+        for (int q = 0; q < INV_ROWS; q++) {
+            const int r = tid + q * blockDim.x;
+            const double v = fabs(a[q][s]);
+            if (r >= k + s && r < nu && v > best) {
+                best = v;
+                br = r;
+            }
+        }
+        for (int o = 16; o > 0; o >>= 1) {
+            const double ob = __shfl_xor_sync(0xffffffffu, best, o);
+            const int orow = __shfl_xor_sync(0xffffffffu, br, o);
+            if (ob > best || (ob == best && orow < br)) {
+                best = ob;
+                br = orow;
+            }
+        }
+        if (lane == 0) {
+            best_s[warp] = best;
+            row_s[warp] = br;
+        }
+        __syncthreads();
+        best = lane < nw ? best_s[lane] : -1.0;
+        br = lane < nw ? row_s[lane] : nu;
+        for (int o = 16; o > 0; o >>= 1) {
+            const double ob = __shfl_xor_sync(0xffffffffu, best, o);
+            const int orow = __shfl_xor_sync(0xffffffffu, br, o);
+            if (ob > best || (ob == best && orow < br)) {
+                best = ob;
+                br = orow;
+            }
+        }
+        if (!(best > tol)) {   // uniform over the CTA
+            if (tid == 0) *ok = 0;
+            return;
+        }
+        const int pr = br;
+        // the owners publish the pivot row, scaled, and the row it changes places with
+#pragma unroll
+        for (int q = 0; q < INV_ROWS; q++) {
+            const int r = tid + q * blockDim.x;
+            if (r == pr) {
+                const double pinv = 1.0 / a[q][s];
+#pragma unroll
+                for (int c = 0; c < INV_NB; c++) prow[c] = (c == s ? 1.0 : a[q][c]) * pinv;
+                src_s[0] = src[q];
+                piv[k + s] = pr;
+            }
+            if (r == k + s) {
+#pragma unroll
+                for (int c = 0; c < INV_NB; c++) srow[c] = a[q][c];
+                src_s[1] = src[q];
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int q = 0; q < INV_ROWS; q++) {
+            const int r = tid + q * blockDim.x;
+            if (r == k + s) {
+#pragma unroll
+                for (int c = 0; c < INV_NB; c++) a[q][c] = prow[c];
+                src[q] = src_s[0];
+            } else {
+                if (r == pr) {
+#pragma unroll
+                    for (int c = 0; c < INV_NB; c++) a[q][c] = srow[c];
+                    src[q] = src_s[1];
+                }
+                const double f = a[q][s];
+#pragma unroll
+                for (int c = 0; c < INV_NB; c++) a[q][c] = (c == s ? 0.0 : a[q][c]) - f * prow[c];
+            }
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < INV_ROWS; q++) {
+        const int r = tid + q * blockDim.x;
+        if (r < nu) {
+            perm[r] = src[q];
+#pragma unroll
+            for (int c = 0; c < INV_NB; c++) T[(long long)r * INV_NB + c] = a[q][c];
+        }
+    }
+}
+
+__global__ void __launch_bounds__(256) k_inv_update(int nu, int k, const double* __restrict__ Mo,
+                                                    double* __restrict__ Mn, const double* __restrict__ T,
+                                                    const int* __restrict__ perm, const int* ok)
+{
+    __shared__ double t[32][INV_NB + 1], p[INV_NB][32];
+    if (!*ok) return;
+    const int x = threadIdx.x & 31, y = threadIdx.x >> 5;
+    const int r0 = blockIdx.y * 32, c = blockIdx.x * 32 + x;
+    const int w = min(INV_NB, nu - k);
+    if (r0 + (int)(threadIdx.x >> 3) < nu)
+        t[threadIdx.x >> 3][threadIdx.x & 7] = T[(long long)(r0 + (threadIdx.x >> 3)) * INV_NB + (threadIdx.x & 7)];
+    p[y][x] = y < w && c < nu ? Mo[(long long)perm[k + y] * nu + c] : 0.0;
+    __syncthreads();
+    if (c >= nu) return;
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        const int rl = y + 8 * q, r = r0 + rl;
+        if (r >= nu) continue;
+        double v;
+        if (c >= k && c < k + w) {
+            v = t[rl][c - k];
+        } else {
+            v = r >= k && r < k + w ? 0.0 : Mo[(long long)perm[r] * nu + c];
+#pragma unroll
+            for (int s = 0; s < INV_NB; s++) v += (s < w ? t[rl][s] : 0.0) * p[s][x];
+        }
+        Mn[(long long)r * nu + c] = v;
+    }
+}
+
+// Undo the row interchanges (swap columns k <-> piv[k], last first) on the way
+// into the row-major inverses.
+__global__ void __launch_bounds__(256) k_inv_end(int nu, const double* __restrict__ M, const int* __restrict__ piv,
+                                                 double* __restrict__ inv64, float* __restrict__ inv32, const int* ok)
+{
+    __shared__ int col[EXACT_MAX];
+    __shared__ int pv[EXACT_MAX];
+    if (!*ok) return;
+    for (int j = threadIdx.x; j < nu; j += blockDim.x) {
+        col[j] = j;
+        pv[j] = piv[j];
+    }
+    __syncthreads();
+    if (threadIdx.x == 0)
+        for (int j = nu - 1; j >= 0; j--) {
+            const int t = col[j];
+            col[j] = col[pv[j]];
+            col[pv[j]] = t;
+        }
+    __syncthreads();
+    for (int r = blockIdx.x; r < nu; r += gridDim.x)
+        for (int j = threadIdx.x; j < nu; j += blockDim.x) {
+            const double v = M[(long long)r * nu + col[j]];
+            if (inv64) inv64[(long long)r * nu + j] = v;
+            if (inv32) inv32[(long long)r * nu + j] = (float)v;
+        }
 }
 
 // Exact coarsest solve unless AGB_BOTTOM_EXACT=0 (read when an operator is created).
@@ -492,10 +731,47 @@ bool use_exact_bottom()
     return !(s && s[0] == '0');
 }
 
-void launch_bottom_invert(cudaStream_t st, const LevelDesc& L, const double* A, float* inv, int* ok)
+bool bottom_exact_fits(const LevelDesc& L) { return !L.singular() && 3 * L.count() <= EXACT_MAX; }
+
+// Work of the panel elimination: two copies of the matrix, T, perm, piv, amax.
+size_t bottom_invert_work_bytes(const LevelDesc& L)
 {
     const size_t nu = 3 * (size_t)L.count();
-    k_bottom_invert<<<1, 1024, nu * nu * sizeof(double), st>>>(L, A, inv, ok);
+    return bottom_dense_fits(L) ? 0 : (2 * nu * nu + nu * INV_NB + 1) * sizeof(double) + 2 * nu * sizeof(int);
+}
+
+// *ok = 1 and the inverses of A, or *ok = 0 (a kernel of the chain that finds
+// *ok cleared leaves at once).
+void launch_bottom_invert(cudaStream_t st, const LevelDesc& L, const double* A, double* inv64, float* inv32,
+                          double* work, int* ok)
+{
+    const int nu = 3 * (int)L.count();
+    if (bottom_dense_fits(L)) {
+        k_bottom_invert<<<1, 1024, (size_t)nu * nu * sizeof(double), st>>>(L, A, inv64, inv32, ok);
+        count_launch();
+        return;
+    }
+    const size_t n2 = (size_t)nu * nu;
+    double *M0 = work, *M1 = work + n2, *T = work + 2 * n2;
+    unsigned long long* amax = (unsigned long long*)(T + (size_t)nu * INV_NB);
+    int *perm = (int*)(amax + 1), *piv = perm + nu;
+    const dim3 tiles((nu + 31) / 32, (nu + 31) / 32);
+    const int rows = nu <= 1024 ? 1 : 2, threads = ((nu + rows - 1) / rows + 31) / 32 * 32;
+    cudaMemsetAsync(amax, 0, sizeof(*amax), st);
+    cudaMemsetAsync(ok, 1, sizeof(int), st);   // any value but 0
+    k_inv_begin<<<tiles, 256, 0, st>>>(nu, A, M0, amax);
+    count_launch();
+    for (int k = 0; k < nu; k += INV_NB) {
+        if (rows == 1) k_inv_panel<1><<<1, threads, 0, st>>>(nu, k, M0, T, perm, piv, amax, ok);
+        else k_inv_panel<2><<<1, threads, 0, st>>>(nu, k, M0, T, perm, piv, amax, ok);
+        k_inv_update<<<tiles, 256, 0, st>>>(nu, k, M0, M1, T, perm, ok);
+        count_launch();
+        count_launch();
+        double* t = M0;
+        M0 = M1;
+        M1 = t;
+    }
+    k_inv_end<<<64, 256, 0, st>>>(nu, M0, piv, inv64, inv32, ok);
     count_launch();
 }
 
@@ -529,11 +805,13 @@ void launch_bottom_assemble(cudaStream_t st, int sym, const LevelDesc& L, const 
 template <typename T>
 void launch_bottom_dense(cudaStream_t st, const LevelDesc& L, const double* A, const double* diag64, T* cor,
                          const T* res, int maxiter, double tol_rel, double tol_abs, int* ret_slot, int nub, int nuf,
-                         double omega, const float* inv, const int* inv_ok)
+                         double omega, const T* inv, const int* inv_ok)
 {
     const size_t nu = 3 * (size_t)L.count();
     const size_t smem = (nu * nu + nu) * sizeof(T);
-    pdl_launch(k_bottom_dense<T, T>, dim3(1), dim3(DENSE_MAX), smem, st, L, A, diag64, cor, res, maxiter, tol_rel,
+    // the exact product takes a row a warp; the BiCGStab solve the first CTA
+    const unsigned grid = inv ? (unsigned)((nu + DENSE_MAX / 32 - 1) / (DENSE_MAX / 32)) : 1u;
+    pdl_launch(k_bottom_dense<T, T>, dim3(grid), dim3(DENSE_MAX), smem, st, L, A, diag64, cor, res, maxiter, tol_rel,
                tol_abs, nub, nuf, omega, ret_slot, inv, inv_ok);
     count_launch();
 }
@@ -548,7 +826,7 @@ void init_bottom_attributes()
 }
 
 template void launch_bottom_dense<double>(cudaStream_t, const LevelDesc&, const double*, const double*, double*,
-                                          const double*, int, double, double, int*, int, int, double, const float*,
+                                          const double*, int, double, double, int*, int, int, double, const double*,
                                           const int*);
 template void launch_bottom_dense<float>(cudaStream_t, const LevelDesc&, const double*, const double*, float*,
                                          const float*, int, double, double, int*, int, int, double, const float*,
@@ -557,24 +835,29 @@ template void launch_bottom_dense<float>(cudaStream_t, const LevelDesc&, const d
 template <typename T>
 void launch_bottom(cudaStream_t st, int sym, const LevelDesc& L, const BCTable& bc, bool uniform, const double* ddw64,
                    const double* diag64, T* cor, const T* res, double* work, int maxiter, double tol_rel,
-                   double tol_abs, int* ret_slot, int nub, int nuf, double omega)
+                   double tol_abs, int* ret_slot, int nub, int nuf, double omega, const T* inv, const int* inv_ok)
 {
     const Geo<double> g = make_geo<double>(L);
+    const size_t nu = 3 * (size_t)L.count();
+    const unsigned grid = inv ? (unsigned)((nu + BOT_THREADS / 32 - 1) / (BOT_THREADS / 32)) : 1u;
+    const size_t smem = inv ? nu * sizeof(T) : 0;
     if (sym == SYM_ISO)
-        k_bottom<T, SYM_ISO><<<1, BOT_THREADS, 0, st>>>(L, bc, g, uniform ? 1 : 0, ddw64, diag64, cor, res, work,
-                                                        maxiter, tol_rel, tol_abs, nub, nuf, omega, ret_slot);
+        k_bottom<T, SYM_ISO><<<grid, BOT_THREADS, smem, st>>>(L, bc, g, uniform ? 1 : 0, ddw64, diag64, cor, res, work,
+                                                              maxiter, tol_rel, tol_abs, nub, nuf, omega, ret_slot,
+                                                              inv, inv_ok);
     else
-        k_bottom<T, SYM_MM><<<1, BOT_THREADS, 0, st>>>(L, bc, g, uniform ? 1 : 0, ddw64, diag64, cor, res, work,
-                                                       maxiter, tol_rel, tol_abs, nub, nuf, omega, ret_slot);
+        k_bottom<T, SYM_MM><<<grid, BOT_THREADS, smem, st>>>(L, bc, g, uniform ? 1 : 0, ddw64, diag64, cor, res, work,
+                                                             maxiter, tol_rel, tol_abs, nub, nuf, omega, ret_slot,
+                                                             inv, inv_ok);
     count_launch();
 }
 
 template void launch_bottom<double>(cudaStream_t, int, const LevelDesc&, const BCTable&, bool, const double*,
                                     const double*, double*, const double*, double*, int, double, double, int*, int,
-                                    int, double);
+                                    int, double, const double*, const int*);
 template void launch_bottom<float>(cudaStream_t, int, const LevelDesc&, const BCTable&, bool, const double*,
                                    const double*, float*, const float*, double*, int, double, double, int*, int, int,
-                                   double);
+                                   double, const float*, const int*);
 
 }  // namespace agb
 
