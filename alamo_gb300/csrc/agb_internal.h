@@ -259,6 +259,8 @@ agb_status learned_direction(agb_learned net, cudaStream_t st, int sym, const Le
                              const float* ddw32, float* z);
 agb_status learned_features(cudaStream_t st, int sym, const LevelDesc& L, const float* r, const float* ddw32,
                             void* feat, double* acc);
+// error flag the tensor-core kernels set when a bounded wait runs out (kernels_conv_tc.cu)
+int* conv_tc_error_address();
 // nodal grid transfers of channels-last BF16 fields (kernels_conv.cu)
 void launch_prolong(cudaStream_t st, const int gf[3], const int gc[3], int C, const void* crs, int c_cs, int c_c0,
                     void* fine, int f_cs, int f_c0, float beta, float s);

@@ -1,14 +1,12 @@
 // kernels_conv.cu -- the learned correction's kernels besides the forward
-// convolution (kernels_conv_tc.cu): weight and bias gradients, the weight
-// flip of the data gradient, nodal grid transfers between the network's
+// convolution (kernels_conv_tc.cu) and the weight and bias gradients
+// (kernels_wgrad_tc.cu): the weight flip of the data gradient, nodal grid transfers between the network's
 // levels, masked gradient sums, and Adam.
 //
 // Fields are channels-last BF16 over nodal grids g = (gx, gy, gz), voxel =
 // x + gx (y + gy z), with a channel stride cs and a channel slice [c0, c0 +
 // C); the convolutions pad with zeros outside the grid.
 //
-//   wgrad     dW[tap][co][ci] += sum_v dy[v][co] in[v + off(tap)][ci]   (FP32)
-//   bgrad     db[co] += sum_v dy[v][co]
 //   flip      wt[26 - tap][ci][co] = w[tap][co][ci]: the data gradient of a
 //             layer is the forward convolution of dy with wt
 //   prolong   fine = beta fine + s P coarse, P trilinear between nodal grids
@@ -41,75 +39,6 @@ struct Grid {
     int g[3];
     __host__ __device__ long long count() const { return (long long)g[0] * g[1] * g[2]; }
 };
-
-// ---------------------------------------------------------------------------
-// weight gradient: one CTA per (tap, 16-output block, 16-input block, voxel
-// chunk); thread (co, ci) of a 16 x 16 block accumulates in FP32 over the
-// chunk, staged 64 voxels at a time in shared memory; one atomic per output.
-// ---------------------------------------------------------------------------
-constexpr int WG_V = 64;          // voxels per staging step
-constexpr int WG_CHUNK = 4096;    // voxels per CTA
-
-__global__ void __launch_bounds__(256) k_wgrad0(Grid G, int cin, int cout, const __nv_bfloat16* __restrict__ x, int x_cs,
-                                                int x_c0, const __nv_bfloat16* __restrict__ dy, int dy_cs, int dy_c0,
-                                                float* __restrict__ dw)
-{
-    __shared__ float ds[WG_V][17], xs[WG_V][17];
-    const int tap = blockIdx.y;
-    const int nb_ci = cin / 16;
-    const int co0 = (blockIdx.z / nb_ci) * 16, ci0 = (blockIdx.z % nb_ci) * 16;
-    const int dx = tap % 3 - 1, dyy = (tap / 3) % 3 - 1, dz = tap / 9 - 1;
-    const int tid = threadIdx.x, tco = tid >> 4, tci = tid & 15;
-    const long long V = (long long)G.g[0] * G.g[1] * G.g[2];
-    const long long v0 = (long long)blockIdx.x * WG_CHUNK;
-    const long long v1 = min(V, v0 + WG_CHUNK);
-    float acc = 0.f;
-    for (long long vb = v0; vb < v1; vb += WG_V) {
-        // stage dy[v][co0..+15] and x[v + off][ci0..+15] for 64 voxels (4 values per thread each)
-#pragma unroll
-        for (int q = 0; q < 4; q++) {
-            const int e = tid + 256 * q;   // 0 .. 1023
-            const int vl = e >> 4, c = e & 15;
-            const long long v = vb + vl;
-            float d = 0.f, xv = 0.f;
-            if (v < v1) {
-                d = __bfloat162float(dy[v * dy_cs + dy_c0 + co0 + c]);
-                const int ix = (int)(v % G.g[0]), iy = (int)((v / G.g[0]) % G.g[1]), iz = (int)(v / ((long long)G.g[0] * G.g[1]));
-                const int jx = ix + dx, jy = iy + dyy, jz = iz + dz;
-                if (jx >= 0 && jx < G.g[0] && jy >= 0 && jy < G.g[1] && jz >= 0 && jz < G.g[2]) {
-                    const long long w = jx + (long long)G.g[0] * (jy + (long long)G.g[1] * jz);
-                    xv = __bfloat162float(x[w * x_cs + x_c0 + ci0 + c]);
-                }
-            }
-            ds[vl][c] = d;
-            xs[vl][c] = xv;
-        }
-        __syncthreads();
-#pragma unroll 8
-        for (int v = 0; v < WG_V; v++) acc = fmaf(ds[v][tco], xs[v][tci], acc);
-        __syncthreads();
-    }
-    atomicAdd(dw + ((long long)tap * cout + co0 + tco) * cin + ci0 + tci, acc);
-}
-
-// db[co] += sum_v dy[v][c0 + co]
-__global__ void k_bgrad0(long long V, int cout, const __nv_bfloat16* __restrict__ dy, int dy_cs, int dy_c0,
-                         float* __restrict__ db)
-{
-    __shared__ float red[32];
-    const int co = blockIdx.y;
-    float s = 0.f;
-    for (long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x; v < V; v += (long long)gridDim.x * blockDim.x)
-        s += __bfloat162float(dy[v * dy_cs + dy_c0 + co]);
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
-    __syncthreads();
-    if (threadIdx.x < 32) {
-        s = threadIdx.x < (int)(blockDim.x >> 5) ? red[threadIdx.x] : 0.f;
-        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if (threadIdx.x == 0) atomicAdd(db + co, s);
-    }
-}
 
 // wt[26 - tap][ci][co] = w[tap][co][ci]
 __global__ void k_conv3_flip(int cin, int cout, const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ wt)
@@ -256,27 +185,6 @@ void launch_prolong_t(cudaStream_t st, const int gf[3], const int gc[3], int C, 
 }  // namespace agb
 
 using namespace agb;
-
-extern "C" agb_status agb_conv3_wgrad0(const int g[3], int cin, int cout, const void* x, int x_cs, int x_c0,
-                                       const void* dy, int dy_cs, int dy_c0, float* dw, float* db, void* stream)
-{
-    if (!grid_ok(g) || !x || !dy || !dw || cin < 16 || cin % 16 || cout < 16 || cout % 16 ||
-        !slice_ok(x_cs, x_c0, cin) || !slice_ok(dy_cs, dy_c0, cout)) {
-        set_error("agb_conv3_wgrad0: bad argument (channels multiples of 16, slices inside their strides)");
-        return AGB_BADARG;
-    }
-    Grid G{{g[0], g[1], g[2]}};
-    const long long V = G.count();
-    const long long chunks = (V + WG_CHUNK - 1) / WG_CHUNK;
-    cudaStream_t st = (cudaStream_t)stream;
-    dim3 grid((unsigned)chunks, 27, (unsigned)((cout / 16) * (cin / 16)));
-    k_wgrad0<<<grid, 256, 0, st>>>(G, cin, cout, (const __nv_bfloat16*)x, x_cs, x_c0, (const __nv_bfloat16*)dy, dy_cs,
-                                   dy_c0, dw);
-    agb_status s = launched();
-    if (s != AGB_OK || !db) return s;
-    k_bgrad0<<<dim3(sm_count(), cout), 256, 0, st>>>(V, cout, (const __nv_bfloat16*)dy, dy_cs, dy_c0, db);
-    return launched();
-}
 
 extern "C" agb_status agb_conv3_flip(int cin, int cout, const void* w, void* wt, void* stream)
 {

@@ -43,6 +43,7 @@
 #include "agb.h"
 #include "agb_internal.h"
 #include "tma.cuh"
+#include "umma.cuh"
 
 namespace agb {
 namespace {
@@ -61,53 +62,6 @@ template <int COUT> struct TcLayout {
     static constexpr int SMEM = BAR_OFF + 32 + 128;             // barriers, tmem slot, alignment room
     static constexpr int TMEM_COLS = COUT <= 32 ? 32 : (COUT <= 64 ? 64 : (COUT <= 128 ? 128 : 256));
 };
-
-// Shared-memory matrix descriptor of a no-swizzle K-major operand: start
-// address, leading byte offset (between the two 8-element K halves), stride
-// byte offset (between 8-row groups), descriptor version 1.
-__device__ __forceinline__ uint64_t umma_desc(uint32_t saddr, uint32_t lbo, uint32_t sbo)
-{
-    return (uint64_t)((saddr >> 4) & 0x3FFF) | ((uint64_t)((lbo >> 4) & 0x3FFF) << 16) |
-           ((uint64_t)((sbo >> 4) & 0x3FFF) << 32) | (1ull << 46);
-}
-
-// Instruction descriptor of kind::f16: FP32 accumulator, BF16 A and B, both
-// K-major, M = 128, N = n.
-__host__ __device__ constexpr uint32_t umma_idesc_bf16(int n)
-{
-    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(TC_M >> 4) << 24);
-}
-
-__device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                          uint32_t accumulate)
-{
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
-        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-
-__device__ __forceinline__ void umma_commit(uint32_t bar)
-{
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
-                 : "memory");
-}
-
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, float v[16])
-{
-    uint32_t r[16];
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, "
-        "%15}, [%16];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-        : "r"(taddr));
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-    for (int i = 0; i < 16; i++) v[i] = __uint_as_float(r[i]);
-}
 
 struct TcArgs {
     int nx, ny, nz;
@@ -136,10 +90,7 @@ __global__ void __launch_bounds__(TC_THREADS) k_conv3_tc(const __grid_constant__
     const int x0 = (t % ntx) * TC_M, y = (t / ntx) % a.ny, z = t / (ntx * a.ny);
 
     if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
-                     "r"((uint32_t)Lay::TMEM_COLS)
-                     : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        tmem_alloc(smem_u32(tmem_slot), (uint32_t)Lay::TMEM_COLS);
     }
     if (tid == 0) {
         mbar_init(bar_load, 1);
@@ -147,54 +98,52 @@ __global__ void __launch_bounds__(TC_THREADS) k_conv3_tc(const __grid_constant__
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         *okflag = 1;
     }
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    umma_fence_before();
     __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    umma_fence_after();
     const uint32_t taddr = *tmem_slot;
 
-    if (tid == 0) {
+    if (warp == 0) {
         const int nstage = a.cin / 16;
-        constexpr uint32_t idesc = umma_idesc_bf16(COUT);
+        constexpr uint32_t idesc = umma_idesc_bf16(TC_M, COUT, false);
         bool ok = true;
         int pend_load = -1, pend_mma = -1;   // parity of a phase issued and not seen complete
+        const uint64_t ad = umma_desc(sA, TC_CHUNK_PAD, 128), bd = umma_desc(sW, COUT * 16, 128);
         for (int s = 0; s < nstage && ok; s++) {
-            mbar_expect(bar_load, 2 * TC_CHUNK + Lay::W_BYTES);
-            for (int c = 0; c < 2; c++)
-                tma_load4(sA + c * TC_CHUNK_PAD, &tin, a.in_c0 + 16 * s + 8 * c, x0 - 1, y - 1, z - 1, bar_load);
-            bulk_load(sW, a.wp + (size_t)s * 27 * 2 * COUT * 8, Lay::W_BYTES, bar_load);
-            pend_load = s & 1;
-            if (!mbar_wait(bar_load, (uint32_t)(s & 1))) {
-                ok = false;
-                break;
+            if (lane == 0) {
+                mbar_expect(bar_load, 2 * TC_CHUNK + Lay::W_BYTES);
+                for (int c = 0; c < 2; c++)
+                    tma_load4(sA + c * TC_CHUNK_PAD, &tin, a.in_c0 + 16 * s + 8 * c, x0 - 1, y - 1, z - 1, bar_load);
+                bulk_load(sW, a.wp + (size_t)s * 27 * 2 * COUT * 8, Lay::W_BYTES, bar_load);
             }
+            pend_load = s & 1;
+            ok = __all_sync(0xffffffffu, mbar_wait(bar_load, (uint32_t)(s & 1)));
+            if (!ok) break;
             pend_load = -1;
-#pragma unroll 1
+#pragma unroll
             for (int tap = 0; tap < 27; tap++) {
                 const int dx = tap % 3, dy = (tap / 3) % 3, dz = tap / 9;   // each offset + 1
-                const uint32_t aaddr = sA + ((dz * 3 + dy) * TC_HX + dx) * 16;
-                const uint32_t baddr = sW + tap * 2 * COUT * 16;
-                umma_bf16(taddr, umma_desc(aaddr, TC_CHUNK_PAD, 128), umma_desc(baddr, COUT * 16, 128), idesc,
+                umma_bf16(taddr, umma_advance(ad, (dz * 3 + dy) * TC_HX + dx), umma_advance(bd, tap * 2 * COUT), idesc,
                           (s > 0 || tap > 0) ? 1u : 0u);
             }
             umma_commit(bar_mma);
             pend_mma = s & 1;
-            if (!mbar_wait(bar_mma, (uint32_t)(s & 1))) {
-                ok = false;
-                break;
-            }
+            ok = __all_sync(0xffffffffu, mbar_wait(bar_mma, (uint32_t)(s & 1)));
+            if (!ok) break;
             pend_mma = -1;
         }
-        if (!ok) {
+        if (!ok && lane == 0) {
             // bounded drain of what is still in flight, then report
             if (pend_load >= 0) mbar_wait(bar_load, (uint32_t)pend_load);
             if (pend_mma >= 0) mbar_wait(bar_mma, (uint32_t)pend_mma);
             atomicExch(a.err, 1);
             *okflag = 0;
         }
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncwarp();
+        umma_fence_before();
     }
     __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    umma_fence_after();
     if (*okflag) {
         const int x = x0 + 32 * warp + lane;
         const bool mine = x < a.nx;
@@ -229,12 +178,10 @@ __global__ void __launch_bounds__(TC_THREADS) k_conv3_tc(const __grid_constant__
             }
         }
     }
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    umma_fence_before();
     __syncthreads();
     if (warp == 0)
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr),
-                     "r"((uint32_t)Lay::TMEM_COLS)
-                     : "memory");
+        tmem_free(taddr, (uint32_t)Lay::TMEM_COLS);
 }
 
 // wp[((s * 27 + tap) * 2 + h) * cout + co][e] = w[tap][co0 + co][16 s + 8 h + e], w of w_cout rows per tap
@@ -319,6 +266,17 @@ void init_conv_tc_attributes()
     tc_attr<64>();
 }
 
+// Device address of the error flag of the tensor-core kernels (null without one).
+int* conv_tc_error_address()
+{
+    static int* err = [] {
+        int* p = nullptr;
+        if (cudaGetSymbolAddress((void**)&p, g_tc_error) != cudaSuccess) p = nullptr;
+        return p;
+    }();
+    return err;
+}
+
 // Reads and clears the error flag the tensor-core convolution sets when a
 // bounded wait runs out.
 int conv_tc_error_take()
@@ -372,11 +330,7 @@ extern "C" agb_status agb_conv3_tc(const int n[3], int cin, int cout, const void
         set_error("agb_conv3_tc: channel strides and slice starts must be multiples of 8, pointers 16-byte aligned");
         return AGB_BADARG;
     }
-    static int* err = [] {
-        int* p = nullptr;
-        if (cudaGetSymbolAddress((void**)&p, g_tc_error) != cudaSuccess) p = nullptr;
-        return p;
-    }();
+    int* err = conv_tc_error_address();
     static bool attr = [] {
         init_conv_tc_attributes();
         return true;
