@@ -1633,44 +1633,79 @@ agb_status agb_newton_solve(agb_solver s, const double* F0, double* u, const dou
     return st == AGB_OK ? sst : st;
 }
 
+// A caller's output buffer as the device writes it: itself, the mapped address
+// of pinned memory, or null (pageable memory the device does not reach).
+static double* device_view(agb_op op, double* p, int mem)
+{
+    if (mem == AGB_MEM_DEVICE) return p;
+    if (double* m = (double*)mapped_host(p, mem)) return m;
+    return !pinned_host(p, mem) && directly_readable(op, p, mem) ? p : nullptr;
+}
+
+// u of the fields computed from a displacement: read in place in device
+// memory (*full), else imported into the operator's work buffer.
+static agb_status post_input(agb_op op, const double* u, int mem, const double** du, bool* full)
+{
+    *full = mem == AGB_MEM_DEVICE;
+    if (*full) {
+        *du = u;
+        return caller_ready(mem);
+    }
+    Level& v = op->lev[0];
+    *du = v.hold64;
+    return upload<double, double>(op, v.L, 3, false, u, mem, v.hold64);
+}
+
+// Copies a box of `count` doubles the device wrote into pageable memory.
+static agb_status post_copy(agb_op op, double* dst, const double* src, size_t count)
+{
+    CK(cudaMemcpyAsync(dst, src, count * sizeof(double), cudaMemcpyDeviceToHost, op->st));
+    return AGB_OK;
+}
+
+// Stress, strain and energy of u into caller buffers (any may be null).
+static agb_status post_fields(agb_op op, const double* F0, const double* u, double* sigma, double* eps, double* energy,
+                              int mem)
+{
+    Level& v = op->lev[0];
+    const size_t N = (size_t)(v.L.n[0] + 1) * (v.L.n[1] + 1) * (v.L.n[2] + 1);
+    double* dF0 = nullptr;
+    TRY(load_F0(op, F0, mem, &dF0));
+    const double* du = nullptr;
+    bool full = false;
+    TRY(post_input(op, u, mem, &du, &full));
+    double* want[3] = {sigma, eps, energy};
+    double *dev[3] = {nullptr, nullptr, nullptr}, *tmp[3] = {nullptr, nullptr, nullptr};
+    const size_t count[3] = {9 * N, 9 * N, N};
+    agb_status st = AGB_OK;
+    for (int q = 0; q < 3 && st == AGB_OK; q++) {
+        if (!want[q]) continue;
+        dev[q] = device_view(op, want[q], mem);
+        if (!dev[q] && (st = op->alloc(&tmp[q], count[q])) == AGB_OK) dev[q] = tmp[q];
+    }
+    if (st == AGB_OK) {
+        launch_post(op->st, op->sym, v.L, v.ddw64, dF0, du, full, dev[0], dev[1], dev[2]);
+        if (cudaGetLastError() != cudaSuccess) st = fail(AGB_CUDA, "stress/strain/energy launch failed");
+    }
+    for (int q = 0; q < 3 && st == AGB_OK; q++)
+        if (tmp[q]) st = post_copy(op, want[q], tmp[q], count[q]);
+    if (st == AGB_OK && cudaStreamSynchronize(op->st) != cudaSuccess) st = fail(AGB_CUDA, "stress/strain/energy failed");
+    for (int q = 0; q < 3; q++) release(op, tmp[q]);
+    return st;
+}
+
 agb_status agb_stress(agb_op op, const double* F0, const double* u, double* sigma9, int mem)
 {
     if (!op || !u || !sigma9) return fail(AGB_BADARG, "null argument");
     if (!op->model_set) return fail(AGB_STATE, "SetModel must be called first");
-    Level& v = op->lev[0];
-    double *dF0 = nullptr, *sg = nullptr;
-    TRY(load_F0(op, F0, mem, &dF0));
-    agb_status st = op->alloc(&sg, 9 * (size_t)v.L.S);
-    if (st == AGB_OK) st = upload<double, double>(op, v.L, 3, false, u, mem, v.hold64);
-    if (st == AGB_OK) {
-        launch_stress(op->st, op->sym, v.L, v.ddw64, dF0, v.hold64, sg);
-        st = download<double, double>(op, v.L, 9, true, sg, sigma9, mem);
-    }
-    if (st == AGB_OK && cudaStreamSynchronize(op->st) != cudaSuccess) st = fail(AGB_CUDA, "stress failed");
-    release(op, sg);
-    return st;
+    return post_fields(op, F0, u, sigma9, nullptr, nullptr, mem);
 }
 
 agb_status agb_strain_energy(agb_op op, const double* u, double* eps9, double* energy, int mem)
 {
     if (!op || !u || (!eps9 && !energy)) return fail(AGB_BADARG, "null argument");
     if (!op->model_set) return fail(AGB_STATE, "SetModel must be called first");
-    Level& v = op->lev[0];
-    double *de = nullptr, *dw = nullptr;
-    agb_status st = AGB_OK;
-    if (eps9) st = op->alloc(&de, 9 * (size_t)v.L.S);
-    if (st == AGB_OK && energy) st = op->alloc(&dw, (size_t)v.L.S);
-    if (st == AGB_OK) st = upload<double, double>(op, v.L, 3, false, u, mem, v.hold64);
-    if (st == AGB_OK) {
-        launch_strain_energy(op->st, op->sym, v.L, v.ddw64, v.hold64, de, dw);
-        if (cudaGetLastError() != cudaSuccess) st = fail(AGB_CUDA, "strain/energy launch failed");
-    }
-    if (st == AGB_OK && eps9) st = download<double, double>(op, v.L, 9, true, de, eps9, mem);
-    if (st == AGB_OK && energy) st = download<double, double>(op, v.L, 1, false, dw, energy, mem);
-    if (st == AGB_OK && cudaStreamSynchronize(op->st) != cudaSuccess) st = fail(AGB_CUDA, "strain/energy failed");
-    if (de) release(op, de);
-    if (dw) release(op, dw);
-    return st;
+    return post_fields(op, nullptr, u, nullptr, eps9, energy, mem);
 }
 
 agb_status agb_traction_xhi(agb_op op, const double* F0, const double* u, double trac[3], int mem)
@@ -1678,22 +1713,20 @@ agb_status agb_traction_xhi(agb_op op, const double* F0, const double* u, double
     if (!op || !u || !trac) return fail(AGB_BADARG, "null argument");
     if (!op->model_set) return fail(AGB_STATE, "SetModel must be called first");
     Level& v = op->lev[0];
-    double *dF0 = nullptr, *sg = nullptr;
+    double* dF0 = nullptr;
     TRY(load_F0(op, F0, mem, &dF0));
-    agb_status st = op->alloc(&sg, 9 * (size_t)v.L.S);
-    if (st == AGB_OK) st = upload<double, double>(op, v.L, 3, false, u, mem, v.hold64);
-    if (st == AGB_OK) {
-        launch_stress(op->st, op->sym, v.L, v.ddw64, dF0, v.hold64, sg);
-        launch_traction_xhi(op->st, v.L, sg, op->d_slots + 4);
-        if (cudaMemcpyAsync(op->h_slots + 4, op->d_slots + 4, 3 * sizeof(double), cudaMemcpyDeviceToHost, op->st) !=
-                cudaSuccess ||
-            cudaStreamSynchronize(op->st) != cudaSuccess)
-            st = fail(AGB_CUDA, "traction failed");
-        else
-            for (int r = 0; r < 3; r++) trac[r] = op->h_slots[4 + r];
-    }
-    release(op, sg);
-    return st;
+    const double* du = nullptr;
+    bool full = false;
+    TRY(post_input(op, u, mem, &du, &full));
+    // the bottom solve's work (8 x 3 x 64 doubles at least) is free outside a solve
+    launch_traction_xhi(op->st, op->sym, v.L, v.ddw64, dF0, du, full, op->bottom_work, op->d_slots + 4);
+    if (cudaGetLastError() != cudaSuccess ||
+        cudaMemcpyAsync(op->h_slots + 4, op->d_slots + 4, 3 * sizeof(double), cudaMemcpyDeviceToHost, op->st) !=
+            cudaSuccess ||
+        cudaStreamSynchronize(op->st) != cudaSuccess)
+        return fail(AGB_CUDA, "traction failed");
+    for (int r = 0; r < 3; r++) trac[r] = op->h_slots[4 + r];
+    return AGB_OK;
 }
 
 agb_status agb_op_time_sweep(agb_op op, int level, int precision, int mode, int reps, double* ms_per_launch)

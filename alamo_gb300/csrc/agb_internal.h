@@ -310,11 +310,13 @@ void launch_bottom(cudaStream_t st, int sym, const LevelDesc& L, const BCTable& 
 
 void launch_newton_rhs(cudaStream_t st, int sym, const LevelDesc& L, const BCTable& bc, const double* ddw,
                        const double* F0, const double* u, const double* b, double* rhs, double* dw_work);
-void launch_stress(cudaStream_t st, int sym, const LevelDesc& L, const double* ddw, const double* F0,
-                   const double* u, double* sigma);
-void launch_strain_energy(cudaStream_t st, int sym, const LevelDesc& L, const double* ddw, const double* u,
-                          double* eps, double* energy);
-void launch_traction_xhi(cudaStream_t st, const LevelDesc& L, const double* sigma, double* out3);
+// u in padded storage, or (full) in the caller's unpadded box; sigma and eps (9
+// a node, interleaved) and energy are caller boxes, any of them null
+void launch_post(cudaStream_t st, int sym, const LevelDesc& L, const double* ddw, const double* F0, const double* u,
+                 bool full, double* sigma, double* eps, double* energy);
+// part: scratch of 768 doubles
+void launch_traction_xhi(cudaStream_t st, int sym, const LevelDesc& L, const double* ddw, const double* F0,
+                         const double* u, bool full, double* part, double* out3);
 void launch_bc_init(cudaStream_t st, const LevelDesc& L, const BCTable& bc, double* rhs, int homogeneous);
 
 }  // namespace agb

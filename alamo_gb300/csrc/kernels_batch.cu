@@ -943,7 +943,7 @@ __global__ void __launch_bounds__(256) k_batch_rhs(const BProb* __restrict__ pro
             }
             c_mul_mat<double, SYM>(cpv, E, Dp);
             c_mul_mat<double, SYM>(cmv, E, Dm);
-            for (int r = 0; r < 3; r++) ret[r] += (Dp[r][d] - Dm[r][d]) / 2. / L.dx[d];
+            for (int r = 0; r < 3; r++) ret[r] += (Dp[r][d] - Dm[r][d]) * P.h1[d];
         }
         for (int r = 0; r < 3; r++) rhs[P.vo + r * L.S + nb.base] = 0.0 - ret[r];
     }
@@ -971,7 +971,7 @@ __global__ void __launch_bounds__(256) k_batch_mean_stress(const BProb* __restri
             for (int p = 0; p < 3; p++)
                 for (int d = 0; d < 3; d++)
                     G[p][d] = (u[P.vo + p * L.S + nb.base + nb.o[d][2]] - u[P.vo + p * L.S + nb.base + nb.o[d][0]]) *
-                                  0.5 / L.dx[d] -
+                                  P.h1[d] -
                               F0[tl.prob * 9 + p * 3 + d];
             for (int m = 0; m < NCoef<SYM>::value; m++) c[m] = ddw[P.co + m * L.S + nb.base];
             c_mul_mat<double, SYM>(c, G, S);

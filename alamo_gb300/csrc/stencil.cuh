@@ -429,9 +429,10 @@ __device__ __forceinline__ void boundary_row(const A& acc, const Geo<T>& g, cons
 #pragma unroll
         for (int d = 0; d < 3; d++) {
             const int ox = d == 0, oy = d == 1, oz = d == 2;
-            if (mn[d]) G[p][d] = (acc.u(p, ox, oy, oz) - u[p]) * g.i1[d];          // StencilType::Hi
-            else if (mx[d]) G[p][d] = (u[p] - acc.u(p, -ox, -oy, -oz)) * g.i1[d];  // StencilType::Lo
-            else G[p][d] = (acc.u(p, ox, oy, oz) - acc.u(p, -ox, -oy, -oz)) * g.h1[d];
+            // StencilType::Hi on the lo face, Lo on the hi face, central between:
+            // one difference and one product with the operands selected
+            const T hi = mx[d] ? u[p] : acc.u(p, ox, oy, oz), lo = mn[d] ? u[p] : acc.u(p, -ox, -oy, -oz);
+            G[p][d] = (hi - lo) * (mn[d] || mx[d] ? g.i1[d] : g.h1[d]);
         }
     }
     T c[NCoef<SYM>::value];
