@@ -261,6 +261,10 @@ agb_status learned_features(cudaStream_t st, int sym, const LevelDesc& L, const 
                             void* feat, double* acc);
 // error flag the tensor-core kernels set when a bounded wait runs out (kernels_conv_tc.cu)
 int* conv_tc_error_address();
+// the convolution by planes (kernels_conv_march.cu); false: it does not serve this shape
+bool launch_conv3_march(cudaStream_t st, const int n[3], int cin, int cout, const void* in, int in_cs, int in_c0,
+                        const void* wp, const float* bias, void* out, int out_cs, int out_c0, int out_f32, int relu,
+                        int* err);
 // nodal grid transfers of channels-last BF16 fields (kernels_conv.cu)
 void launch_prolong(cudaStream_t st, const int gf[3], const int gc[3], int C, const void* crs, int c_cs, int c_c0,
                     void* fine, int f_cs, int f_c0, float beta, float s);

@@ -336,6 +336,16 @@ extern "C" agb_status agb_conv3_tc(const int n[3], int cin, int cout, const void
         return true;
     }();
     (void)attr;
+    if (err && launch_conv3_march((cudaStream_t)stream, n, cin, cout, in, in_cs, in_c0, wp, bias, out, out_cs, out_c0,
+                                  out_f32, relu, err)) {
+        count_launch();
+        const cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess) {
+            set_error(cudaGetErrorString(e));
+            return AGB_CUDA;
+        }
+        return AGB_OK;
+    }
     CUtensorMap m;
     if (!err || !tc_map(in, in_cs, n, &m)) {
         set_error("agb_conv3_tc: tensor map encoding failed");

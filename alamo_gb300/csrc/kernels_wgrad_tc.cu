@@ -81,11 +81,6 @@ __host__ __device__ inline int smem_bytes(int kx, int cb, int co, int T, int sta
     return 128 + stages * stage_bytes(kx, cb, co, T) + 16 * x_pitch(kx) + 128;
 }
 
-__device__ __forceinline__ void copy16(uint32_t dst, const void* src, bool valid)
-{
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(valid ? 16 : 0) : "memory");
-}
-
 // `lines` lines from (x0, y0, z) of GROUPS x 8 channels into dst, `len` voxels each
 template <int GROUPS, int COPY>
 __device__ __forceinline__ void copy_lines(uint32_t dst, int pitch, int lines, int len, const __nv_bfloat16* base,
@@ -176,7 +171,7 @@ __global__ void __launch_bounds__(WtThreads<CO>::all, 1) k_wgrad_tc(WtArgs a)
             copy_lines<CB / 8, COPY>(dst, xp, a.T + 2, a.kx + 2, a.x + ci0, a.x_cs, x0 - 1, y0 - 1, z + dz - 1, a, t);
             copy_lines<CO / 8, COPY>(dst + xbytes, dp, a.T, a.kx, a.dy + co0, a.dy_cs, x0, y0, z, a, t);
             // the thread's arrival, once its copies so far have landed
-            asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(full + 8 * s) : "memory");
+            copy_arrive(full + 8 * s);
             n++;
         }
         asm volatile("cp.async.wait_all;" ::: "memory");   // the shared memory outlives the copies

@@ -69,4 +69,16 @@ __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_
                  : "memory");
 }
 
+// 16 bytes global -> shared by the calling thread, zeros when not `valid` (src
+// must still be an address of the field); and the thread's arrival on `bar`
+// once its copies so far have landed.
+__device__ __forceinline__ void copy16(uint32_t dst, const void* src, bool valid)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(valid ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void copy_arrive(uint32_t bar)
+{
+    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
+}
+
 }  // namespace agb

@@ -28,8 +28,12 @@ __host__ __device__ constexpr uint32_t umma_idesc_bf16(int m, int n, bool mn_maj
            ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
 }
 
-// The descriptor of the operand `units` 16-byte units further on.
-__device__ __forceinline__ uint64_t umma_advance(uint64_t desc, int units) { return desc + (uint64_t)(int64_t)units; }
+// The descriptor of the operand `units` 16-byte units further on (within the
+// address field: shared memory ends below 2^18 bytes).
+__device__ __forceinline__ uint64_t umma_advance(uint64_t desc, int units)
+{
+    return (desc & 0xffffffff00000000ull) | (uint32_t)((uint32_t)desc + (uint32_t)units);
+}
 
 // One MMA, issued by one elected lane.  The whole (converged) warp calls this
 // with the same operands: the compiler then keeps descriptors in uniform
@@ -105,5 +109,15 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float v[16])
 #pragma unroll
     for (int i = 0; i < 16; i++) v[i] = __uint_as_float(r[i]);
 }
+
+// Zeros into 16 columns of the warp's 32 lanes.
+__device__ __forceinline__ void tmem_zero16(uint32_t taddr)
+{
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, "
+                 "%1, %1};" ::"r"(taddr),
+                 "r"(0u)
+                 : "memory");
+}
+__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
 }  // namespace agb
