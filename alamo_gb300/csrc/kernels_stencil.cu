@@ -674,16 +674,29 @@ bool use_pipe_kernel()
     return v;
 }
 
-// Whether the interior of a level goes to the tiled FP32 kernels (TMA, or
-// cp.async when a tensor map cannot be made): a box with no periodic direction,
-// large enough to fill every SM several times.
+// Whether the interior of a level may go to the marching kernels: a box with
+// no periodic direction, large enough to fill every SM several times.
 static bool big_level(const LevelDesc& L)
 {
     return !L.per[0] && !L.per[1] && !L.per[2] && L.n[0] >= march_min_cells() && L.n[1] >= 16 && L.n[2] >= 16;
 }
-static bool tiled_f32(const LevelDesc& L) { return big_level(L) && (use_tma_kernel() || use_pipe_kernel()); }
+// FP32: the tiled kernels read each value from HBM once (132 bytes a node and
+// Jacobi sweep with general moduli, 56 isotropic); k_rows reads 204 (56) with the
+// divergence but has neither a shared-memory ring to fill nor a second launch
+// for the shell, so it wins while a level's sweep stays in half of the L2.
+// Jacobi, tiled / k_rows: general 65^3 nodes 20.5 / 13.2 us, 81^3 32.8 / 33.7,
+// 113^3 70.7 / 82.6, 129^3 84.3 / 108.6; isotropic 65^3 15.4 / 10.3, 97^3 27.6 /
+// 20.5, 129^3 56.1 / 63.7.
+static bool tiled_f32(int sym, const LevelDesc& L)
+{
+    const long long bytes = 4LL * L.count() * (sym == SYM_MM ? 21 + 18 + 12 : 2 + 12);
+    return big_level(L) && bytes > (64LL << 20) && (use_tma_kernel() || use_pipe_kernel());
+}
 
-bool stencil_uses_div(int sym, bool fp32, const LevelDesc& L) { return sym == SYM_MM && !(fp32 && tiled_f32(L)); }
+bool stencil_uses_div(int sym, bool fp32, const LevelDesc& L)
+{
+    return sym == SYM_MM && !(fp32 && tiled_f32(sym, L));
+}
 
 template <typename T, int SYM, int MODE, bool CUBE>
 static void rows_dispatch(cudaStream_t st, const LevelDesc& L, const BCTable& bc, const Geo<T>& g, bool uniform,
@@ -725,7 +738,7 @@ static void stencil_dispatch(cudaStream_t st, const LevelDesc& L, const BCTable&
 {
     const Geo<T> g = make_geo<T>(L);
     if constexpr (sizeof(T) == 4) {
-        if (tiled_f32(L)) {
+        if (tiled_f32(SYM, L)) {
             // interior by the tiled kernel, boundary shell by the per-node
             // kernel (the TMA kernel also takes the x-face nodes)
             bool tma = false;

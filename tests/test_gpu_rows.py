@@ -53,3 +53,31 @@ def test_rows_match_oracle(gpu_lib, box, sym, cube):
     g.uniform = 1
     assert rel_err(op.Fapply(0, u), O.fapply(g, ddw, u)) < 1e-12
     op.close()
+
+
+@pytest.mark.parametrize("n,sym", [([100, 61, 60], O.MAJORMINOR), ([130, 101, 95], O.ISO)])
+@pytest.mark.parametrize("uniform", [False, True])
+def test_fp32_tiled_boxes(gpu_lib, n, sym, uniform):
+    """The smallest ragged boxes whose FP32 sweep exceeds half of the L2 and so
+    goes to the tiled kernels; the FP32 bar of the other operator tests."""
+    from alamo_gb300 import Constant, Elastic
+    dx = [1 / 100, 1 / 61, 1 / 90]
+    bt, bv = random_bc(51, ("disp",))
+    g = O.make_grid(n, dx=dx, sym=sym, bc_type=bt, bc_val=bv)
+    op = Elastic(n, dx, "isotropic" if sym == O.ISO else "majorminor")
+    bc = Constant()
+    bc.type[:] = bt
+    bc.val[:] = bv
+    op.SetBC(bc)
+    ddw = random_ddw(n, sym, 52)
+    op.SetModel(ddw)
+    if uniform:
+        op.SetUniform(True)
+        g.uniform = 1
+    d32 = ddw.astype(np.float32).astype(np.float64)
+    u = random_field(n, 53, dtype=np.float32)
+    b = random_field(n, 54, dtype=np.float32)
+    assert rel_err(op.Fapply(0, u).astype(np.float64), O.fapply(g, d32, u.astype(np.float64))) < 1e-5
+    x = op.Fsmooth(0, u.copy(), b).astype(np.float64)
+    assert rel_err(x, O.fsmooth(g, d32, O.diagonal(g, d32), u.astype(np.float64), b.astype(np.float64))) < 1e-5
+    op.close()
