@@ -237,8 +237,8 @@ template <typename T> struct BEngine {
             BLevel& v = b->lev[l];
             if (v.t32_smooth.empty()) continue;
             BLevel& c = b->lev[l + 1];
-            launch_batch_transfer<T>(b->st, 0, false, b->grid, v.d_probs, c.d_probs, v.c_t32_smooth,
-                                     (int)v.t32_smooth.size(), act, A::cor(c), A::cor(v));
+            launch_batch_transfer<T>(b->st, 0, false, b->grid, v.d_probs, c.d_probs, c.c_t32_full,
+                                     (int)c.t32_full.size(), act, A::cor(c), A::cor(v));
             smooth(l, A::cor(v), A::res(v), b->p.post_smooth);
         }
     }
@@ -272,8 +272,8 @@ template <typename T> struct BEngine {
             BLevel& v = b->lev[l];
             if (v.t32_smooth.empty()) continue;
             BLevel& c = b->lev[l + 1];
-            launch_batch_transfer<T>(b->st, 0, true, b->grid, v.d_probs, c.d_probs, v.c_t32_smooth,
-                                     (int)v.t32_smooth.size(), act, A::cor(c), A::cor(v));
+            launch_batch_transfer<T>(b->st, 0, true, b->grid, v.d_probs, c.d_probs, c.c_t32_full,
+                                     (int)c.t32_full.size(), act, A::cor(c), A::cor(v));
             launch_batch_stencil<T>(b->st, b->sym, MODE_RESID, v.shape, b->grid, v.d_probs, v.c_tS_smooth,
                                     (int)v.tS_smooth.size(), act, b->bc, false, A::ddw(v), A::cor(v), A::res(v),
                                     nullptr, A::rescor(v), (T)0, nullptr);

@@ -531,7 +531,8 @@ __global__ void __launch_bounds__(256, 3) k_batch_pipe(const BProb* __restrict__
 }
 
 // Full weighting (restriction) or trilinear prolongation between the levels of
-// every listed problem.  Tiles cover the destination level.
+// every listed problem.  Tiles cover the coarse level (32 x 4 x 2 shape): a
+// thread takes one coarse node or cell (RestrictNode, InterpCell).
 template <typename T>
 __global__ void __launch_bounds__(256) k_batch_transfer(int restrict_not_interp, int assign,
                                                         const BProb* __restrict__ pf, const BProb* __restrict__ pc,
@@ -545,36 +546,18 @@ __global__ void __launch_bounds__(256) k_batch_transfer(int restrict_not_interp,
         if (active && !active[tl.prob]) continue;
         const LevelDesc& Lf = pf[tl.prob].L;
         const LevelDesc& Lc = pc[tl.prob].L;
-        const LevelDesc& Ld = restrict_not_interp ? Lc : Lf;
-        // tiles of batched transfers always use the 32x4x2 shape
         int i, j, k;
-        if (!tile_node<32, 4, 2>(tl, Ld, i, j, k)) continue;
+        if (!tile_node<32, 4, 2>(tl, Lc, i, j, k)) continue;
+        const long long vf = pf[tl.prob].vo, vc = pc[tl.prob].vo;
         if (restrict_not_interp) {
-            const bool bI = !Lc.per[0] && (i == 0 || i == Lc.n[0]);
-            const bool bJ = !Lc.per[1] && (j == 0 || j == Lc.n[1]);
-            const bool bK = !Lc.per[2] && (k == 0 || k == Lc.n[2]);
-            const long long q = pc[tl.prob].vo + Lc.idx(i, j, k);
-            for (int c = 0; c < 3; c++) {
-                const T* s = src + pf[tl.prob].vo + c * Lf.S;
-                auto f = [&](int a, int b, int d) -> T {
-                    return __ldg(s + Lf.idx(wrapn(2 * i + a, Lf.n[0], Lf.per[0]), wrapn(2 * j + b, Lf.n[1], Lf.per[1]),
-                                            wrapn(2 * k + d, Lf.n[2], Lf.per[2])));
-                };
-                dst[q + c * Lc.S] = full_weight<T>(f, bI, bJ, bK);
-            }
+            const RestrictNode<T> r(Lf, Lc, i, j, k);
+            const long long q = vc + Lc.idx(i, j, k);
+#pragma unroll
+            for (int c = 0; c < 3; c++) dst[q + c * Lc.S] = r(src + vf + c * Lf.S);
         } else {
-            const int I = i >> 1, J = j >> 1, K = k >> 1;
-            const int I1 = wrapn(I + 1, Lc.n[0], Lc.per[0]), J1 = wrapn(J + 1, Lc.n[1], Lc.per[1]),
-                      K1 = wrapn(K + 1, Lc.n[2], Lc.per[2]);
-            const bool ei = !(i & 1), ej = !(j & 1), ek = !(k & 1);
-            const long long q = pf[tl.prob].vo + Lf.idx(i, j, k);
-            for (int c = 0; c < 3; c++) {
-                const T* cs = src + pc[tl.prob].vo + c * Lc.S;
-                auto C = [&](int a, int b, int d) -> T { return __ldg(cs + Lc.idx(a ? I1 : I, b ? J1 : J, d ? K1 : K)); };
-                const T v = interp_node<T>(C, ei, ej, ek);
-                T* o = dst + q + c * Lf.S;
-                *o = assign ? v : (*o + v);
-            }
+            const InterpCell<T> cell(Lf, Lc, i, j, k);
+#pragma unroll
+            for (int c = 0; c < 3; c++) cell(src + vc + c * Lc.S, dst + vf + c * Lf.S, assign != 0);
         }
     }
 }
@@ -590,18 +573,9 @@ __global__ void __launch_bounds__(256) k_batch_avg_ddw(const BProb* __restrict__
         const LevelDesc& Lc = pc[tl.prob].L;
         int I, J, K;
         if (!tile_node<32, 4, 2>(tl, Lc, I, J, K)) continue;
-        const bool bI = !Lc.per[0] && (I == 0 || I == Lc.n[0]);
-        const bool bJ = !Lc.per[1] && (J == 0 || J == Lc.n[1]);
-        const bool bK = !Lc.per[2] && (K == 0 || K == Lc.n[2]);
         const long long q = pc[tl.prob].co + Lc.idx(I, J, K);
-        for (int m = 0; m < ncoef; m++) {
-            const double* s = fine + pf[tl.prob].co + m * Lf.S;
-            auto f = [&](int a, int b, int d) -> double {
-                return s[Lf.idx(wrapn(2 * I + a, Lf.n[0], Lf.per[0]), wrapn(2 * J + b, Lf.n[1], Lf.per[1]),
-                                wrapn(2 * K + d, Lf.n[2], Lf.per[2]))];
-            };
-            crse[q + m * Lc.S] = full_weight<double>(f, bI, bJ, bK);
-        }
+        const RestrictNode<double> r(Lf, Lc, I, J, K);
+        for (int m = 0; m < ncoef; m++) crse[q + m * Lc.S] = r(fine + pf[tl.prob].co + m * Lf.S);
     }
 }
 

@@ -20,113 +20,37 @@ static inline dim3 grid_for(const LevelDesc& L, dim3 blk)
     return dim3((L.nn[0] + blk.x - 1) / blk.x, (L.nn[1] + blk.y - 1) / blk.y, (L.nn[2] + blk.z - 1) / blk.z);
 }
 
-// Fine-level offsets of the nodes 2I-1, 2I, 2I+1 (periodic wrap) in the three
-// directions of a coarse node, computed once per thread: each of the 27
-// reads of a full weighting is then one add of three offsets.
-struct FineOffsets {
-    int ox[3];
-    int oy[3];
-    long long oz[3];
-    __device__ __forceinline__ FineOffsets(const LevelDesc& Lf, int I, int J, int K)
-    {
-#pragma unroll
-        for (int a = 0; a < 3; a++) {
-            ox[a] = wrapn(2 * I + a - 1, Lf.n[0], Lf.per[0]);
-            oy[a] = Lf.P * wrapn(2 * J + a - 1, Lf.n[1], Lf.per[1]);
-            oz[a] = (long long)Lf.P * Lf.nn[1] * wrapn(2 * K + a - 1, Lf.n[2], Lf.per[2]);
-        }
-    }
-    __device__ __forceinline__ long long at(int a, int b, int d) const { return ox[a + 1] + oy[b + 1] + oz[d + 1]; }
-};
-
+// One coarse node and component a thread (blockIdx.z counts planes and
+// components): on the coarse levels the three components side by side are
+// three times the threads, and the FP64 sums a third as long.  257^3 -> 129^3
+// nodes, FP32: 103 us (27 reads and a loop over the components: 135); 9^3 -> 5^3,
+// FP64: 5.3 us (10.5).
 template <typename T>
-__global__ void k_restrict(LevelDesc Lf, LevelDesc Lc, const T* __restrict__ fine, T* __restrict__ crse, int ncomp)
+__global__ void __launch_bounds__(256) k_restrict(LevelDesc Lf, LevelDesc Lc, const T* __restrict__ fine,
+                                                  T* __restrict__ crse, int ncomp)
 {
     pdl_entry();
     const int I = blockIdx.x * blockDim.x + threadIdx.x;
     const int J = blockIdx.y * blockDim.y + threadIdx.y;
-    const int K = blockIdx.z * blockDim.z + threadIdx.z;
+    const int c = blockIdx.z % ncomp, K = (blockIdx.z / ncomp) * blockDim.z + threadIdx.z;
     if (I >= Lc.nn[0] || J >= Lc.nn[1] || K >= Lc.nn[2]) return;
-    const bool bI = !Lc.per[0] && (I == 0 || I == Lc.n[0]);
-    const bool bJ = !Lc.per[1] && (J == 0 || J == Lc.n[1]);
-    const bool bK = !Lc.per[2] && (K == 0 || K == Lc.n[2]);
-    const long long q = Lc.idx(I, J, K);
-    const FineOffsets o(Lf, I, J, K);
-    for (int c = 0; c < ncomp; c++) {
-        const T* src = fine + c * Lf.S;
-        auto f = [&](int a, int b, int d) -> T { return __ldg(src + o.at(a, b, d)); };
-        crse[c * Lc.S + q] = full_weight<T>(f, bI, bJ, bK);
-    }
+    const RestrictNode<T> r(Lf, Lc, I, J, K);
+    crse[c * Lc.S + Lc.idx(I, J, K)] = r(fine + c * Lf.S);
 }
 
-template <typename T> struct Pair;
-template <> struct Pair<float> { typedef float2 type; };
-template <> struct Pair<double> { typedef double2 type; };
-
-// Trilinear prolongation of the coarse correction.  A thread owns the fine
-// pair i = 2I, 2I+1 of one row (the even node takes the coarse value at I,
-// the odd one the mean with I+1), so a warp never splits on the parity of i;
-// the parities of j and k are uniform over a warp (one row per warp).  The
-// pair is read and written as one 8- or 16-byte vector (rows start on
-// 32-byte boundaries and 2I is even).  Each fine value is the same
-// expression, summed in the same order, as the per-node form
-// (Operator.cpp:365-434).
+// One coarse cell and component a thread.  129^3 -> 257^3 nodes, FP32, additive:
+// 72 us (a fine pair a thread, looping over the components: 175).
 template <typename T>
-__global__ void k_interp(LevelDesc Lf, LevelDesc Lc, T* __restrict__ fine, const T* __restrict__ crse, int assign)
+__global__ void __launch_bounds__(256) k_interp(LevelDesc Lf, LevelDesc Lc, T* __restrict__ fine,
+                                                const T* __restrict__ crse, int assign)
 {
     pdl_entry();
     const int I = blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = blockIdx.y * blockDim.y + threadIdx.y;
-    const int k = blockIdx.z * blockDim.z + threadIdx.z;
-    const int i = 2 * I;
-    if (i >= Lf.nn[0] || j >= Lf.nn[1] || k >= Lf.nn[2]) return;
-    const bool two = i + 1 < Lf.nn[0];
-    const int J = j >> 1, K = k >> 1;
-    const int I1 = wrapn(I + 1, Lc.n[0], Lc.per[0]), J1 = wrapn(J + 1, Lc.n[1], Lc.per[1]),
-              K1 = wrapn(K + 1, Lc.n[2], Lc.per[2]);
-    const bool ej = !(j & 1), ek = !(k & 1);
-    const long long q = Lf.idx(i, j, k);
-    const long long r00 = Lc.idx(0, J, K), r10 = Lc.idx(0, J1, K), r01 = Lc.idx(0, J, K1), r11 = Lc.idx(0, J1, K1);
-    for (int c = 0; c < 3; c++) {
-        const T* cs = crse + c * Lc.S;
-        // C(a, b, d): coarse value at (a ? I1 : I, b ? J1 : J, d ? K1 : K)
-        auto C = [&](int a, int b, int d) -> T {
-            const long long r = b ? (d ? r11 : r10) : (d ? r01 : r00);
-            return __ldg(cs + r + (a ? I1 : I));
-        };
-        T te, to = (T)0;
-        if (ej && ek) {
-            te = C(0, 0, 0);
-            if (two) to = (T)0.5 * (C(0, 0, 0) + C(1, 0, 0));
-        } else if (ek) {
-            te = (T)0.5 * (C(0, 0, 0) + C(0, 1, 0));
-            if (two) to = (T)0.25 * (C(0, 0, 0) + C(1, 0, 0) + C(0, 1, 0) + C(1, 1, 0));
-        } else if (ej) {
-            te = (T)0.5 * (C(0, 0, 0) + C(0, 0, 1));
-            if (two) to = (T)0.25 * (C(0, 0, 0) + C(0, 0, 1) + C(1, 0, 0) + C(1, 0, 1));
-        } else {
-            te = (T)0.25 * (C(0, 0, 0) + C(0, 1, 0) + C(0, 0, 1) + C(0, 1, 1));
-            if (two)
-                to = (T)0.125 * (C(0, 0, 0) + C(1, 0, 0) + C(0, 1, 0) + C(0, 0, 1) + C(0, 1, 1) + C(1, 0, 1) +
-                                 C(1, 1, 0) + C(1, 1, 1));
-        }
-        T* o = fine + c * Lf.S + q;
-        if (two) {
-            typedef typename Pair<T>::type V;
-            V v;
-            if (assign) {
-                v.x = te;
-                v.y = to;
-            } else {
-                v = *reinterpret_cast<const V*>(o);
-                v.x = v.x + te;
-                v.y = v.y + to;
-            }
-            *reinterpret_cast<V*>(o) = v;
-        } else {
-            *o = assign ? te : (*o + te);
-        }
-    }
+    const int J = blockIdx.y * blockDim.y + threadIdx.y;
+    const int c = blockIdx.z % 3, K = (blockIdx.z / 3) * blockDim.z + threadIdx.z;
+    if (I >= Lc.nn[0] || J >= Lc.nn[1] || K >= Lc.nn[2]) return;
+    const InterpCell<T> cell(Lf, Lc, I, J, K);
+    cell(crse + c * Lc.S, fine + c * Lf.S, assign != 0);
 }
 
 template <typename T>
@@ -136,18 +60,9 @@ __global__ void k_avg_ddw(LevelDesc Lf, LevelDesc Lc, const T* __restrict__ fine
     const int J = blockIdx.y * blockDim.y + threadIdx.y;
     const int K = blockIdx.z * blockDim.z + threadIdx.z;
     if (I >= Lc.nn[0] || J >= Lc.nn[1] || K >= Lc.nn[2]) return;
-    const bool bI = !Lc.per[0] && (I == 0 || I == Lc.n[0]);
-    const bool bJ = !Lc.per[1] && (J == 0 || J == Lc.n[1]);
-    const bool bK = !Lc.per[2] && (K == 0 || K == Lc.n[2]);
     const long long q = Lc.idx(I, J, K);
-    for (int m = 0; m < ncoef; m++) {
-        const T* src = fine + m * Lf.S;
-        auto f = [&](int a, int b, int d) -> T {
-            return src[Lf.idx(wrapn(2 * I + a, Lf.n[0], Lf.per[0]), wrapn(2 * J + b, Lf.n[1], Lf.per[1]),
-                              wrapn(2 * K + d, Lf.n[2], Lf.per[2]))];
-        };
-        crse[m * Lc.S + q] = full_weight<T>(f, bI, bJ, bK);
-    }
+    const RestrictNode<T> r(Lf, Lc, I, J, K);
+    for (int m = 0; m < ncoef; m++) crse[m * Lc.S + q] = r(fine + m * Lf.S);
 }
 
 template <typename TD, typename TS>
@@ -346,21 +261,30 @@ static inline int blocks_1d(long long n)
     return (int)(b < cap ? (b < 1 ? 1 : b) : cap);
 }
 
+// Blocks over the coarse nodes: 32-wide rows, 8 x 8 x 4 (and 8 x 4 x 2, which
+// spread over more SMs, on the smallest levels) where rows are short.
+static inline dim3 transfer_block(const LevelDesc& Lc)
+{
+    if (Lc.nn[0] > 20) return dim3(32, 4, 2);
+    return Lc.count() <= 1000 ? dim3(8, 4, 2) : dim3(8, 8, 4);
+}
+
 template <typename T>
 void launch_restriction(cudaStream_t st, const LevelDesc& Lf, const LevelDesc& Lc, const T* fine, T* crse, int ncomp)
 {
-    dim3 blk(32, 4, 2);
-    pdl_launch(k_restrict<T>, grid_for(Lc, blk), blk, 0, st, Lf, Lc, fine, crse, ncomp); count_launch();
+    const dim3 blk = transfer_block(Lc);
+    dim3 grd = grid_for(Lc, blk);
+    grd.z *= ncomp;
+    pdl_launch(k_restrict<T>, grd, blk, 0, st, Lf, Lc, fine, crse, ncomp); count_launch();
 }
 
 template <typename T>
 void launch_interpolation(cudaStream_t st, const LevelDesc& Lf, const LevelDesc& Lc, T* fine, const T* crse,
                           bool assign)
 {
-    dim3 blk(32, 4, 2);
-    // one thread per fine pair (2I, 2I+1) of a row
-    const dim3 grd(((Lf.nn[0] + 1) / 2 + blk.x - 1) / blk.x, (Lf.nn[1] + blk.y - 1) / blk.y,
-                   (Lf.nn[2] + blk.z - 1) / blk.z);
+    const dim3 blk = transfer_block(Lc);
+    dim3 grd = grid_for(Lc, blk);
+    grd.z *= 3;
     pdl_launch(k_interp<T>, grd, blk, 0, st, Lf, Lc, fine, crse, assign ? 1 : 0); count_launch();
 }
 
