@@ -56,10 +56,20 @@ struct BLevel {
     BProb* d_probs = nullptr;
     int shape = 0;
     std::vector<BTile> tS_smooth, t32_smooth, t32_full;
-    BTile *d_tS_smooth = nullptr, *d_t32_smooth = nullptr, *d_t32_full = nullptr;
+    BTile *d_tS_smooth = nullptr, *d_t32_full = nullptr;
     // the same lists restricted to the problems still iterating (compact()),
     // padded to full length with end markers (prob = -1); the cycle graphs use these
-    BTile *c_tS_smooth = nullptr, *c_t32_smooth = nullptr, *c_t32_full = nullptr;
+    BTile *c_tS_smooth = nullptr, *c_t32_full = nullptr;
+    // the same problems as segments, whole lists and compacted ones, with the
+    // number of segments of each (d_nseg: smooth, full, compacted smooth, compacted full)
+    std::vector<BSeg> seg_smooth, seg_full;
+    BSeg *d_seg_smooth = nullptr, *d_seg_full = nullptr, *c_seg_smooth = nullptr, *c_seg_full = nullptr;
+    int* d_nseg = nullptr;
+    BSegList segs_full(bool compacted) const
+    {
+        return BSegList{compacted ? c_seg_full : d_seg_full, d_nseg + (compacted ? 3 : 1), (int)seg_full.size()};
+    }
+    BSegList segs_smooth() const { return BSegList{c_seg_smooth, d_nseg + 2, (int)seg_smooth.size()}; }
     std::vector<int> bottoms;
     int* d_bottoms = nullptr;
     long long nvec = 0, ncoef = 0, nwork = 0;
@@ -96,6 +106,19 @@ void make_tiles(const std::vector<BProb>& probs, const std::vector<int>& which, 
         for (int z = 0; z < nz; z++)
             for (int y = 0; y < ny; y++)
                 for (int x = 0; x < nx; x++) out.push_back(BTile{p, (short)x, (short)y, (short)z, 0});
+    }
+}
+
+void make_segs(const std::vector<BProb>& probs, const std::vector<int>& which, std::vector<BSeg>& out)
+{
+    out.clear();
+    for (int p : which) {
+        const LevelDesc& L = probs[p].L;
+        const long long n = (long long)L.P * L.nn[1] * L.nn[2];   // a multiple of 8
+        for (int c = 0; c < 3; c++)
+            for (long long e = 0; e < n; e += BSEG)
+                out.push_back(BSeg{probs[p].vo + c * L.S + e, (int)std::min<long long>(BSEG, n - e), p, c, (int)e, L.P,
+                                   L.nn[0]});
     }
 }
 
@@ -201,12 +224,11 @@ template <typename T> struct BEngine {
     {
         BLevel& v = b->lev[l];
         if (ns <= 0 || v.tS_smooth.empty()) {
-            launch_batch_vec(b->st, BV_ZERO, b->grid, v.d_probs, v.c_t32_smooth, (int)v.t32_smooth.size(), act, x,
-                             nullptr, 0.0, nullptr, fp32);
+            launch_batch_vec(b->st, BV_ZERO, b->grid, v.segs_smooth(), act, x, nullptr, 0.0, nullptr, fp32);
             return;
         }
-        launch_batch_vec(b->st, BV_JACOBI0, b->grid, v.d_probs, v.c_t32_smooth, (int)v.t32_smooth.size(), act,
-                         A::tmp(v), rhs, b->omega, nullptr, fp32, A::dinv(v));
+        launch_batch_vec(b->st, BV_JACOBI0, b->grid, v.segs_smooth(), act, A::tmp(v), rhs, b->omega, nullptr, fp32,
+                         A::dinv(v));
         launch_batch_stencil<T>(b->st, b->sym, MODE_JACOBI, v.shape, b->grid, v.d_probs, v.c_tS_smooth,
                                 (int)v.tS_smooth.size(), act, b->bc, false, A::ddw(v), A::tmp(v), rhs, A::dinv(v), x,
                                 (T)b->omega, nullptr);
@@ -256,15 +278,20 @@ template <typename T> struct BEngine {
     // that level on the residual of it, and the sum.  The roles of res/rescor
     // and cor/hold are swapped around the V-cycle instead of copying, and
     // swapped back (the captured graph replays from the same roles).
-    void fcycle()
+    // The residual is `top` on level 0, which is left as it is.  A problem whose
+    // only level is level 0 has its residual copied to where bottom() reads it.
+    void fcycle(const T* top)
     {
         const int L = b->Lmax;
+        if (!b->lev[0].bottoms.empty())
+            launch_batch_vec(b->st, BV_COPY, b->grid, b->lev[0].segs_full(true), act, A::res(b->lev[0]), top, 0.0,
+                             nullptr, 1);
         for (int l = 0; l + 1 < L; l++) {
             BLevel& v = b->lev[l];
             if (v.t32_smooth.empty()) continue;
             BLevel& c = b->lev[l + 1];
             launch_batch_transfer<T>(b->st, 1, false, b->grid, v.d_probs, c.d_probs, c.c_t32_full,
-                                     (int)c.t32_full.size(), act, A::res(v), A::res(c));
+                                     (int)c.t32_full.size(), act, l ? A::res(v) : top, A::res(c));
         }
         for (int l = 0; l < L; l++)
             if (!b->lev[l].bottoms.empty()) bottom(l);
@@ -275,13 +302,12 @@ template <typename T> struct BEngine {
             launch_batch_transfer<T>(b->st, 0, true, b->grid, v.d_probs, c.d_probs, c.c_t32_full,
                                      (int)c.t32_full.size(), act, A::cor(c), A::cor(v));
             launch_batch_stencil<T>(b->st, b->sym, MODE_RESID, v.shape, b->grid, v.d_probs, v.c_tS_smooth,
-                                    (int)v.tS_smooth.size(), act, b->bc, false, A::ddw(v), A::cor(v), A::res(v),
-                                    nullptr, A::rescor(v), (T)0, nullptr);
+                                    (int)v.tS_smooth.size(), act, b->bc, false, A::ddw(v), A::cor(v),
+                                    l ? A::res(v) : top, nullptr, A::rescor(v), (T)0, nullptr);
             std::swap(v.res32, v.rescor32);
             std::swap(v.cor32, v.hold32);
             vcycle_from(l, true);
-            launch_batch_vec(b->st, BV_AXPY, b->grid, v.d_probs, v.c_t32_smooth, (int)v.t32_smooth.size(), act,
-                             v.hold32, v.cor32, 1.0, nullptr, 1);
+            launch_batch_vec(b->st, BV_AXPY, b->grid, v.segs_smooth(), act, v.hold32, v.cor32, 1.0, nullptr, 1);
             std::swap(v.res32, v.rescor32);
             std::swap(v.cor32, v.hold32);
         }
@@ -341,8 +367,17 @@ agb_status build_levels(agb_batch b)
         v.tS_smooth = v.t32_smooth;
         BTRY(b->upload_vec(v.probs, &v.d_probs));
         BTRY(b->upload_vec(v.t32_full, &v.d_t32_full));
-        BTRY(b->upload_vec(v.t32_smooth, &v.d_t32_smooth));
         BTRY(b->upload_vec(v.tS_smooth, &v.d_tS_smooth));
+        make_segs(v.probs, full, v.seg_full);
+        make_segs(v.probs, smooth, v.seg_smooth);
+        BTRY(b->upload_vec(v.seg_full, &v.d_seg_full));
+        BTRY(b->upload_vec(v.seg_smooth, &v.d_seg_smooth));
+        BTRY(b->alloc(&v.c_seg_full, v.seg_full.size()));
+        BTRY(b->alloc(&v.c_seg_smooth, v.seg_smooth.size()));
+        const std::vector<int> nseg = {(int)v.seg_smooth.size(), (int)v.seg_full.size(), (int)v.seg_smooth.size(),
+                                       (int)v.seg_full.size()};
+        BTRY(b->upload_vec(nseg, &v.d_nseg));
+        BCK(cudaStreamSynchronize(b->st));   // nseg is this scope's
         BTRY(b->upload_vec(v.bottoms, &v.d_bottoms));
         BTRY(b->alloc(&v.ddw64, v.ncoef));
         BTRY(b->alloc(&v.diag64, v.nvec));
@@ -463,7 +498,6 @@ agb_status autotune(agb_batch b)
     }
     for (auto& v : b->lev) {
         BTRY(b->alloc(&v.c_t32_full, v.t32_full.size()));
-        BTRY(b->alloc(&v.c_t32_smooth, v.t32_smooth.size()));
         BTRY(b->alloc(&v.c_tS_smooth, v.tS_smooth.size()));
     }
     b->compact_tiles = -1;
@@ -495,10 +529,22 @@ agb_status compact(agb_batch b, const std::vector<int>& mask)
         BCK(cudaStreamSynchronize(b->st));
         return AGB_OK;
     };
+    std::vector<BSeg> hs;
+    auto put_seg = [&](const std::vector<BSeg>& full, BSeg* d, int* n) -> agb_status {
+        hs.clear();
+        for (const BSeg& s : full)
+            if (mask[s.prob]) hs.push_back(s);
+        const int count = (int)hs.size();
+        if (count) BCK(cudaMemcpyAsync(d, hs.data(), hs.size() * sizeof(BSeg), cudaMemcpyHostToDevice, b->st));
+        BCK(cudaMemcpyAsync(n, &count, sizeof(int), cudaMemcpyHostToDevice, b->st));
+        BCK(cudaStreamSynchronize(b->st));   // hs and count are reused
+        return AGB_OK;
+    };
     for (auto& v : b->lev) {
         BTRY(put(v.t32_full, v.c_t32_full));
-        BTRY(put(v.t32_smooth, v.c_t32_smooth));
         BTRY(put(v.tS_smooth, v.c_tS_smooth));
+        BTRY(put_seg(v.seg_smooth, v.c_seg_smooth, v.d_nseg + 2));
+        BTRY(put_seg(v.seg_full, v.c_seg_full, v.d_nseg + 3));
     }
     b->compact_tiles = keep;
     b->compact_mask = mask;
@@ -515,11 +561,10 @@ agb_status compact(agb_batch b, const std::vector<int>& mask)
 template <typename T> void project(agb_batch b, const int* act, T* y, bool norms, bool compacted = false)
 {
     BLevel& v = b->lev[0];
-    const BTile* tl = compacted ? v.c_t32_full : v.d_t32_full;
+    const BSegList segs = v.segs_full(compacted);
     cudaMemsetAsync(b->sums, 0, sizeof(double) * 3 * b->np, b->st);
-    launch_batch_mean3<T>(b->st, b->grid, v.d_probs, tl, (int)v.t32_full.size(), act, y, b->sums, 0);
-    launch_batch_mean3<T>(b->st, b->grid, v.d_probs, tl, (int)v.t32_full.size(), act, y, b->sums, 1,
-                          norms ? (void*)b->d_norms : nullptr);
+    launch_batch_mean3<T>(b->st, b->grid, v.d_probs, segs, act, y, b->sums, 0);
+    launch_batch_mean3<T>(b->st, b->grid, v.d_probs, segs, act, y, b->sums, 1, norms ? (void*)b->d_norms : nullptr);
 }
 
 // compacted: use the lists of the problems still iterating (inside the cycle graphs)
@@ -577,51 +622,52 @@ template <class Fn> agb_status bcapture(agb_batch b, cudaGraphExec_t* out, long 
 }
 
 // One GCR iteration of every problem still iterating (d_iactive), with k
-// directions stored: z = V(r) (the batched FP32 V-cycle on res32(0), which it
-// leaves unchanged), w = A z (projected on fully periodic problems), w and z
-// orthogonalised against the stored directions, and the residual minimised
-// over the new one; max |r| per problem into the norm slots (FP32 encoding).
+// directions stored: z = M(r) (the batched FP32 cycle on kr32, which it leaves
+// unchanged, straight into the direction's array), w = A z (projected on fully
+// periodic problems), w and z orthogonalised against the stored directions,
+// and the residual minimised over the new one; max |r| per problem into the
+// norm slots (FP32 encoding).  dots holds <w, w> and <w, r> of every direction.
 void gcr_iter_body(agb_batch b, int k)
 {
     BLevel& v0 = b->lev[0];
     const int* act = b->d_iactive;
     const int np = b->np;
     BEngine<float> E{b, act};
-    launch_batch_vec(b->st, BV_COPY, b->grid, v0.d_probs, v0.c_t32_full, (int)v0.t32_full.size(), act, v0.res32,
-                     b->kr32, 0.0, nullptr, 1);
-    if (b->p.max_fmg_iter > 0) E.fcycle();
-    else E.vcycle();
     float* z = b->kZ[k];
     float* w = b->kW[k];
-    launch_batch_vec(b->st, BV_COPY, b->grid, v0.d_probs, v0.c_t32_full, (int)v0.t32_full.size(), act, z, v0.cor32,
-                     0.0, nullptr, 1);
+    // the cycle's correction is z, its residual kr32
+    float *cor = v0.cor32, *res = v0.res32;
+    v0.cor32 = z;
+    if (b->p.max_fmg_iter > 0) {
+        E.fcycle(b->kr32);
+    } else {
+        v0.res32 = b->kr32;   // a V-cycle only reads it
+        E.vcycle();
+    }
+    v0.cor32 = cor;
+    v0.res32 = res;
+    const BSegList segs = v0.segs_full(true);
     int shape, nt;
     const BTile* tl;
     fine_tiles(b, true, &shape, &tl, &nt);
     launch_batch_stencil<float>(b->st, b->sym, MODE_APPLY, shape, b->grid, v0.d_probs, tl, nt, act, b->bc, false,
                                 v0.ddw32, z, nullptr, nullptr, w, 0.0f, nullptr);
     if (b->per[0] && b->per[1] && b->per[2]) project<float>(b, act, w, false, true);
-    cudaMemsetAsync(b->kdots, 0, sizeof(double) * (size_t)np * GCR_MAX, b->st);
-    cudaMemsetAsync(b->kd2, 0, sizeof(double) * (size_t)np * 2, b->st);
-    if (k > 0) {
-        GcrVecs W, Z;
-        for (int i = 0; i < k; i++) {
-            W.v[i] = b->kW[i];
-            Z.v[i] = b->kZ[i];
-        }
-        launch_batch_multidot(b->st, b->grid, v0.d_probs, v0.c_t32_full, (int)v0.t32_full.size(), act, k, w, W,
-                              v0.dinv32, b->kdots, GCR_MAX);
-        launch_batch_gcr_orth(b->st, b->grid, v0.d_probs, v0.c_t32_full, (int)v0.t32_full.size(), act, k, b->kdots,
-                              GCR_MAX, W, Z, w, z);
+    double* dots = b->kd2 + (size_t)k * np * 2;
+    cudaMemsetAsync(dots, 0, sizeof(double) * (size_t)np * 2, b->st);
+    GcrVecs W, Z;
+    for (int i = 0; i < k; i++) {
+        W.v[i] = b->kW[i];
+        Z.v[i] = b->kZ[i];
     }
-    GcrVecs P;
-    P.v[0] = w;
-    P.v[1] = b->kr32;
-    launch_batch_multidot(b->st, b->grid, v0.d_probs, v0.c_t32_full, (int)v0.t32_full.size(), act, 2, w, P,
-                          v0.dinv32, b->kd2, 2);
+    if (k > 0) {
+        cudaMemsetAsync(b->kdots, 0, sizeof(double) * (size_t)np * GCR_MAX, b->st);
+        launch_batch_multidot(b->st, b->grid, segs, act, k, w, W, v0.dinv32, b->kdots, GCR_MAX);
+    }
+    launch_batch_gcr_orth(b->st, b->grid, segs, act, k, b->kdots, GCR_MAX, b->kd2, np, W, Z, w, z, b->kr32, v0.dinv32,
+                          dots);
     cudaMemsetAsync(b->d_norms, 0, sizeof(double) * np, b->st);
-    launch_batch_gcr_step(b->st, b->grid, v0.d_probs, v0.c_t32_full, (int)v0.t32_full.size(), act, b->kd2, w, z,
-                          b->sol32, b->kr32, b->d_norms);
+    launch_batch_gcr_step(b->st, b->grid, segs, act, dots, w, z, b->sol32, b->kr32, b->d_norms);
     cudaMemcpyAsync(b->h_norms, b->d_norms, sizeof(double) * np, cudaMemcpyDeviceToHost, b->st);
 }
 
@@ -640,7 +686,7 @@ agb_status gcr_setup(agb_batch b, int m)
     }
     if (!b->kdots) {
         BTRY(b->alloc(&b->kdots, (size_t)b->np * GCR_MAX));
-        BTRY(b->alloc(&b->kd2, (size_t)b->np * 2));
+        BTRY(b->alloc(&b->kd2, (size_t)b->np * 2 * GCR_MAX));
         BTRY(b->alloc(&b->kr32, v0.nvec));
     }
     b->gk.resize(m, nullptr);
@@ -802,8 +848,8 @@ agb_status agb_batch_solve(agb_batch b, double tol_rel, double tol_abs, agb_solv
             BTRY(bcapture(b, &b->g64, &b->g64_k, [&] {
                 BEngine<double> E{b, b->d_active};
                 E.vcycle();
-                launch_batch_vec(b->st, BV_AXPY, b->grid, v0.d_probs, v0.c_t32_full, (int)v0.t32_full.size(),
-                                 b->d_active, b->x64, v0.cor64, 1.0, nullptr, 0);
+                launch_batch_vec(b->st, BV_AXPY, b->grid, v0.segs_full(true), b->d_active, b->x64, v0.cor64, 1.0,
+                                 nullptr, 0);
                 residual0<double>(b, b->d_active, b->x64, b->b64, v0.res64, true);
             }));
         for (int it = 0; it < b->p.max_iter && any(b->active); it++) {
@@ -825,8 +871,8 @@ agb_status agb_batch_solve(agb_batch b, double tol_rel, double tol_abs, agb_solv
             BTRY(bcapture(b, &b->g32, &b->g32_k, [&] {
                 BEngine<float> E{b, b->d_iactive};
                 E.vcycle();
-                launch_batch_vec(b->st, BV_AXPY, b->grid, v0.d_probs, v0.c_t32_full, (int)v0.t32_full.size(),
-                                 b->d_iactive, b->sol32, v0.cor32, 1.0, nullptr, 1);
+                launch_batch_vec(b->st, BV_AXPY, b->grid, v0.segs_full(true), b->d_iactive, b->sol32, v0.cor32, 1.0,
+                                 nullptr, 1);
                 residual0<float>(b, b->d_iactive, b->sol32, b->rhs32, v0.res32, true);
             }));
         const int m = std::min(std::max(b->p.krylov, 0), GCR_MAX);
@@ -841,12 +887,12 @@ agb_status agb_batch_solve(agb_batch b, double tol_rel, double tol_abs, agb_solv
             }
             BCK(cudaMemcpyAsync(b->scale, scale.data(), sizeof(double) * np, cudaMemcpyHostToDevice, b->st));
             BCK(cudaMemcpyAsync(b->d_iactive, b->iactive.data(), sizeof(int) * np, cudaMemcpyHostToDevice, b->st));
-            launch_batch_vec(b->st, BV_SCALE_TO32, b->grid, v0.d_probs, v0.d_t32_full, (int)v0.t32_full.size(),
-                             b->d_active, b->rhs32, v0.res64, 0.0, b->scale, 1);
-            launch_batch_vec(b->st, BV_COPY, b->grid, v0.d_probs, v0.d_t32_full, (int)v0.t32_full.size(), b->d_active,
-                             m > 0 ? b->kr32 : v0.res32, b->rhs32, 0.0, nullptr, 1);
-            launch_batch_vec(b->st, BV_ZERO, b->grid, v0.d_probs, v0.d_t32_full, (int)v0.t32_full.size(), b->d_active,
-                             b->sol32, nullptr, 0.0, nullptr, 1);
+            launch_batch_vec(b->st, BV_SCALE_TO32, b->grid, v0.segs_full(false), b->d_active, b->rhs32, v0.res64, 0.0,
+                             b->scale, 1);
+            launch_batch_vec(b->st, BV_COPY, b->grid, v0.segs_full(false), b->d_active, m > 0 ? b->kr32 : v0.res32,
+                             b->rhs32, 0.0, nullptr, 1);
+            launch_batch_vec(b->st, BV_ZERO, b->grid, v0.segs_full(false), b->d_active, b->sol32, nullptr, 0.0, nullptr,
+                             1);
             std::vector<int> slow(np, 0);
             for (int it = 0; it < b->p.inner_max_iter && any(b->iactive); it++) {
                 BTRY(compact(b, b->iactive));
@@ -872,8 +918,8 @@ agb_status agb_batch_solve(agb_batch b, double tol_rel, double tol_abs, agb_solv
                 }
                 BCK(cudaMemcpyAsync(b->d_iactive, b->iactive.data(), sizeof(int) * np, cudaMemcpyHostToDevice, b->st));
             }
-            launch_batch_vec(b->st, BV_ACC_FROM32, b->grid, v0.d_probs, v0.d_t32_full, (int)v0.t32_full.size(),
-                             b->d_active, b->x64, b->sol32, 0.0, b->scale, 0);
+            launch_batch_vec(b->st, BV_ACC_FROM32, b->grid, v0.segs_full(false), b->d_active, b->x64, b->sol32, 0.0,
+                             b->scale, 0);
             BTRY(residual0<double>(b, b->d_active, b->x64, b->b64, v0.res64));
             BCK(cudaStreamSynchronize(b->st));
             for (int q = 0; q < np; q++) {

@@ -139,6 +139,22 @@ struct BTile {
     short pad;
 };
 
+// A run of consecutive elements of one component of one problem (up to BSEG,
+// a multiple of 8), for the elementwise and reducing kernels.
+constexpr int BSEG = 4096;
+struct BSeg {
+    long long base;     // first element in the level arena
+    int count;
+    int prob, comp;
+    int first;          // its place in the component
+    int pitch, row;     // row pitch, nodes of a row
+};
+struct BSegList {
+    const BSeg* d;
+    const int* n;       // segments in the list (on the device: compacted lists shrink)
+    int max;            // at most
+};
+
 enum BatchVecOp { BV_ZERO = 0, BV_COPY = 1, BV_AXPY = 2, BV_SCALE_TO32 = 3, BV_ACC_FROM32 = 4, BV_JACOBI0 = 5 };
 
 template <typename T>
@@ -152,9 +168,8 @@ void launch_batch_avg_ddw(cudaStream_t st, int grid, const BProb* pf, const BPro
                           const double* fine, double* crse, int ncoef);
 void launch_batch_diag(cudaStream_t st, int sym, int grid, const BProb* probs, const BTile* tiles, int ntiles,
                        const BCTable& bc, const double* ddw, double* diag, double* dinv64, float* dinv32);
-void launch_batch_vec(cudaStream_t st, int op, int grid, const BProb* probs, const BTile* tiles, int ntiles,
-                      const int* active, void* y, const void* x, double a, const double* scale, int fp32,
-                      const void* x2 = nullptr);
+void launch_batch_vec(cudaStream_t st, int op, int grid, BSegList segs, const int* active, void* y, const void* x,
+                      double a, const double* scale, int fp32, const void* x2 = nullptr);
 void launch_batch_bottom(cudaStream_t st, int sym, int fp32, const BProb* probs, const int* plist, int np,
                          const int* active, const BCTable& bc, bool uniform, const void* ddw, const double* diag,
                          void* cor, const void* res, double* work, int maxiter, double tol_rel, double tol_abs, int nub,
@@ -167,22 +182,20 @@ void launch_batch_mean_stress(cudaStream_t st, int sym, int grid, const BProb* p
 // problem, zeroed by the caller), or (subtract) y -= sums / count, with the
 // per-problem max |y| after it into norm_slots when given
 template <typename T>
-void launch_batch_mean3(cudaStream_t st, int grid, const BProb* probs, const BTile* tiles, int ntiles,
-                        const int* active, T* y, double* sums, int subtract, void* norm_slots = nullptr);
+void launch_batch_mean3(cudaStream_t st, int grid, const BProb* probs, BSegList segs, const int* active, T* y,
+                        double* sums, int subtract, void* norm_slots = nullptr);
 int batch_shape_count();
 void batch_shape_dims(int shape, int dims[3]);
-// Per-problem GCR over the batched FP32 cycle (kernels_batch.cu; GcrVecs
-// and GCR_MAX as for the single-box inner GCR).  Tiles: the 32 x 4 x 2 lists.
+// Per-problem GCR over the batched FP32 cycle (kernels_batch.cu; GcrVecs and
+// GCR_MAX as for the single-box inner GCR).
 struct GcrVecs;
-void launch_batch_multidot(cudaStream_t st, int grid, const BProb* probs, const BTile* tiles, int ntiles,
-                           const int* active, int k, const float* x, const GcrVecs& V, const float* d, double* out,
-                           int stride);
-void launch_batch_gcr_orth(cudaStream_t st, int grid, const BProb* probs, const BTile* tiles, int ntiles,
-                           const int* active, int k, const double* beta, int stride, const GcrVecs& W,
-                           const GcrVecs& Z, float* w, float* z);
-void launch_batch_gcr_step(cudaStream_t st, int grid, const BProb* probs, const BTile* tiles, int ntiles,
-                           const int* active, const double* dots, float* w, float* z, float* c, float* r,
-                           void* norm_slots);
+void launch_batch_multidot(cudaStream_t st, int grid, BSegList segs, const int* active, int k, const float* x,
+                           const GcrVecs& V, const float* d, double* out, int stride);
+void launch_batch_gcr_orth(cudaStream_t st, int grid, BSegList segs, const int* active, int k, const double* beta,
+                           int stride, const double* all, int np, const GcrVecs& W, const GcrVecs& Z, float* w,
+                           float* z, const float* r, const float* d, double* dots);
+void launch_batch_gcr_step(cudaStream_t st, int grid, BSegList segs, const int* active, const double* dots,
+                           const float* w, const float* z, float* c, float* r, void* norm_slots);
 // whether stencil tile shape `shape` serves batches of this symmetry and periodicity
 bool batch_shape_ok(int shape, int sym, const int per[3]);
 

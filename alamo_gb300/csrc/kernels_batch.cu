@@ -15,6 +15,7 @@
 #include <algorithm>
 #include <cstdlib>
 #include <mutex>
+#include <type_traits>
 #include <unordered_map>
 
 #include "agb_internal.h"
@@ -618,7 +619,37 @@ __global__ void __launch_bounds__(256) k_batch_diag(const BProb* __restrict__ pr
     }
 }
 
-// Per-node vector operations over the listed problems (3 components).
+// ---------------------------------------------------------------------------
+// Elementwise and reducing kernels over segments: runs of up to BSEG
+// consecutive elements of one component of one problem (padded rows included:
+// padding is zero in every vector and stays zero).  A CTA takes a contiguous
+// part of the list, so its segments mostly belong to one problem and its sums
+// go out once; a thread has four 16-byte vectors of every array in flight.
+// The node tiles these kernels used before cost a chain of dependent loads (tile,
+// problem, node) for 256 nodes, and their per-problem scalars were FP64 roots
+// and divisions in every thread; here one thread makes them once a problem.
+// Bound by HBM.  48 RVEs (17.3 M nodes), finest level, us before and now: GCR
+// step 872 and 175, the sums and the subtraction of the FP32 zero-mean
+// projection 305 and 37, 305 and 75; the solve 160 to 128 ms with the copies
+// around the cycle gone.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ void seg_range(const BSegList& list, int& s0, int& s1)
+{
+    const long long n = *list.n;
+    s0 = (int)(n * blockIdx.x / gridDim.x);
+    s1 = (int)(n * (blockIdx.x + 1) / gridDim.x);
+}
+
+// f(element offset, q): every vector of VE elements of a segment, q = 0 .. per thread
+template <int VE, class F> __device__ __forceinline__ void seg_each(const BSeg& s, const F& f)
+{
+#pragma unroll
+    for (int q = 0; q < BSEG / (256 * VE); q++) {
+        const int e = (threadIdx.x + 256 * q) * VE;
+        if (e < s.count) f(s.base + e);
+    }
+}
+
 //   BV_ZERO        y = 0
 //   BV_COPY        y = x
 //   BV_AXPY        y += a x
@@ -627,42 +658,169 @@ __global__ void __launch_bounds__(256) k_batch_diag(const BProb* __restrict__ pr
 //   BV_JACOBI0     y = a (x * x2): the first damped-Jacobi sweep from a zero
 //                  guess (x the right-hand side, x2 = 1/D, a = omega), the
 //                  sweep kernels' expression with A 0 = 0
-__global__ void __launch_bounds__(256) k_batch_vec(int op, const BProb* __restrict__ probs,
-                                                   const BTile* __restrict__ tiles, int ntiles,
-                                                   const int* __restrict__ active, void* y, const void* x, double a,
-                                                   const double* __restrict__ scale, int fp32, const void* x2)
+template <int OP, typename T>
+__global__ void __launch_bounds__(256) k_seg_vec(BSegList list, const int* __restrict__ active, void* yv,
+                                                 const void* xv, double a, const double* __restrict__ scale,
+                                                 const void* x2v)
 {
-    for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
-        const BTile tl = tiles[t];
-        if (tl.prob < 0) break;   // compacted list: only end markers follow (uniform over the CTA)
-        if (active && !active[tl.prob]) continue;
-        const BProb& P = probs[tl.prob];
-        int i, j, k;
-        if (!tile_node<32, 4, 2>(tl, P.L, i, j, k)) continue;
-        const long long q0 = P.vo + P.L.idx(i, j, k);
-        for (int c = 0; c < 3; c++) {
-            const long long q = q0 + c * P.L.S;
-            if (op == BV_SCALE_TO32) {
-                ((float*)y)[q] = (float)(((const double*)x)[q] / scale[tl.prob]);
-            } else if (op == BV_ACC_FROM32) {
-                ((double*)y)[q] += (double)((const float*)x)[q] * scale[tl.prob];
-            } else if (fp32) {
-                float* yy = (float*)y;
-                const float* xx = (const float*)x;
-                if (op == BV_ZERO) yy[q] = 0.f;
-                else if (op == BV_COPY) yy[q] = xx[q];
-                else if (op == BV_JACOBI0) yy[q] = (float)a * (xx[q] * ((const float*)x2)[q]);
-                else yy[q] += (float)a * xx[q];
-            } else {
-                double* yy = (double*)y;
-                const double* xx = (const double*)x;
-                if (op == BV_ZERO) yy[q] = 0.0;
-                else if (op == BV_COPY) yy[q] = xx[q];
-                else if (op == BV_JACOBI0) yy[q] = a * (xx[q] * ((const double*)x2)[q]);
-                else yy[q] += a * xx[q];
+    int s0, s1;
+    seg_range(list, s0, s1);
+    int prob = -1;
+    double sc = 1.0;   // 1 / scale or scale of the current problem (an FP64 division a problem, not an element)
+    for (int t = s0; t < s1; t++) {
+        const BSeg s = list.d[t];
+        if (active && !active[s.prob]) continue;   // uniform over the CTA
+        if constexpr (OP == BV_SCALE_TO32 || OP == BV_ACC_FROM32) {
+            if (s.prob != prob) {
+                prob = s.prob;
+                sc = OP == BV_SCALE_TO32 ? 1.0 / scale[prob] : scale[prob];
             }
+            seg_each<2>(s, [&](long long e) {
+                if (OP == BV_SCALE_TO32) {
+                    const double2 x = *reinterpret_cast<const double2*>((const double*)xv + e);
+                    *reinterpret_cast<float2*>((float*)yv + e) = make_float2((float)(x.x * sc), (float)(x.y * sc));
+                } else {
+                    const float2 x = *reinterpret_cast<const float2*>((const float*)xv + e);
+                    double2* y = reinterpret_cast<double2*>((double*)yv + e);
+                    double2 v = *y;
+                    v.x += (double)x.x * sc;
+                    v.y += (double)x.y * sc;
+                    *y = v;
+                }
+            });
+        } else if constexpr (sizeof(T) == 4) {
+            const float f = (float)a;
+            seg_each<4>(s, [&](long long e) {
+                float4* y = reinterpret_cast<float4*>((float*)yv + e);
+                float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (OP != BV_ZERO) {
+                    const float4 x = *reinterpret_cast<const float4*>((const float*)xv + e);
+                    if (OP == BV_COPY) v = x;
+                    else if (OP == BV_JACOBI0) {
+                        const float4 d = *reinterpret_cast<const float4*>((const float*)x2v + e);
+                        v = make_float4(f * (x.x * d.x), f * (x.y * d.y), f * (x.z * d.z), f * (x.w * d.w));
+                    } else {
+                        v = *y;
+                        v = make_float4(v.x + f * x.x, v.y + f * x.y, v.z + f * x.z, v.w + f * x.w);
+                    }
+                }
+                *y = v;
+            });
+        } else {
+            seg_each<2>(s, [&](long long e) {
+                double2* y = reinterpret_cast<double2*>((double*)yv + e);
+                double2 v = make_double2(0.0, 0.0);
+                if (OP != BV_ZERO) {
+                    const double2 x = *reinterpret_cast<const double2*>((const double*)xv + e);
+                    if (OP == BV_COPY) v = x;
+                    else if (OP == BV_JACOBI0) {
+                        const double2 d = *reinterpret_cast<const double2*>((const double*)x2v + e);
+                        v = make_double2(a * (x.x * d.x), a * (x.y * d.y));
+                    } else {
+                        v = *y;
+                        v = make_double2(v.x + a * x.x, v.y + a * x.y);
+                    }
+                }
+                *y = v;
+            });
         }
     }
+}
+
+// Sum over the CTA of K values a thread (every thread calls it); the totals,
+// added in FP64, are left in out[0 .. K) of shared memory.
+template <int K> __device__ __forceinline__ void seg_reduce(const double (&v)[K], double (&red)[K][8], double* out)
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int i = 0; i < K; i++) {
+        double t = v[i];
+        for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+        if (lane == 0) red[i][warp] = t;
+    }
+    __syncthreads();
+    if (threadIdx.x < K) {
+        double t = 0;
+        for (int w = 0; w < 8; w++) t += red[threadIdx.x][w];
+        out[threadIdx.x] = t;
+    }
+    __syncthreads();
+}
+
+__device__ __forceinline__ unsigned int abs_bits(float v) { return __float_as_uint(v) & 0x7fffffffu; }
+__device__ __forceinline__ unsigned long long abs_bits(double v)
+{
+    return (unsigned long long)__double_as_longlong(v) & 0x7fffffffffffffffull;
+}
+__device__ __forceinline__ float as_value(unsigned int b) { return __uint_as_float(b); }
+__device__ __forceinline__ double as_value(unsigned long long b) { return __longlong_as_double((long long)b); }
+
+// Per-problem component sums (sums[3 prob + c]), or with subtract y -= sums /
+// count over the nodes (not the padding), and the per-problem max |y| after it.
+// A thread's sums over its few elements are in T.
+template <typename T, int SUB>
+__global__ void __launch_bounds__(256) k_seg_mean3(const BProb* __restrict__ probs, BSegList list,
+                                                   const int* __restrict__ active, T* __restrict__ y,
+                                                   double* __restrict__ sums, void* norm_slots)
+{
+    constexpr int VE = 16 / sizeof(T);
+    typedef typename std::conditional<sizeof(T) == 4, float4, double2>::type V;
+    typedef decltype(abs_bits(T())) Bits;
+    __shared__ double red[1][8], tot[1];
+    __shared__ T mean_s;
+    int s0, s1;
+    seg_range(list, s0, s1);
+    T acc = 0, mean = 0;
+    Bits m = 0;   // max |y| by its bits: order-preserving for |y|, NaN above all, and no FP64 compare
+    int prob = -1, comp = -1;
+    auto flush = [&]() {   // every thread of the CTA together
+        if (prob < 0) return;
+        if (SUB) {
+            if (norm_slots) tile_max<T>(as_value(m), norm_slots, prob);
+        } else {
+            const double v[1] = {(double)acc};
+            seg_reduce<1>(v, red, tot);
+            if (threadIdx.x == 0) atomicAdd(&sums[prob * 3 + comp], tot[0]);
+        }
+        acc = 0;
+        m = 0;
+    };
+    for (int t = s0; t < s1; t++) {
+        const BSeg s = list.d[t];
+        if (active && !active[s.prob]) continue;
+        if (s.prob != prob || s.comp != comp) {
+            flush();
+            prob = s.prob;
+            comp = s.comp;
+            if (SUB) {
+                __syncthreads();
+                if (threadIdx.x == 0) mean_s = (T)(sums[prob * 3 + comp] / (double)probs[prob].L.count());
+                __syncthreads();
+                mean = mean_s;
+            }
+        }
+        const int P = s.pitch, nn0 = s.row;
+        seg_each<VE>(s, [&](long long e) {
+            V* p = reinterpret_cast<V*>(y + e);
+            V v = *p;
+            T* w = reinterpret_cast<T*>(&v);
+            if (!SUB) {
+#pragma unroll
+                for (int i = 0; i < VE; i++) acc += w[i];
+                return;
+            }
+            const int i0 = P == nn0 ? 0 : (int)((s.first + (e - s.base)) % P);   // VE divides the pitch
+#pragma unroll
+            for (int i = 0; i < VE; i++)
+                if (i0 + i < nn0) {
+                    w[i] -= mean;
+                    const Bits a = abs_bits(w[i]);
+                    m = a > m ? a : m;
+                }
+            *p = v;
+        });
+    }
+    flush();
 }
 
 // ---------------------------------------------------------------------------
@@ -966,88 +1124,20 @@ __global__ void __launch_bounds__(256) k_batch_mean_stress(const BProb* __restri
     }
 }
 
-// per-problem component sums over the stored nodes (sums[prob*3 + c]); with
-// `subtract`, y -= sums/count instead
 template <typename T>
-__global__ void __launch_bounds__(256) k_batch_mean3(const BProb* __restrict__ probs, const BTile* __restrict__ tiles,
-                                                     int ntiles, const int* __restrict__ active, T* __restrict__ y,
-                                                     double* __restrict__ sums, int subtract, void* norm_slots)
+void launch_batch_mean3(cudaStream_t st, int grid, const BProb* probs, BSegList segs, const int* active, T* y,
+                        double* sums, int subtract, void* norm_slots)
 {
-    // A CTA visits tiles t, t + gridDim.x, ...; tiles are ordered by problem, so
-    // consecutive visits mostly stay in one problem.  Each thread accumulates
-    // its sums (or its max |y|) while the problem stays the same, and the CTA
-    // reduces and flushes them with one atomic per value when it changes.
-    __shared__ double red[3][8];
-    T s0 = 0, s1 = 0, s2 = 0;   // a thread's sums over its few nodes of one problem, in T
-    T m = 0;
-    T mean[3] = {0, 0, 0};      // subtract: the current problem's means (one division per problem change)
-    int cur = -1;
-    auto flush = [&]() {   // called by every thread of the CTA together
-        if (cur < 0) return;
-        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-        if (subtract) {
-            if (norm_slots) tile_max<T>(m, norm_slots, cur);
-        } else {
-            double v[3] = {(double)s0, (double)s1, (double)s2};
-            for (int c = 0; c < 3; c++) {
-                for (int o = 16; o > 0; o >>= 1) v[c] += __shfl_xor_sync(0xffffffffu, v[c], o);
-                if (lane == 0) red[c][warp] = v[c];
-            }
-            __syncthreads();
-            if (threadIdx.x < 3) {
-                double t = 0;
-                for (int w = 0; w < 8; w++) t += red[threadIdx.x][w];
-                atomicAdd(&sums[cur * 3 + threadIdx.x], t);
-            }
-            __syncthreads();
-        }
-        s0 = s1 = s2 = 0;
-        m = 0;
-    };
-    for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
-        const BTile tl = tiles[t];
-        if (tl.prob < 0) break;   // compacted list: only end markers follow (uniform over the CTA)
-        if (active && !active[tl.prob]) continue;   // uniform over the CTA
-        const BProb& P = probs[tl.prob];
-        if (tl.prob != cur) {
-            flush();
-            cur = tl.prob;
-            if (subtract) {
-                const double cnt = (double)P.L.count();
-                for (int c = 0; c < 3; c++) mean[c] = (T)(sums[cur * 3 + c] / cnt);
-            }
-        }
-        int i, j, k;
-        if (!tile_node<32, 4, 2>(tl, P.L, i, j, k)) continue;
-        const long long q = P.vo + P.L.idx(i, j, k);
-        if (subtract) {
-            for (int c = 0; c < 3; c++) {
-                const T v = y[q + c * P.L.S] - mean[c];
-                y[q + c * P.L.S] = v;
-                const T a = fabs(v);
-                m = (a > m || a != a) ? a : m;
-            }
-        } else {
-            s0 += y[q];
-            s1 += y[q + P.L.S];
-            s2 += y[q + 2 * P.L.S];
-        }
-    }
-    flush();
-}
-
-template <typename T>
-void launch_batch_mean3(cudaStream_t st, int grid, const BProb* probs, const BTile* tiles, int ntiles,
-                        const int* active, T* y, double* sums, int subtract, void* norm_slots)
-{
-    grid = fit_grid((const void*)k_batch_mean3<T>, grid, st);
-    k_batch_mean3<T><<<grid, 256, 0, st>>>(probs, tiles, ntiles, active, y, sums, subtract, norm_slots);
+    grid = std::min(grid, segs.max);
+    if (grid < 1) return;
+    if (subtract) k_seg_mean3<T, 1><<<grid, 256, 0, st>>>(probs, segs, active, y, sums, norm_slots);
+    else k_seg_mean3<T, 0><<<grid, 256, 0, st>>>(probs, segs, active, y, sums, norm_slots);
     count_launch();
 }
-template void launch_batch_mean3<double>(cudaStream_t, int, const BProb*, const BTile*, int, const int*, double*,
-                                         double*, int, void*);
-template void launch_batch_mean3<float>(cudaStream_t, int, const BProb*, const BTile*, int, const int*, float*,
-                                        double*, int, void*);
+template void launch_batch_mean3<double>(cudaStream_t, int, const BProb*, BSegList, const int*, double*, double*, int,
+                                         void*);
+template void launch_batch_mean3<float>(cudaStream_t, int, const BProb*, BSegList, const int*, float*, double*, int,
+                                        void*);
 
 // ---------------------------------------------------------------------------
 // launchers
@@ -1147,191 +1237,225 @@ void launch_batch_diag(cudaStream_t st, int sym, int grid, const BProb* probs, c
     count_launch();
 }
 
-void launch_batch_vec(cudaStream_t st, int op, int grid, const BProb* probs, const BTile* tiles, int ntiles,
-                      const int* active, void* y, const void* x, double a, const double* scale, int fp32,
-                      const void* x2)
+void launch_batch_vec(cudaStream_t st, int op, int grid, BSegList segs, const int* active, void* y, const void* x,
+                      double a, const double* scale, int fp32, const void* x2)
 {
-    grid = fit_grid((const void*)k_batch_vec, grid, st);
-    k_batch_vec<<<grid, 256, 0, st>>>(op, probs, tiles, ntiles, active, y, x, a, scale, fp32, x2);
+    grid = std::min(grid, segs.max);
+    if (grid < 1) return;
+#define V_(OP)                                                                                          \
+    case OP:                                                                                            \
+        if (fp32) k_seg_vec<OP, float><<<grid, 256, 0, st>>>(segs, active, y, x, a, scale, x2);         \
+        else k_seg_vec<OP, double><<<grid, 256, 0, st>>>(segs, active, y, x, a, scale, x2);             \
+        break;
+    switch (op) {
+        V_(BV_ZERO) V_(BV_COPY) V_(BV_AXPY) V_(BV_SCALE_TO32) V_(BV_ACC_FROM32) V_(BV_JACOBI0)
+    }
+#undef V_
     count_launch();
 }
 
 // ---------------------------------------------------------------------------
 // Per-problem GCR over the batched FP32 cycle (the single-box inner_gcr32 on
-// every problem at once).  Tiles are the 32 x 4 x 2 lists, ordered by
-// problem; a CTA flushes its sums to the problem's slots when its tiles move
-// to another problem.  Inner products are weighted by d^2 (d = 1/diag).
+// every problem at once), over segments.  Inner products are weighted by d^2
+// (d = 1/diag); a thread sums its elements in FP32, threads are combined in FP64.
+// Directions are kept as they come, with ww_i = <w_i, w_i> beside them
+// (dots[i][2 prob]), so the step writes only the solution and the residual.
 // ---------------------------------------------------------------------------
 
-// out[p * stride + i] += sum over problem p's nodes of x v_i d^2, i < K
+// out[prob * stride + i] += sum of x v_i d^2, i < K
 template <int K>
-__global__ void __launch_bounds__(256) k_batch_multidot(const BProb* __restrict__ probs,
-                                                        const BTile* __restrict__ tiles, int ntiles,
-                                                        const int* __restrict__ active, const float* __restrict__ x,
-                                                        GcrVecs V, const float* __restrict__ d,
-                                                        double* __restrict__ out, int stride)
+__global__ void __launch_bounds__(256) k_seg_multidot(BSegList list, const int* __restrict__ active,
+                                                      const float* __restrict__ x, GcrVecs V,
+                                                      const float* __restrict__ d, double* __restrict__ out,
+                                                      int stride)
 {
-    __shared__ double red[K][8];
+    __shared__ double red[K][8], tot[K];
+    int s0, s1;
+    seg_range(list, s0, s1);
     float acc[K];
 #pragma unroll
     for (int i = 0; i < K; i++) acc[i] = 0;
-    int cur = -1;
-    auto flush = [&]() {   // every thread of the CTA together
-        if (cur < 0) return;
-        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int prob = -1;
+    auto flush = [&]() {
+        if (prob < 0) return;
+        double v[K];
 #pragma unroll
         for (int i = 0; i < K; i++) {
-            double a = (double)acc[i];
-            for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-            if (lane == 0) red[i][warp] = a;
+            v[i] = (double)acc[i];
             acc[i] = 0;
         }
-        __syncthreads();
-        if (threadIdx.x < K) {
-            double t = 0;
-            for (int w = 0; w < 8; w++) t += red[threadIdx.x][w];
-            atomicAdd(out + (long long)cur * stride + threadIdx.x, t);
-        }
-        __syncthreads();
+        seg_reduce<K>(v, red, tot);
+        if (threadIdx.x < K) atomicAdd(out + (long long)prob * stride + threadIdx.x, tot[threadIdx.x]);
     };
-    for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
-        const BTile tl = tiles[t];
-        if (tl.prob < 0) break;   // compacted list: only end markers follow (uniform over the CTA)
-        if (active && !active[tl.prob]) continue;
-        if (tl.prob != cur) {
+    for (int t = s0; t < s1; t++) {
+        const BSeg s = list.d[t];
+        if (active && !active[s.prob]) continue;
+        if (s.prob != prob) {
             flush();
-            cur = tl.prob;
+            prob = s.prob;
         }
-        const BProb& P = probs[tl.prob];
-        int i, j, k;
-        if (!tile_node<32, 4, 2>(tl, P.L, i, j, k)) continue;
-        const long long q = P.vo + P.L.idx(i, j, k);
-        for (int c = 0; c < 3; c++) {
-            const long long e = q + c * P.L.S;
-            const float dd = d[e];
-            const float xw = x[e] * dd * dd;
+        seg_each<4>(s, [&](long long e) {
+            const float4 dd = __ldg(reinterpret_cast<const float4*>(d + e));
+            const float4 xx = __ldg(reinterpret_cast<const float4*>(x + e));
+            const float4 w = make_float4(xx.x * dd.x * dd.x, xx.y * dd.y * dd.y, xx.z * dd.z * dd.z,
+                                         xx.w * dd.w * dd.w);
 #pragma unroll
-            for (int m = 0; m < K; m++) acc[m] += xw * V.v[m][e];
-        }
+            for (int i = 0; i < K; i++) {
+                const float4 v = __ldg(reinterpret_cast<const float4*>(V.v[i] + e));
+                acc[i] += (w.x * v.x + w.y * v.y) + (w.z * v.z + w.w * v.w);
+            }
+        });
     }
     flush();
 }
 
-// w -= sum_i beta_i(p) W_i, z -= sum_i beta_i(p) Z_i on problem p's nodes, i < K
+// w -= sum_i (beta_i / ww_i) W_i and z likewise (i < K), and the new direction's
+// <w, w> and <w, r> into dots[2 prob], dots[2 prob + 1].  beta_i at beta[prob *
+// stride + i], ww_i at all[(i * np + prob) * 2].
 template <int K>
-__global__ void __launch_bounds__(256) k_batch_gcr_orth(const BProb* __restrict__ probs,
-                                                        const BTile* __restrict__ tiles, int ntiles,
-                                                        const int* __restrict__ active,
-                                                        const double* __restrict__ beta, int stride, GcrVecs W,
-                                                        GcrVecs Z, float* __restrict__ w, float* __restrict__ z)
+__global__ void __launch_bounds__(256) k_seg_gcr_orth(BSegList list, const int* __restrict__ active,
+                                                      const double* __restrict__ beta, int stride,
+                                                      const double* __restrict__ all, int np, GcrVecs W, GcrVecs Z,
+                                                      float* __restrict__ w, float* __restrict__ z,
+                                                      const float* __restrict__ r, const float* __restrict__ d,
+                                                      double* __restrict__ dots)
 {
-    for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
-        const BTile tl = tiles[t];
-        if (tl.prob < 0) break;
-        if (active && !active[tl.prob]) continue;
-        const BProb& P = probs[tl.prob];
-        int i, j, k;
-        if (!tile_node<32, 4, 2>(tl, P.L, i, j, k)) continue;
-        float bb[K];
+    __shared__ double red[2][8], tot[2];
+    __shared__ float coef[K > 0 ? K : 1];
+    int s0, s1;
+    seg_range(list, s0, s1);
+    float ww = 0, wr = 0, b[K > 0 ? K : 1];
+    int prob = -1;
+    auto flush = [&]() {
+        if (prob < 0) return;
+        const double v[2] = {(double)ww, (double)wr};
+        seg_reduce<2>(v, red, tot);
+        if (threadIdx.x < 2) atomicAdd(dots + 2 * (long long)prob + threadIdx.x, tot[threadIdx.x]);
+        ww = wr = 0;
+    };
+    for (int t = s0; t < s1; t++) {
+        const BSeg s = list.d[t];
+        if (active && !active[s.prob]) continue;
+        if (s.prob != prob) {
+            flush();
+            prob = s.prob;
+            if (K > 0) {
+                __syncthreads();
+                if (threadIdx.x < K) {
+                    const double n = all[((long long)threadIdx.x * np + prob) * 2];
+                    coef[threadIdx.x] = n > 0 ? (float)(beta[(long long)prob * stride + threadIdx.x] / n) : 0.0f;
+                }
+                __syncthreads();
 #pragma unroll
-        for (int m = 0; m < K; m++) bb[m] = (float)beta[(long long)tl.prob * stride + m];
-        const long long q = P.vo + P.L.idx(i, j, k);
-        for (int c = 0; c < 3; c++) {
-            const long long e = q + c * P.L.S;
-            float tw = w[e], tz = z[e];
-#pragma unroll
-            for (int m = 0; m < K; m++) {
-                tw -= bb[m] * W.v[m][e];
-                tz -= bb[m] * Z.v[m][e];
+                for (int i = 0; i < K; i++) b[i] = coef[i];
             }
-            w[e] = tw;
-            z[e] = tz;
         }
+        seg_each<4>(s, [&](long long e) {
+            float4 tw = *reinterpret_cast<const float4*>(w + e);
+            if (K > 0) {
+                float4 tz = *reinterpret_cast<const float4*>(z + e);
+#pragma unroll
+                for (int i = 0; i < K; i++) {
+                    const float4 wi = __ldg(reinterpret_cast<const float4*>(W.v[i] + e));
+                    const float4 zi = __ldg(reinterpret_cast<const float4*>(Z.v[i] + e));
+                    tw = make_float4(tw.x - b[i] * wi.x, tw.y - b[i] * wi.y, tw.z - b[i] * wi.z, tw.w - b[i] * wi.w);
+                    tz = make_float4(tz.x - b[i] * zi.x, tz.y - b[i] * zi.y, tz.z - b[i] * zi.z, tz.w - b[i] * zi.w);
+                }
+                *reinterpret_cast<float4*>(w + e) = tw;
+                *reinterpret_cast<float4*>(z + e) = tz;
+            }
+            const float4 dd = __ldg(reinterpret_cast<const float4*>(d + e));
+            const float4 rr = __ldg(reinterpret_cast<const float4*>(r + e));
+            const float4 u = make_float4(tw.x * dd.x * dd.x, tw.y * dd.y * dd.y, tw.z * dd.z * dd.z,
+                                         tw.w * dd.w * dd.w);
+            ww += (u.x * tw.x + u.y * tw.y) + (u.z * tw.z + u.w * tw.w);
+            wr += (u.x * rr.x + u.y * rr.y) + (u.z * rr.z + u.w * rr.w);
+        });
     }
+    flush();
 }
 
-// with ww = dots[2p], rw = dots[2p+1]: (w, z) scaled to unit norm,
-// c += (rw / ww) z, r -= (rw / ww) w, max |r| per problem -> norm_slots
-__global__ void __launch_bounds__(256) k_batch_gcr_step(const BProb* __restrict__ probs,
-                                                        const BTile* __restrict__ tiles, int ntiles,
-                                                        const int* __restrict__ active,
-                                                        const double* __restrict__ dots, float* __restrict__ w,
-                                                        float* __restrict__ z, float* __restrict__ c,
-                                                        float* __restrict__ r, void* norm_slots)
+// with ww = dots[2p], wr = dots[2p+1]: c += (wr / ww) z, r -= (wr / ww) w, max |r|
+// per problem -> norm_slots
+__global__ void __launch_bounds__(256) k_seg_gcr_step(BSegList list, const int* __restrict__ active,
+                                                      const double* __restrict__ dots, const float* __restrict__ w,
+                                                      const float* __restrict__ z, float* __restrict__ c,
+                                                      float* __restrict__ r, void* norm_slots)
 {
-    float nrm = 0;
-    int cur = -1;
-    for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
-        const BTile tl = tiles[t];
-        if (tl.prob < 0) break;
-        if (active && !active[tl.prob]) continue;
-        if (tl.prob != cur) {
-            if (cur >= 0) tile_max<float>(nrm, norm_slots, cur);
+    __shared__ float a_s;
+    int s0, s1;
+    seg_range(list, s0, s1);
+    float nrm = 0, a = 0;
+    int prob = -1;
+    for (int t = s0; t < s1; t++) {
+        const BSeg s = list.d[t];
+        if (active && !active[s.prob]) continue;
+        if (s.prob != prob) {
+            if (prob >= 0) tile_max<float>(nrm, norm_slots, prob);
             nrm = 0;
-            cur = tl.prob;
+            prob = s.prob;
+            __syncthreads();
+            if (threadIdx.x == 0) {
+                const double ww = dots[2 * prob];
+                a_s = ww > 0 ? (float)(dots[2 * prob + 1] / ww) : 0.0f;
+            }
+            __syncthreads();
+            a = a_s;
         }
-        const BProb& P = probs[tl.prob];
-        int i, j, k;
-        if (!tile_node<32, 4, 2>(tl, P.L, i, j, k)) continue;
-        const double ww = dots[2 * tl.prob], rw = dots[2 * tl.prob + 1];
-        const float inv = ww > 0 ? (float)(1.0 / sqrt(ww)) : 0.0f;
-        const float a = ww > 0 ? (float)(rw / sqrt(ww)) : 0.0f;
-        const long long q = P.vo + P.L.idx(i, j, k);
-        for (int cc = 0; cc < 3; cc++) {
-            const long long e = q + cc * P.L.S;
-            const float wu = w[e] * inv, zu = z[e] * inv;
-            w[e] = wu;
-            z[e] = zu;
-            c[e] += a * zu;
-            const float rn = r[e] - a * wu;
-            r[e] = rn;
-            const float v = fabsf(rn);
-            nrm = (v > nrm || v != v) ? v : nrm;
-        }
+        seg_each<4>(s, [&](long long e) {
+            const float4 ww = __ldg(reinterpret_cast<const float4*>(w + e));
+            const float4 zz = __ldg(reinterpret_cast<const float4*>(z + e));
+            float4 cc = *reinterpret_cast<const float4*>(c + e), rr = *reinterpret_cast<const float4*>(r + e);
+            cc = make_float4(cc.x + a * zz.x, cc.y + a * zz.y, cc.z + a * zz.z, cc.w + a * zz.w);
+            rr = make_float4(rr.x - a * ww.x, rr.y - a * ww.y, rr.z - a * ww.z, rr.w - a * ww.w);
+            *reinterpret_cast<float4*>(c + e) = cc;
+            *reinterpret_cast<float4*>(r + e) = rr;
+            const float v[4] = {fabsf(rr.x), fabsf(rr.y), fabsf(rr.z), fabsf(rr.w)};
+#pragma unroll
+            for (int i = 0; i < 4; i++) nrm = (v[i] > nrm || v[i] != v[i]) ? v[i] : nrm;
+        });
     }
-    if (cur >= 0) tile_max<float>(nrm, norm_slots, cur);
+    if (prob >= 0) tile_max<float>(nrm, norm_slots, prob);
 }
 
-void launch_batch_multidot(cudaStream_t st, int grid, const BProb* probs, const BTile* tiles, int ntiles,
-                           const int* active, int k, const float* x, const GcrVecs& V, const float* d, double* out,
-                           int stride)
+void launch_batch_multidot(cudaStream_t st, int grid, BSegList segs, const int* active, int k, const float* x,
+                           const GcrVecs& V, const float* d, double* out, int stride)
 {
+    grid = std::min(grid, segs.max);
+    if (grid < 1) return;
     switch (k) {
-#define K_(K)                                                                                                 \
-    case K:                                                                                                   \
-        k_batch_multidot<K><<<fit_grid((const void*)k_batch_multidot<K>, grid, st), 256, 0, st>>>(            \
-            probs, tiles, ntiles, active, x, V, d, out, stride);                                              \
-        break;
-        K_(1) K_(2) K_(3) K_(4) K_(5) K_(6) K_(7) K_(8) K_(9) K_(10) K_(11) K_(12) K_(13) K_(14) K_(15) K_(16)
+#define K_(K) case K: k_seg_multidot<K><<<grid, 256, 0, st>>>(segs, active, x, V, d, out, stride); break;
+        K_(1) K_(2) K_(3) K_(4) K_(5) K_(6) K_(7) K_(8) K_(9) K_(10) K_(11) K_(12) K_(13) K_(14) K_(15)
 #undef K_
     default: return;
     }
     count_launch();
 }
 
-void launch_batch_gcr_orth(cudaStream_t st, int grid, const BProb* probs, const BTile* tiles, int ntiles,
-                           const int* active, int k, const double* beta, int stride, const GcrVecs& W,
-                           const GcrVecs& Z, float* w, float* z)
+void launch_batch_gcr_orth(cudaStream_t st, int grid, BSegList segs, const int* active, int k, const double* beta,
+                           int stride, const double* all, int np, const GcrVecs& W, const GcrVecs& Z, float* w,
+                           float* z, const float* r, const float* d, double* dots)
 {
+    grid = std::min(grid, segs.max);
+    if (grid < 1) return;
     switch (k) {
-#define K_(K)                                                                                                 \
-    case K:                                                                                                   \
-        k_batch_gcr_orth<K><<<fit_grid((const void*)k_batch_gcr_orth<K>, grid, st), 256, 0, st>>>(            \
-            probs, tiles, ntiles, active, beta, stride, W, Z, w, z);                                          \
+#define K_(K)                                                                                                         \
+    case K:                                                                                                           \
+        k_seg_gcr_orth<K><<<grid, 256, 0, st>>>(segs, active, beta, stride, all, np, W, Z, w, z, r, d, dots);          \
         break;
-        K_(1) K_(2) K_(3) K_(4) K_(5) K_(6) K_(7) K_(8) K_(9) K_(10) K_(11) K_(12) K_(13) K_(14) K_(15) K_(16)
+        K_(0) K_(1) K_(2) K_(3) K_(4) K_(5) K_(6) K_(7) K_(8) K_(9) K_(10) K_(11) K_(12) K_(13) K_(14) K_(15)
 #undef K_
     default: return;
     }
     count_launch();
 }
 
-void launch_batch_gcr_step(cudaStream_t st, int grid, const BProb* probs, const BTile* tiles, int ntiles,
-                           const int* active, const double* dots, float* w, float* z, float* c, float* r,
-                           void* norm_slots)
+void launch_batch_gcr_step(cudaStream_t st, int grid, BSegList segs, const int* active, const double* dots,
+                           const float* w, const float* z, float* c, float* r, void* norm_slots)
 {
-    grid = fit_grid((const void*)k_batch_gcr_step, grid, st);
-    k_batch_gcr_step<<<grid, 256, 0, st>>>(probs, tiles, ntiles, active, dots, w, z, c, r, norm_slots);
+    grid = std::min(grid, segs.max);
+    if (grid < 1) return;
+    k_seg_gcr_step<<<grid, 256, 0, st>>>(segs, active, dots, w, z, c, r, norm_slots);
     count_launch();
 }
 
