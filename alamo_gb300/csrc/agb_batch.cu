@@ -353,6 +353,13 @@ agb_status build_levels(agb_batch b)
             P.hm[0] = 0.25 / (h[0] * h[1]);
             P.hm[1] = 0.25 / (h[0] * h[2]);
             P.hm[2] = 0.25 / (h[1] * h[2]);
+            P.cube = P.h1[0] == P.h1[1] && P.h1[1] == P.h1[2];
+            for (int d = 0; d < 3; d++) {
+                P.h1f[d] = (float)P.h1[d];
+                P.i1f[d] = (float)P.i1[d];
+                P.h2f[d] = (float)P.h2[d];
+                P.hmf[d] = (float)P.hm[d];
+            }
             full.push_back(q);
             if (l < b->bottom[q]) smooth.push_back(q);
             else {

@@ -129,8 +129,9 @@ struct BProb {
     long long co;     // element offset of its moduli (ncoef planes)
     long long wo;     // element offset of its bottom-solve work (8 x 3 planes, FP64)
     int bottom;       // coarsest level of this problem
-    int pad;
+    int cube;         // the cells are cubes
     double h1[3], i1[3], h2[3], hm[3];   // reciprocal grid factors (FP64)
+    float h1f[3], i1f[3], h2f[3], hmf[3];   // and rounded to FP32 (a conversion from FP64 runs at the FP64 rate)
 };
 
 struct BTile {
