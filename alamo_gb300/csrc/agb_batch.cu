@@ -72,6 +72,12 @@ struct BLevel {
     BSegList segs_smooth() const { return BSegList{c_seg_smooth, d_nseg + 2, (int)seg_smooth.size()}; }
     std::vector<int> bottoms;
     int* d_bottoms = nullptr;
+    // of bottoms, those the FP32 cycles solve on stored rows, and the others
+    std::vector<int> bottoms_rows, bottoms_big;
+    int *d_bottoms_rows = nullptr, *d_bottoms_big = nullptr;
+    int max_unknowns = 0;   // of bottoms_rows
+    long long nrows = 0;
+    float* rows = nullptr;
     long long nvec = 0, ncoef = 0, nwork = 0;
     double *ddw64 = nullptr, *diag64 = nullptr, *dinv64 = nullptr;
     double *cor64 = nullptr, *res64 = nullptr, *rescor64 = nullptr, *tmp64 = nullptr;
@@ -267,7 +273,12 @@ template <typename T> struct BEngine {
     void bottom(int l)
     {
         BLevel& v = b->lev[l];
-        launch_batch_bottom(b->st, b->sym, fp32, v.d_probs, v.d_bottoms, (int)v.bottoms.size(), act, b->bc, false,
+        if constexpr (fp32)
+            launch_batch_bottom_rows(b->st, v.d_probs, v.d_bottoms_rows, (int)v.bottoms_rows.size(), v.max_unknowns, act,
+                                     v.rows, v.diag64, A::cor(v), A::res(v), b->p.bottom_max_iter, b->p.bottom_tol_rel,
+                                     b->p.bottom_tol_abs, b->p.bottom_smooth, b->p.final_smooth, b->omega);
+        launch_batch_bottom(b->st, b->sym, fp32, v.d_probs, fp32 ? v.d_bottoms_big : v.d_bottoms,
+                            (int)(fp32 ? v.bottoms_big : v.bottoms).size(), act, b->bc, false,
                             fp32 ? (const void*)BArr<float>::ddw(v) : (const void*)v.ddw64, v.diag64, A::cor(v),
                             A::res(v), v.work, b->p.bottom_max_iter, b->p.bottom_tol_rel, b->p.bottom_tol_abs,
                             b->p.bottom_smooth, b->p.final_smooth, b->omega);
@@ -333,6 +344,7 @@ agb_status build_levels(agb_batch b)
             BProb& P = v.probs[q];
             memset(&P, 0, sizeof(P));
             P.bottom = b->bottom[q];
+            P.ro = -1;
             if (l > b->bottom[q]) continue;   // level absent: count 0
             int nc[3];
             double h[3];
@@ -366,6 +378,15 @@ agb_status build_levels(agb_batch b)
                 P.wo = v.nwork;
                 v.nwork += 8 * 3 * P.L.S;
                 v.bottoms.push_back(q);
+                const long long nu = 3 * P.L.count();
+                if (b->p.precision == AGB_PREC_MIXED && nu <= ROWS_MAX) {
+                    P.ro = v.nrows;
+                    v.nrows += nu * ROWS_COEFS;
+                    v.bottoms_rows.push_back(q);
+                    v.max_unknowns = std::max(v.max_unknowns, (int)nu);
+                } else {
+                    v.bottoms_big.push_back(q);
+                }
             }
         }
         make_tiles(v.probs, full, d32, v.t32_full);
@@ -386,6 +407,8 @@ agb_status build_levels(agb_batch b)
         BTRY(b->upload_vec(nseg, &v.d_nseg));
         BCK(cudaStreamSynchronize(b->st));   // nseg is this scope's
         BTRY(b->upload_vec(v.bottoms, &v.d_bottoms));
+        BTRY(b->upload_vec(v.bottoms_rows, &v.d_bottoms_rows));
+        BTRY(b->upload_vec(v.bottoms_big, &v.d_bottoms_big));
         BTRY(b->alloc(&v.ddw64, v.ncoef));
         BTRY(b->alloc(&v.diag64, v.nvec));
         BTRY(b->alloc(&v.dinv64, v.nvec));
@@ -396,6 +419,7 @@ agb_status build_levels(agb_batch b)
         BTRY(b->alloc(&v.work, std::max<long long>(v.nwork, 1)));
         if (b->p.precision == AGB_PREC_MIXED) {
             BTRY(b->alloc(&v.ddw32, v.ncoef));
+            BTRY(b->alloc(&v.rows, v.nrows));
             BTRY(b->alloc(&v.dinv32, v.nvec));
             BTRY(b->alloc(&v.cor32, v.nvec));
             BTRY(b->alloc(&v.res32, v.nvec));
@@ -437,6 +461,7 @@ agb_status prepare(agb_batch b)
         BLevel& v = b->lev[l];
         launch_batch_diag(b->st, b->sym, b->grid, v.d_probs, v.d_t32_full, (int)v.t32_full.size(), b->bc, v.ddw64,
                           v.diag64, v.dinv64, v.dinv32);
+        launch_batch_rows(b->st, b->sym, v.d_probs, v.d_bottoms_rows, (int)v.bottoms_rows.size(), b->bc, v.ddw64, v.rows);
         if (v.ddw32) {
             LevelDesc flat;
             memset(&flat, 0, sizeof(flat));

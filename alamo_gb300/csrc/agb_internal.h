@@ -128,6 +128,7 @@ struct BProb {
     long long vo;     // element offset of this problem's 3-component vectors in the level arena
     long long co;     // element offset of its moduli (ncoef planes)
     long long wo;     // element offset of its bottom-solve work (8 x 3 planes, FP64)
+    long long ro;     // element offset of its stored rows (k_batch_rows; -1: none)
     int bottom;       // coarsest level of this problem
     int cube;         // the cells are cubes
     double h1[3], i1[3], h2[3], hm[3];   // reciprocal grid factors (FP64)
@@ -175,6 +176,14 @@ void launch_batch_bottom(cudaStream_t st, int sym, int fp32, const BProb* probs,
                          const int* active, const BCTable& bc, bool uniform, const void* ddw, const double* diag,
                          void* cor, const void* res, double* work, int maxiter, double tol_rel, double tol_abs, int nub,
                          int nuf, double omega);
+// FP32 bottom solves on stored rows: problems of at most ROWS_MAX coarsest unknowns
+constexpr int ROWS_MAX = 512;
+constexpr int ROWS_COEFS = 57;   // stored coefficients an unknown
+void launch_batch_rows(cudaStream_t st, int sym, const BProb* probs, const int* plist, int np, const BCTable& bc,
+                       const double* ddw64, float* rows);
+void launch_batch_bottom_rows(cudaStream_t st, const BProb* probs, const int* plist, int np, int max_unknowns,
+                              const int* active, const float* rows, const double* diag, float* cor, const float* res,
+                              int maxiter, double tol_rel, double tol_abs, int nub, int nuf, double omega);
 void launch_batch_rhs(cudaStream_t st, int sym, int grid, const BProb* probs, const BTile* tiles, int ntiles,
                       const double* ddw, const double* F0, double* rhs);
 void launch_batch_mean_stress(cudaStream_t st, int sym, int grid, const BProb* probs, const BTile* tiles, int ntiles,

@@ -38,8 +38,30 @@ __device__ __forceinline__ long long dense_to_padded(const LevelDesc& L, int q, 
 // partials in warp order (so all threads hold the same value and take the
 // same branches).  Reductions that need no value in between share a barrier:
 // (max|r|, rh.r) at the end of an iteration, (t.t, t.s), and the publication
-// of s with max|s|.  A x is summed as four interleaved partial sums.
+// of s with max|s|.
 enum { RED_SUM = 0, RED_MAX = 1 };
+
+// Row q of A x, A column-major in shared memory: four partial sums over j = 4t + s,
+// so the loads of the next columns overlap the multiply-adds.
+template <typename R> struct DenseRow {
+    const R* __restrict__ A;
+    const R* __restrict__ xs;
+    int nu, q;
+    __device__ __forceinline__ R operator()() const
+    {
+        R y0 = 0, y1 = 0, y2 = 0, y3 = 0;
+        int j = 0;
+#pragma unroll 2
+        for (; j + 3 < nu; j += 4) {
+            y0 += A[j * nu + q] * xs[j];
+            y1 += A[(j + 1) * nu + q] * xs[j + 1];
+            y2 += A[(j + 2) * nu + q] * xs[j + 2];
+            y3 += A[(j + 3) * nu + q] * xs[j + 3];
+        }
+        for (; j < nu; j++) y0 += A[j * nu + q] * xs[j];
+        return (y0 + y1) + (y2 + y3);
+    }
+};
 
 template <typename R> struct BlockRed {
     R* red;    // shared: 2 buffers x 3 values x 32 warps
@@ -74,9 +96,10 @@ template <typename R> struct BlockRed {
 };
 
 // Right-hand side read with L2-coherent loads (it may have been written
-// earlier in the same kernel by other CTAs).  `red` holds 2 x 3 x 32 values.
-template <typename T, typename R>
-__device__ void dense_bottom_block(const LevelDesc& L, const R* __restrict__ A, R* __restrict__ xs, R* __restrict__ red,
+// earlier in the same kernel by other CTAs).  `red` holds 2 x 3 x 32 values;
+// prod() returns a thread's row of A x for the x published in xs.
+template <typename T, typename R, class Prod>
+__device__ void dense_bottom_block(const LevelDesc& L, const Prod& prod, R* __restrict__ xs, R* __restrict__ red,
                                    const double* __restrict__ diag, T* __restrict__ cor, const T* __restrict__ res,
                                    int maxiter, double eps_rel_d, double eps_abs_d, int nub, int nuf, double omega_d,
                                    int* ret_slot)
@@ -91,23 +114,7 @@ __device__ void dense_bottom_block(const LevelDesc& L, const R* __restrict__ A, 
     const R eps_rel = (R)eps_rel_d, eps_abs = (R)eps_abs_d, omega = (R)omega_d;
     const bool sing = L.singular();
     BlockRed<R> br{red, 0};
-    // y = A x for the vector published in xs: four partial sums over j = 4t + s,
-    // so the loads of the next columns overlap the multiply-adds
-    auto product = [&]() -> R {
-        R y0 = 0, y1 = 0, y2 = 0, y3 = 0;
-        if (ok) {
-            int j = 0;
-#pragma unroll 2
-            for (; j + 3 < nu; j += 4) {
-                y0 += A[j * nu + q] * xs[j];
-                y1 += A[(j + 1) * nu + q] * xs[j + 1];
-                y2 += A[(j + 2) * nu + q] * xs[j + 2];
-                y3 += A[(j + 3) * nu + q] * xs[j + 3];
-            }
-            for (; j < nu; j++) y0 += A[j * nu + q] * xs[j];
-        }
-        return (y0 + y1) + (y2 + y3);
-    };
+    auto product = [&]() -> R { return ok ? prod() : (R)0; };
     auto publish = [&](R x) {
         if (ok) xs[q] = x;
     };

@@ -19,6 +19,7 @@
 #include <unordered_map>
 
 #include "agb_internal.h"
+#include "bottom.cuh"
 #include "stencil.cuh"
 #include "transfer.cuh"
 
@@ -1075,6 +1076,137 @@ __global__ void __launch_bounds__(BB_THREADS) k_batch_bottom(const BProb* __rest
     BFOR(q) cor[q] = (T)sol[q];
 }
 
+// ---------------------------------------------------------------------------
+// FP32 bottom solves on stored rows.  A coarsest level of up to ROWS_MAX
+// unknowns keeps its operator's rows, 19 neighbours (no row reaches a corner)
+// x 3 components an unknown, made once a model from the FP64 moduli
+// (k_batch_rows); the solve runs one thread an unknown with its row and its
+// Krylov entries in registers, the vector that is multiplied in shared memory
+// and one barrier a reduction (dense_bottom_block).  k_batch_bottom evaluates
+// the row from the moduli in every product, with all vectors in global memory
+// and three barriers a sum: its time is a chain of latencies.  48 RVEs (8 to
+// 125 coarsest nodes): 92 and 182 us a call before, 47 now; the solve 119 to
+// 108 ms.
+// Above ROWS_MAX unknowns the registers of a CTA do not hold a row for each; FP64 cycles keep
+// k_batch_bottom: 57 FP64 multiply-adds an unknown cost more than the row.
+// ---------------------------------------------------------------------------
+constexpr int ROW_OFFS = 19;
+
+__host__ __device__ constexpr int row_off(int o, int d)   // offset o of the 19 in direction d
+{
+    int n = 0;
+    for (int k = -1; k <= 1; k++)
+        for (int j = -1; j <= 1; j++)
+            for (int i = -1; i <= 1; i++) {
+                if (i && j && k) continue;
+                if (n++ == o) return d == 0 ? i : (d == 1 ? j : k);
+            }
+    return 0;
+}
+
+// u = the unit vector of component p at offset (i, j, k) of the node, whatever
+// node that is (on two cells a periodic node is its own two neighbours')
+struct RowAcc {
+    const double* __restrict__ c;
+    long long S;
+    Nbr nb;
+    int p, i, j, k;
+    __device__ __forceinline__ double u(int q, int di, int dj, int dk) const
+    {
+        return q == p && di == i && dj == j && dk == k ? 1.0 : 0.0;
+    }
+    __device__ __forceinline__ double C(int m, int di, int dj, int dk) const
+    {
+        return __ldg(c + m * S + nb.base + nb.o[0][di + 1] + nb.o[1][dj + 1] + nb.o[2][dk + 1]);
+    }
+};
+
+// rows[P.ro + (3 o + p) nu + q]: the coefficient of component p at offset o in row q
+template <int SYM>
+__global__ void __launch_bounds__(256) k_batch_rows(const BProb* __restrict__ probs, const int* __restrict__ plist,
+                                                    BCTable bc, const double* __restrict__ ddw,
+                                                    float* __restrict__ rows)
+{
+    const BProb& P = probs[plist[blockIdx.x]];
+    const LevelDesc& L = P.L;
+    const int cnt = (int)L.count(), nu = 3 * cnt;
+    const Geo<double> g = geo_of<double>(P);
+    for (int t = threadIdx.x; t < cnt * ROW_OFFS * 3; t += blockDim.x) {
+        const int e = t % cnt, col = t / cnt, o = col / 3;
+        const int i = e % L.nn[0], j = (e / L.nn[0]) % L.nn[1], k = e / (L.nn[0] * L.nn[1]);
+        const RowAcc acc{ddw + P.co, L.S, make_nbr(L, i, j, k), col % 3, row_off(o, 0), row_off(o, 1), row_off(o, 2)};
+        const int pos[3] = {i, j, k};
+        int mn[3], mx[3];
+        bool bnd = false;
+        for (int d = 0; d < 3; d++) {
+            mn[d] = !L.per[d] && pos[d] == 0;
+            mx[d] = !L.per[d] && pos[d] == L.n[d];
+            bnd = bnd || mn[d] || mx[d];
+        }
+        double f[3];
+        if (bnd) boundary_row<double, SYM>(acc, g, bc, mn, mx, f);
+        else interior_row<double, SYM>(acc, g, false, f);
+        for (int c = 0; c < 3; c++) rows[P.ro + (long long)col * nu + c * cnt + e] = (float)f[c];
+    }
+}
+
+// One thread's row, its coefficients in registers.
+struct StoredRow {
+    const float* __restrict__ xs;
+    int cnt;
+    int ex[3], ey[3], ez[3];   // places of the neighbours in a component, by direction
+    float w[3 * ROW_OFFS];
+    __device__ __forceinline__ float operator()() const
+    {
+        float y[3] = {0, 0, 0};
+#pragma unroll
+        for (int o = 0; o < ROW_OFFS; o++) {
+            const int at = ex[row_off(o, 0) + 1] + ey[row_off(o, 1) + 1] + ez[row_off(o, 2) + 1];
+#pragma unroll
+            for (int p = 0; p < 3; p++) y[p] += w[3 * o + p] * xs[p * cnt + at];
+        }
+        return (y[0] + y[1]) + y[2];
+    }
+};
+
+__global__ void __launch_bounds__(ROWS_MAX) k_batch_bottom_rows(const BProb* __restrict__ probs,
+                                                                const int* __restrict__ plist,
+                                                                const int* __restrict__ active,
+                                                                const float* __restrict__ rows,
+                                                                const double* __restrict__ diag_all,
+                                                                float* __restrict__ cor_all,
+                                                                const float* __restrict__ res_all, int maxiter,
+                                                                double eps_rel, double eps_abs, int nub, int nuf,
+                                                                double omega)
+{
+    __shared__ float xs[ROWS_MAX], red[2 * 3 * 32];
+    const int pid = plist[blockIdx.x];
+    if (active && !active[pid]) return;
+    const BProb& P = probs[pid];
+    const LevelDesc& L = P.L;
+    StoredRow row;
+    row.cnt = (int)L.count();
+    row.xs = xs;
+    const int nu = 3 * row.cnt;
+    const int q = min((int)threadIdx.x, nu - 1), e = q % row.cnt;   // a thread past the unknowns multiplies nothing
+#pragma unroll
+    for (int m = 0; m < 3 * ROW_OFFS; m++) row.w[m] = __ldg(rows + P.ro + (long long)m * nu + q);
+    const int pos[3] = {e % L.nn[0], (e / L.nn[0]) % L.nn[1], e / (L.nn[0] * L.nn[1])};
+    for (int s = 0; s < 3; s++) {
+        int at[3];
+        for (int d = 0; d < 3; d++) {
+            at[d] = pos[d] + s - 1;
+            if (L.per[d]) at[d] = at[d] < 0 ? L.n[d] - 1 : (at[d] >= L.n[d] ? 0 : at[d]);
+            else at[d] = min(max(at[d], 0), L.n[d]);   // past a face the coefficient is zero
+        }
+        row.ex[s] = at[0];
+        row.ey[s] = L.nn[0] * at[1];
+        row.ez[s] = L.nn[0] * L.nn[1] * at[2];
+    }
+    dense_bottom_block<float, float>(L, row, xs, red, diag_all + P.vo, cor_all + P.vo, res_all + P.vo, maxiter, eps_rel,
+                                     eps_abs, nub, nuf, omega, nullptr);
+}
+
 // rhs = -div(C : (0 - F0)) with a uniform eigenstrain F0 per problem: the
 // Newton right-hand side at u = 0 of an affine model (Newton.H:199-231,
 // Model/Solid/Affine/Isotropic.H:42-45) on a fully periodic box.
@@ -1504,6 +1636,25 @@ void launch_batch_bottom(cudaStream_t st, int sym, int fp32, const BProb* probs,
         else B_(double, SYM_MM);
     }
 #undef B_
+    count_launch();
+}
+
+void launch_batch_rows(cudaStream_t st, int sym, const BProb* probs, const int* plist, int np, const BCTable& bc,
+                       const double* ddw64, float* rows)
+{
+    if (np <= 0) return;
+    if (sym == SYM_ISO) k_batch_rows<SYM_ISO><<<np, 256, 0, st>>>(probs, plist, bc, ddw64, rows);
+    else k_batch_rows<SYM_MM><<<np, 256, 0, st>>>(probs, plist, bc, ddw64, rows);
+    count_launch();
+}
+
+void launch_batch_bottom_rows(cudaStream_t st, const BProb* probs, const int* plist, int np, int max_unknowns,
+                              const int* active, const float* rows, const double* diag, float* cor, const float* res,
+                              int maxiter, double tol_rel, double tol_abs, int nub, int nuf, double omega)
+{
+    if (np <= 0) return;
+    k_batch_bottom_rows<<<np, (max_unknowns + 31) / 32 * 32, 0, st>>>(probs, plist, active, rows, diag, cor, res,
+                                                                     maxiter, tol_rel, tol_abs, nub, nuf, omega);
     count_launch();
 }
 

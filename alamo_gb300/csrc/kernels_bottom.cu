@@ -397,8 +397,9 @@ __global__ void __launch_bounds__(DENSE_MAX) k_bottom_dense(LevelDesc L, const d
     R* A = reinterpret_cast<R*>(dsm_raw);
     dense_load<R>(A, Ag, nu);
     __syncthreads();
-    dense_bottom_block<T, R>(L, A, A + nu * nu, red, diag, cor, res, maxiter, eps_rel_d, eps_abs_d, nub, nuf, omega_d,
-                             ret_slot);
+    R* xs = A + nu * nu;
+    dense_bottom_block<T, R>(L, DenseRow<R>{A, xs, nu, (int)threadIdx.x}, xs, red, diag, cor, res, maxiter, eps_rel_d,
+                             eps_abs_d, nub, nuf, omega_d, ret_slot);
 }
 
 bool bottom_dense_fits(const LevelDesc& L) { return 3 * L.count() <= DENSE_MAX; }
