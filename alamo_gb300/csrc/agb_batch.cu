@@ -497,6 +497,7 @@ agb_status autotune(agb_batch b)
             batch_shape_dims(s, dims);
             std::vector<BTile> tl;
             make_tiles(v.probs, smooth, dims, tl);
+            if (forced < 0 && !batch_shape_worth(s, (int)tl.size(), sm_count())) continue;
             BTile* d = nullptr;
             BCK(cudaMalloc(&d, tl.size() * sizeof(BTile)));
             BCK(cudaMemcpyAsync(d, tl.data(), tl.size() * sizeof(BTile), cudaMemcpyHostToDevice, b->st));

@@ -195,6 +195,7 @@ template <typename T>
 void launch_batch_mean3(cudaStream_t st, int grid, const BProb* probs, BSegList segs, const int* active, T* y,
                         double* sums, int subtract, void* norm_slots = nullptr);
 int batch_shape_count();
+bool batch_shape_worth(int shape, int tiles, int sms);   // whether the tuner tries it on a level of that many tiles
 void batch_shape_dims(int shape, int dims[3]);
 // Per-problem GCR over the batched FP32 cycle (kernels_batch.cu; GcrVecs and
 // GCR_MAX as for the single-box inner GCR).

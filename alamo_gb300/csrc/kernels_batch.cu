@@ -46,12 +46,16 @@ static int fit_grid(const void* kernel, int grid, cudaStream_t)
     return std::min(grid, sms * per);
 }
 
-// Shapes 0-4: one node per thread (k_batch_stencil).  Shape 5: 32 x 8 columns
-// marching through 16 planes (k_batch_march), for fully periodic isotropic
-// batches only.
-static const int kShapes[6][3] = {{32, 4, 2}, {32, 8, 1}, {16, 8, 2}, {8, 8, 4}, {64, 4, 1}, {32, 8, 16}};
-constexpr int kMarchShape = 5;
-int batch_shape_count() { return 6; }
+// Shapes 0-4: one node per thread (k_batch_stencil).  Shapes 5 and 6: 32 x 8 and
+// 16 x 16 columns marching through 16 planes (k_batch_march), for fully periodic
+// isotropic batches only.  32 x 8 leaves a half or a quarter of a warp's row
+// empty on edges that 32 does not divide.  The tuner times 16 x 16 where it has
+// at least half as many tiles as there are SMs: with fewer most of the chip is
+// idle for the 18 steps of a tile.
+static const int kShapes[7][3] = {{32, 4, 2}, {32, 8, 1}, {16, 8, 2}, {8, 8, 4}, {64, 4, 1}, {32, 8, 16}, {16, 16, 16}};
+constexpr int kMarchShape = 5, kMarchShape16 = 6;
+int batch_shape_count() { return 7; }
+bool batch_shape_worth(int shape, int tiles, int sms) { return shape != kMarchShape16 || 2 * tiles >= sms; }
 void batch_shape_dims(int shape, int dims[3])
 {
     for (int d = 0; d < 3; d++) dims[d] = kShapes[shape][d];
@@ -59,7 +63,7 @@ void batch_shape_dims(int shape, int dims[3])
 bool batch_shape_ok(int shape, int sym, const int per[3])
 {
     if (shape < 0 || shape >= batch_shape_count()) return false;
-    if (shape == kMarchShape) return sym == SYM_ISO && per[0] && per[1] && per[2];
+    if (shape == kMarchShape || shape == kMarchShape16) return sym == SYM_ISO && per[0] && per[1] && per[2];
     return true;
 }
 
@@ -141,6 +145,15 @@ __device__ __forceinline__ BTile next_tile(const BTile* __restrict__ tiles, int 
     return t < ntiles ? tiles[t] : e;
 }
 
+// |v| by its bits: order-preserving, NaN above all, and no FP64 compare
+__device__ __forceinline__ unsigned int abs_bits(float v) { return __float_as_uint(v) & 0x7fffffffu; }
+__device__ __forceinline__ unsigned long long abs_bits(double v)
+{
+    return (unsigned long long)__double_as_longlong(v) & 0x7fffffffffffffffull;
+}
+__device__ __forceinline__ float as_value(unsigned int b) { return __uint_as_float(b); }
+__device__ __forceinline__ double as_value(unsigned long long b) { return __longlong_as_double((long long)b); }
+
 // node of the tile handled by this thread (1D CTA of 256 threads)
 template <int BX, int BY, int BZ>
 __device__ __forceinline__ bool tile_node(const BTile& t, const LevelDesc& L, int& i, int& j, int& k)
@@ -219,43 +232,29 @@ __global__ void __launch_bounds__(256) k_batch_stencil(const BProb* __restrict__
 // Marching tile kernel for fully periodic batches with isotropic moduli.
 //
 // A tile is a 32 x 8 block of columns of one problem and a chunk of up to 16
-// planes.  The CTA walks its chunk plane by plane with the displacement in a
-// shared-memory ring of three haloed planes (k-1, k, k+1) and the moduli in a
-// ring of two (k, k+1); the moduli of the own column at k-1 stay in
-// registers.  The halo wraps periodically (node -1 is node n-1, node n is
-// node 0), so every stored node is an interior node of the stencil.  Each
-// value is read from global memory once per tile instead of once per use,
-// and the loads of plane k+2 are in flight (in registers) while plane k is
-// computed.  The per-node arithmetic is interior_row's, as in k_batch_stencil.
+// planes.  The halo wraps periodically (node -1 is node n-1, node n is node 0),
+// so every stored node is an interior node of the stencil.  The CTA walks the
+// chunk plane by plane; every thread copies its halo values of a plane global
+// -> shared with cp.async (the wrapped rows are not contiguous), D - 2 planes
+// ahead of their use, into a ring of D planes: one is in use, one just landed.
+//
+// What a column needs of a plane it forms once, when the plane lands: the value,
+// the central differences and the second differences in x and y (five reads a
+// component).  They go from "above" to "own" to "below" in registers, so the
+// mixed differences xz and yz are differences of registers and only the four
+// corners of xy are read again: 27 + 10 shared reads a node where the row read
+// from the ring takes 57 + 12.  Sweeps of 17.3 M nodes in 48 RVEs (edges 32 to
+// 96): FP32 296 us with every difference read from the ring, 256 as it is on
+// tiles of 32 x 8, 230 on tiles of 16 x 16 (32 columns leave a quarter of the lanes of an
+// edge of 48 empty); 112 us is HBM's time.  The FP64 residual went from 4.0 to
+// 3.3 ms, the next coarser FP32 level from 60 to 44 us.  Issue bound.
+// The row is iso_row's, of the same differences as interior_row's.
 // ---------------------------------------------------------------------------
-constexpr int BM_X = 32, BM_Y = 8, BM_Z = 16;
-constexpr int BMH_X = BM_X + 2, BMH_Y = BM_Y + 2;
-constexpr int BM_HALO = BMH_X * BMH_Y;                  // 340 halo nodes per plane
-constexpr int BM_PER_THREAD = (BM_HALO + 255) / 256;    // 2 per thread (256 threads)
-
-template <typename T, int SYM> struct BMarchSmem {
-    static constexpr int NC = NCoef<SYM>::value;
-    T u[3][3][BM_HALO];    // [ring slot][component][halo node]
-    T c[2][NC][BM_HALO];
-};
-
-template <typename T, int SYM> struct BMarchAcc {
-    const BMarchSmem<T, SYM>* s;
-    int h;               // halo-tile index of the node
-    int um, u0, up;      // u ring slots of planes k-1, k, k+1
-    int c0, cp;          // moduli ring slots of planes k, k+1
-    T cm[NCoef<SYM>::value];
-    __device__ __forceinline__ T u(int p, int di, int dj, int dk) const
-    {
-        const int r = dk < 0 ? um : (dk > 0 ? up : u0);
-        return s->u[r][p][h + di + BMH_X * dj];
-    }
-    __device__ __forceinline__ T C(int m, int di, int dj, int dk) const
-    {
-        if (dk < 0) return cm[m];
-        if (dk > 0) return s->c[cp][m][h];
-        return s->c[c0][m][h + di + BMH_X * dj];
-    }
+constexpr int BM_Z = 16;
+template <typename T, int BX> struct BMarch {
+    static constexpr int BY = 256 / BX;
+    static constexpr int HX = BX + 2, HALO = HX * (BY + 2);   // halo nodes of a plane: 340 or 324, two a thread at most
+    static constexpr int D = sizeof(T) == 4 ? 4 : 3;          // planes in the ring (static shared memory: 48 KB)
 };
 
 __device__ __forceinline__ int pwrap(int i, int n)
@@ -264,17 +263,42 @@ __device__ __forceinline__ int pwrap(int i, int n)
     return i < 0 ? i + n : i;
 }
 
-template <typename T, int SYM, int MODE>
-__global__ void __launch_bounds__(256) k_batch_march(const BProb* __restrict__ probs, const BTile* __restrict__ tiles,
-                                                     int ntiles, const int* __restrict__ active, int uniform,
-                                                     const T* __restrict__ ddw, const T* __restrict__ x,
-                                                     const T* __restrict__ b, const T* __restrict__ dinv,
-                                                     T* __restrict__ out, T omega, void* norm_slots)
+template <int B> __device__ __forceinline__ void cp_async(void* smem, const void* gmem)
 {
-    __shared__ __align__(16) BMarchSmem<T, SYM> s;
-    constexpr int NC = NCoef<SYM>::value;
-    const int tid = threadIdx.x, tx = tid % BM_X, ty = tid / BM_X;
-    T nrm = 0;
+    const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(sa), "l"(gmem), "n"(B) : "memory");
+}
+__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+// the moduli of a node and its neighbours for iso_row: own column in registers
+template <typename T, int BX> struct BMarchModuli {
+    const T (*s)[BMarch<T, BX>::HALO];   // the plane's two moduli
+    int h;
+    const T *cm, *c0, *cp;    // own column below, at and above the node
+    __device__ __forceinline__ T C(int m, int di, int dj, int dk) const
+    {
+        if (dk < 0) return cm[m];
+        if (dk > 0) return cp[m];
+        return di || dj ? s[m][h + di + BMarch<T, BX>::HX * dj] : c0[m];
+    }
+};
+
+template <typename T, int MODE, int BX>
+__global__ void __launch_bounds__(256, sizeof(T) == 4 && MODE != MODE_RESID ? 3 : 2)
+    k_batch_march(const BProb* __restrict__ probs, const BTile* __restrict__ tiles, int ntiles,
+                  const int* __restrict__ active, int uniform, const T* __restrict__ ddw, const T* __restrict__ x,
+                  const T* __restrict__ b, const T* __restrict__ dinv, T* __restrict__ out, T omega, void* norm_slots)
+{
+    constexpr int D = BMarch<T, BX>::D, BY = BMarch<T, BX>::BY, HX = BMarch<T, BX>::HX, HALO = BMarch<T, BX>::HALO;
+    __shared__ __align__(16) T su[D][3][HALO];
+    __shared__ __align__(16) T sc[D][2][HALO];
+    // a warp's rows: one of 32, or rows w and w + 8 of 16 (8 rows of 18 words
+    // apart: the other 16 banks)
+    const int tid = threadIdx.x, tx = tid % BX, ty = BX == 32 ? tid / 32 : tid / 32 + 8 * (tid / 16 % 2);
+    const int h = (tx + 1) + HX * (ty + 1);
+    typedef decltype(abs_bits(T())) Bits;
+    Bits nrm = 0;
     int cur = -1;
     BTile ahead = next_tile(tiles, blockIdx.x, ntiles);
     for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
@@ -283,278 +307,144 @@ __global__ void __launch_bounds__(256) k_batch_march(const BProb* __restrict__ p
         ahead = next_tile(tiles, t + gridDim.x, ntiles);
         if (active && !active[tl.prob]) continue;
         if (MODE == MODE_RESID && norm_slots && tl.prob != cur) {
-            if (cur >= 0) tile_max<T>(nrm, norm_slots, cur);
+            if (cur >= 0) tile_max<T>(as_value(nrm), norm_slots, cur);
             nrm = 0;
             cur = tl.prob;
         }
         const BProb& P = probs[tl.prob];
         const LevelDesc& L = P.L;
         const Geo<T> g = geo_of<T>(P);
-        const long long S = L.S, plane = (long long)L.P * L.nn[1];
-        const T* xp = x + P.vo;
-        const T* cq = ddw + P.co;
-        const int i0 = tl.bx * BM_X, j0 = tl.by * BM_Y, k0 = tl.bz * BM_Z;
-        const int k1 = min(k0 + BM_Z, L.n[2]);
+        // offsets inside a problem fit 32 bits: three components of 2^31 / 1.5 nodes
+        // would not fit the device beside their moduli and vectors
+        const unsigned S = (unsigned)L.S, plane = (unsigned)L.P * L.nn[1];
+        const int n2 = L.n[2];
+        const int i0 = tl.bx * BX, j0 = tl.by * BY, k0 = tl.bz * BM_Z;
+        const int k1 = min(k0 + BM_Z, n2);
         const int i = i0 + tx, j = j0 + ty;
         const bool mine = i < L.n[0] && j < L.n[1];
-        // in-plane offsets of this thread's halo nodes, wrapped (fixed for the tile)
-        long long hoff[BM_PER_THREAD];
+        const T *xq = x + P.vo, *cq = ddw + P.co, *bv = b + P.vo, *dv = dinv + P.vo;
+        T* ov = out + P.vo;
+        unsigned own = i + (unsigned)L.P * j + plane * k0;   // the own node of plane kk (from plane k0 on)
+        unsigned hoff[2];   // in-plane offsets of this thread's halo nodes, wrapped
 #pragma unroll
-        for (int q = 0; q < BM_PER_THREAD; q++) {
-            const int e = min(tid + 256 * q, BM_HALO - 1);
-            hoff[q] = (long long)pwrap(i0 - 1 + e % BMH_X, L.n[0]) +
-                      (long long)L.P * pwrap(j0 - 1 + e / BMH_X, L.n[1]);
+        for (int q = 0; q < 2; q++) {
+            const int e = min(tid + 256 * q, HALO - 1);
+            hoff[q] = pwrap(i0 - 1 + e % HX, L.n[0]) + (unsigned)L.P * pwrap(j0 - 1 + e / HX, L.n[1]);
         }
-        T ru[BM_PER_THREAD][3], rc[BM_PER_THREAD][NC];
-        auto fetch = [&](int kk) {   // plane kk (wrapped) -> registers
-            const long long pk = plane * pwrap(kk, L.n[2]);
-#pragma unroll
-            for (int q = 0; q < BM_PER_THREAD; q++) {
-                if (tid + 256 * q < BM_HALO) {
-#pragma unroll
-                    for (int c = 0; c < 3; c++) ru[q][c] = __ldg(xp + c * S + hoff[q] + pk);
-#pragma unroll
-                    for (int m = 0; m < NC; m++) rc[q][m] = __ldg(cq + m * S + hoff[q] + pk);
-                }
-            }
-        };
-        auto stash = [&](int ur, int cr, bool with_c) {   // registers -> ring slots
-#pragma unroll
-            for (int q = 0; q < BM_PER_THREAD; q++) {
-                const int e = tid + 256 * q;
-                if (e < BM_HALO) {
-#pragma unroll
-                    for (int c = 0; c < 3; c++) s.u[ur][c][e] = ru[q][c];
-                    if (with_c) {
-#pragma unroll
-                        for (int m = 0; m < NC; m++) s.c[cr][m][e] = rc[q][m];
-                    }
-                }
-            }
-        };
-        BMarchAcc<T, SYM> acc;
-        acc.s = &s;
-        acc.h = (tx + 1) + BMH_X * (ty + 1);
-        acc.um = 0; acc.u0 = 1; acc.up = 2;
-        acc.c0 = 0; acc.cp = 1;
-        {
-            const long long p = (long long)min(i, L.n[0] - 1) + (long long)L.P * min(j, L.n[1] - 1) +
-                                plane * pwrap(k0 - 1, L.n[2]);
-#pragma unroll
-            for (int m = 0; m < NC; m++) acc.cm[m] = __ldg(cq + m * S + p);
-        }
-        fetch(k0 - 1);
-        stash(0, 0, false);
-        fetch(k0);
-        stash(1, 0, true);
-        fetch(k0 + 1);
-        for (int k = k0; k < k1; k++) {
-            stash(acc.up, acc.cp, true);
-            __syncthreads();
-            if (k + 1 < k1) fetch(k + 2);
-            if (mine) {
-                T f[3];
-                interior_row<T, SYM>(acc, g, uniform != 0, f);
-                const long long q0 = P.vo + L.idx(i, j, k);
-#pragma unroll
-                for (int c = 0; c < 3; c++) {
-                    const long long o = q0 + c * S;
-                    if (MODE == MODE_APPLY) out[o] = f[c];
-                    else if (MODE == MODE_RESID) {
-                        const T r = b[o] - f[c];
-                        out[o] = r;
-                        const T a = fabs(r);
-                        nrm = (a > nrm || a != a) ? a : nrm;
-                    } else {
-                        out[o] = s.u[acc.u0][c][acc.h] + omega * ((b[o] - f[c]) * dinv[o]);
-                    }
-                }
-            }
-#pragma unroll
-            for (int m = 0; m < NC; m++) acc.cm[m] = s.c[acc.c0][m][acc.h];
-            __syncthreads();
-            const int r = acc.um;
-            acc.um = acc.u0;
-            acc.u0 = acc.up;
-            acc.up = r;
-            acc.c0 ^= 1;
-            acc.cp ^= 1;
-        }
-    }
-    if (MODE == MODE_RESID && norm_slots && cur >= 0) tile_max<T>(nrm, norm_slots, cur);
-}
-
-// ---------------------------------------------------------------------------
-// The FP32 marching tile kernel with asynchronous plane copies.  Same tiles,
-// halo wrap and per-node arithmetic as k_batch_march, but every thread
-// copies its halo values of a plane global -> shared with 4-byte cp.async
-// (the wrapped halo rows are not contiguous), three planes ahead of the
-// compute: u in a ring of 4 planes (k-1, k, k+1 and plane k+2 in flight),
-// moduli in a ring of 3 (k, k+1, and k+2 in flight); one commit group per
-// plane.  The copies of plane k+3 are issued as soon as plane k is done.
-// ---------------------------------------------------------------------------
-template <int SYM> struct BPipeSmem {
-    static constexpr int NC = NCoef<SYM>::value;
-    float u[4][3][BM_HALO];
-    float c[3][NC][BM_HALO];
-};
-
-template <int SYM> struct BPipeAcc {
-    const BPipeSmem<SYM>* s;
-    int h;
-    int um, u0, up, c0, cp;
-    float cm[NCoef<SYM>::value];
-    __device__ __forceinline__ float u(int p, int di, int dj, int dk) const
-    {
-        const int r = dk < 0 ? um : (dk > 0 ? up : u0);
-        return s->u[r][p][h + di + BMH_X * dj];
-    }
-    __device__ __forceinline__ float C(int m, int di, int dj, int dk) const
-    {
-        if (dk < 0) return cm[m];
-        if (dk > 0) return s->c[cp][m][h];
-        return s->c[c0][m][h + di + BMH_X * dj];
-    }
-};
-
-__device__ __forceinline__ void cp_async4(void* smem, const void* gmem)
-{
-    const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(sa), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void cp_wait1() { asm volatile("cp.async.wait_group 1;" ::: "memory"); }
-__device__ __forceinline__ void cp_wait0() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
-
-template <int SYM, int MODE>
-__global__ void __launch_bounds__(256, 3) k_batch_pipe(const BProb* __restrict__ probs, const BTile* __restrict__ tiles,
-                                                    int ntiles, const int* __restrict__ active, int uniform,
-                                                    const float* __restrict__ ddw, const float* __restrict__ x,
-                                                    const float* __restrict__ b, const float* __restrict__ dinv,
-                                                    float* __restrict__ out, float omega, void* norm_slots)
-{
-    __shared__ __align__(16) BPipeSmem<SYM> s;
-    constexpr int NC = NCoef<SYM>::value;
-    const int tid = threadIdx.x, tx = tid % BM_X, ty = tid / BM_X;
-    float nrm = 0;
-    int cur = -1;
-    BTile ahead = next_tile(tiles, blockIdx.x, ntiles);
-    for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
-        const BTile tl = ahead;
-        if (tl.prob < 0) break;   // compacted list: only end markers follow (uniform over the CTA)
-        ahead = next_tile(tiles, t + gridDim.x, ntiles);
-        if (active && !active[tl.prob]) continue;
-        if (MODE == MODE_RESID && norm_slots && tl.prob != cur) {
-            if (cur >= 0) tile_max<float>(nrm, norm_slots, cur);
-            nrm = 0;
-            cur = tl.prob;
-        }
-        const BProb& P = probs[tl.prob];
-        const LevelDesc& L = P.L;
-        const Geo<float> g = geo_of<float>(P);
-        const long long S = L.S, plane = (long long)L.P * L.nn[1];
-        const float* xp = x + P.vo;
-        const float* cq = ddw + P.co;
-        const int i0 = tl.bx * BM_X, j0 = tl.by * BM_Y, k0 = tl.bz * BM_Z;
-        const int k1 = min(k0 + BM_Z, L.n[2]);
-        const int i = i0 + tx, j = j0 + ty;
-        const bool mine = i < L.n[0] && j < L.n[1];
-        long long hoff[BM_PER_THREAD];
-#pragma unroll
-        for (int q = 0; q < BM_PER_THREAD; q++) {
-            const int e = min(tid + 256 * q, BM_HALO - 1);
-            hoff[q] = (long long)pwrap(i0 - 1 + e % BMH_X, L.n[0]) +
-                      (long long)L.P * pwrap(j0 - 1 + e / BMH_X, L.n[1]);
-        }
-        // copies of plane kk: u into ring slot (kk - k0 + 1) % 4, moduli (when
-        // with_c) into (kk - k0) % 3; one commit group (empty past the chunk)
-        auto issue = [&](int kk, bool with_c) {
+        // copies of plane kk into ring slot w; one commit group (empty past the chunk)
+        auto issue = [&](int kk, int w) {
             if (kk <= k1) {
-                const long long pk = plane * pwrap(kk, L.n[2]);
-                const int ur = (kk - k0 + 1) & 3, cr = (kk - k0 + 3) % 3;
+                const unsigned pk = plane * (kk < 0 ? n2 - 1 : (kk >= n2 ? kk - n2 : kk));
 #pragma unroll
-                for (int q = 0; q < BM_PER_THREAD; q++) {
+                for (int q = 0; q < 2; q++) {
                     const int e = tid + 256 * q;
-                    if (e < BM_HALO) {
+                    if (e < HALO) {
+                        const unsigned o = hoff[q] + pk;
 #pragma unroll
-                        for (int c = 0; c < 3; c++) cp_async4(&s.u[ur][c][e], xp + c * S + hoff[q] + pk);
-                        if (with_c) {
+                        for (int c = 0; c < 3; c++) cp_async<sizeof(T)>(&su[w][c][e], xq + (o + c * S));
 #pragma unroll
-                            for (int m = 0; m < NC; m++) cp_async4(&s.c[cr][m][e], cq + m * S + hoff[q] + pk);
-                        }
+                        for (int m = 0; m < 2; m++) cp_async<sizeof(T)>(&sc[w][m][e], cq + (o + m * S));
                     }
                 }
             }
             cp_commit();
         };
-        BPipeAcc<SYM> acc;
-        acc.s = &s;
-        acc.h = (tx + 1) + BMH_X * (ty + 1);
-        {
-            const long long p = (long long)min(i, L.n[0] - 1) + (long long)L.P * min(j, L.n[1] - 1) +
-                                plane * pwrap(k0 - 1, L.n[2]);
 #pragma unroll
-            for (int m = 0; m < NC; m++) acc.cm[m] = __ldg(cq + m * S + p);
-        }
-        issue(k0 - 1, false);
-        issue(k0, true);
-        issue(k0 + 1, true);
-        issue(k0 + 2, true);
-        // b and 1/D of the own node, one plane ahead in registers
-        float bq[3] = {0, 0, 0}, dq[3] = {0, 0, 0};
-        auto fetch_bd = [&](int kk, float* bb, float* dd) {
-            if (!mine || kk >= k1) return;
-            const long long q0 = P.vo + L.idx(i, j, kk);
+        for (int d = 0; d < D - 2; d++) issue(k0 - 1 + d, d);
+        // of the planes below (m), at (0) and above: value, x and y differences
+        T um[3] = {}, u0[3] = {}, dxm[3] = {}, dx0[3] = {}, dym[3] = {}, dy0[3] = {}, xx0[3] = {}, yy0[3] = {};
+        T cm[2] = {}, c0[2] = {};
+        T bq[3] = {}, dq[3] = {};   // b and 1/D of the own node, read when the plane below it is done
+        int w0 = D - 1, wu = 0, wi = D - 2;   // slots of planes kk - 1, kk and of the plane to copy
+#pragma unroll 3   // the state moves by renaming, not by copies
+        for (int kk = k0 - 1; kk <= k1; kk++) {
+            cp_wait<D - 3>();   // plane kk has landed
+            __syncthreads();    // for every thread; and plane kk - 2, whose slot is filled next, was read by all
+            issue(kk + D - 2, wi);
+            T uu[3], dxu[3], dyu[3], xxu[3], yyu[3], cu[2];
 #pragma unroll
-            for (int c = 0; c < 3; c++) {
-                if (MODE != MODE_APPLY) bb[c] = __ldg(b + q0 + c * S);
-                if (MODE == MODE_JACOBI) dd[c] = __ldg(dinv + q0 + c * S);
+            for (int p = 0; p < 3; p++) {
+                const T* q = &su[wu][p][h];
+                uu[p] = q[0];
+                const T c2 = (T)2 * uu[p], xp = q[1], xm = q[-1], yp = q[HX], ym = q[-HX];
+                dxu[p] = xp - xm;
+                dyu[p] = yp - ym;
+                xxu[p] = (xp - c2) + xm;
+                yyu[p] = (yp - c2) + ym;
             }
-        };
-        fetch_bd(k0, bq, dq);
-        for (int k = k0; k < k1; k++) {
-            float bn[3] = {0, 0, 0}, dn[3] = {0, 0, 0};
-            fetch_bd(k + 1, bn, dn);
-            cp_wait1();   // every group but the newest (plane k+2) has landed
-            __syncthreads();
-            const int it = k - k0;
-            acc.um = it & 3;
-            acc.u0 = (it + 1) & 3;
-            acc.up = (it + 2) & 3;
-            acc.c0 = it % 3;
-            acc.cp = (it + 1) % 3;
-            if (mine) {
-                float f[3];
-                interior_row<float, SYM>(acc, g, uniform != 0, f);
-                const long long q0 = P.vo + L.idx(i, j, k);
+#pragma unroll
+            for (int m = 0; m < 2; m++) cu[m] = sc[wu][m][h];
+            if (mine && kk > k0) {
+                RowD<T> r;
+#pragma unroll
+                for (int p = 0; p < 3; p++) {
+                    const T* q = &su[w0][p][h];
+                    r.d2[0][p] = xx0[p];
+                    r.d2[1][p] = yy0[p];
+                    r.d2[2][p] = (uu[p] - (T)2 * u0[p]) + um[p];
+                    r.mx[0][p] = (q[1 + HX] - q[HX - 1]) - (q[1 - HX] - q[-1 - HX]);
+                    r.mx[1][p] = dxu[p] - dxm[p];
+                    r.mx[2][p] = dyu[p] - dym[p];
+                    r.G[0][p] = dx0[p];
+                    r.G[1][p] = dy0[p];
+                    r.G[2][p] = uu[p] - um[p];
+                }
+                const BMarchModuli<T, BX> mod{sc[w0], h, cm, c0, cu};
+                T f[3];
+                if (g.cube) {
+                    iso_row<T, true>(mod, g, uniform != 0, r, f);
+#pragma unroll
+                    for (int c = 0; c < 3; c++) f[c] *= row_scale<T, true>(g);
+                } else {
+#pragma unroll
+                    for (int p = 0; p < 3; p++) scale_diffs<T, false>(g, r, p);
+                    iso_row<T, false>(mod, g, uniform != 0, r, f);
+                }
 #pragma unroll
                 for (int c = 0; c < 3; c++) {
-                    const long long o = q0 + c * S;
-                    if (MODE == MODE_APPLY) out[o] = f[c];
+                    const unsigned o = own - plane + c * S;
+                    if (MODE == MODE_APPLY) ov[o] = f[c];
                     else if (MODE == MODE_RESID) {
-                        const float r = bq[c] - f[c];
-                        out[o] = r;
-                        const float a = fabsf(r);
-                        nrm = (a > nrm || a != a) ? a : nrm;
+                        const T v = bq[c] - f[c];
+                        ov[o] = v;
+                        const Bits a = abs_bits(v);
+                        nrm = a > nrm ? a : nrm;
                     } else {
-                        out[o] = s.u[acc.u0][c][acc.h] + omega * ((bq[c] - f[c]) * dq[c]);
+                        ov[o] = u0[c] + omega * ((bq[c] - f[c]) * dq[c]);
                     }
                 }
             }
 #pragma unroll
-            for (int m = 0; m < NC; m++) acc.cm[m] = s.c[acc.c0][m][acc.h];
-#pragma unroll
-            for (int c = 0; c < 3; c++) {
-                bq[c] = bn[c];
-                dq[c] = dn[c];
+            for (int p = 0; p < 3; p++) {
+                um[p] = u0[p];
+                u0[p] = uu[p];
+                dxm[p] = dx0[p];
+                dx0[p] = dxu[p];
+                dym[p] = dy0[p];
+                dy0[p] = dyu[p];
+                xx0[p] = xxu[p];
+                yy0[p] = yyu[p];
             }
-            __syncthreads();
-            issue(k + 3, true);   // into the slots of u(k-1) and moduli(k)
+            if (mine && kk >= k0 && kk < k1) {
+#pragma unroll
+                for (int c = 0; c < 3; c++) {
+                    if (MODE != MODE_APPLY) bq[c] = __ldg(bv + (own + c * S));
+                    if (MODE == MODE_JACOBI) dq[c] = __ldg(dv + (own + c * S));
+                }
+            }
+            if (kk >= k0) own += plane;
+#pragma unroll
+            for (int m = 0; m < 2; m++) {
+                cm[m] = c0[m];
+                c0[m] = cu[m];
+            }
+            w0 = wu;
+            wu = wu + 1 == D ? 0 : wu + 1;
+            wi = wi + 1 == D ? 0 : wi + 1;
         }
-        cp_wait0();
-        __syncthreads();
+        __syncthreads();   // every copy has landed and been read: the next tile's may start
     }
-    if (MODE == MODE_RESID && norm_slots && cur >= 0) tile_max<float>(nrm, norm_slots, cur);
+    if (MODE == MODE_RESID && norm_slots && cur >= 0) tile_max<T>(as_value(nrm), norm_slots, cur);
 }
 
 // Full weighting (restriction) or trilinear prolongation between the levels of
@@ -774,14 +664,6 @@ template <int K> __device__ __forceinline__ void seg_reduce(const double (&v)[K]
     }
     __syncthreads();
 }
-
-__device__ __forceinline__ unsigned int abs_bits(float v) { return __float_as_uint(v) & 0x7fffffffu; }
-__device__ __forceinline__ unsigned long long abs_bits(double v)
-{
-    return (unsigned long long)__double_as_longlong(v) & 0x7fffffffffffffffull;
-}
-__device__ __forceinline__ float as_value(unsigned int b) { return __uint_as_float(b); }
-__device__ __forceinline__ double as_value(unsigned long long b) { return __longlong_as_double((long long)b); }
 
 // Per-problem component sums (sums[3 prob + c]), or with subtract y -= sums /
 // count over the nodes (not the padding), and the per-problem max |y| after it.
@@ -1301,17 +1183,6 @@ template void launch_batch_mean3<float>(cudaStream_t, int, const BProb*, BSegLis
 // ---------------------------------------------------------------------------
 // launchers
 // ---------------------------------------------------------------------------
-// The FP32 marching shape uses the asynchronous-copy kernel unless
-// AGB_BATCH_PIPE=0 (then the register-prefetch kernel, as for FP64).
-static bool batch_pipe_enabled()
-{
-    static const bool v = [] {
-        const char* e = getenv("AGB_BATCH_PIPE");
-        return !(e && e[0] == '0');
-    }();
-    return v;
-}
-
 template <typename T, int SYM, int MODE>
 static void bst_shape(cudaStream_t st, int shape, int grid, const BProb* probs, const BTile* tiles, int ntiles,
                       const int* active, const BCTable& bc, bool uniform, const T* ddw, const T* x, const T* b,
@@ -1324,23 +1195,17 @@ static void bst_shape(cudaStream_t st, int shape, int grid, const BProb* probs, 
     // the marching shape is only chosen for isotropic fully periodic batches
     // (batch_shape_ok)
     if constexpr (SYM == SYM_ISO) {
-        if (shape == kMarchShape) {
-            if constexpr (sizeof(T) == 4) {
-                if (batch_pipe_enabled()) {
-                    grid = fit_grid((const void*)k_batch_pipe<SYM, MODE>, grid, st);
-                    k_batch_pipe<SYM, MODE><<<grid, 256, 0, st>>>(probs, tiles, ntiles, active, uniform ? 1 : 0,
-                                                                  (const float*)ddw, (const float*)x, (const float*)b,
-                                                                  (const float*)dinv, (float*)out, (float)omega, norm);
-                    count_launch();
-                    return;
-                }
-            }
-            grid = fit_grid((const void*)k_batch_march<T, SYM, MODE>, grid, st);
-            k_batch_march<T, SYM, MODE><<<grid, 256, 0, st>>>(probs, tiles, ntiles, active, uniform ? 1 : 0, ddw, x, b,
-                                                              dinv, out, omega, norm);
-            count_launch();
-            return;
-        }
+#define M_(BX)                                                                                                       \
+    do {                                                                                                             \
+        grid = fit_grid((const void*)k_batch_march<T, MODE, BX>, grid, st);                                          \
+        k_batch_march<T, MODE, BX><<<grid, 256, 0, st>>>(probs, tiles, ntiles, active, uniform ? 1 : 0, ddw, x, b,   \
+                                                         dinv, out, omega, norm);                                    \
+        count_launch();                                                                                              \
+        return;                                                                                                      \
+    } while (0)
+        if (shape == kMarchShape) M_(32);
+        if (shape == kMarchShape16) M_(16);
+#undef M_
     }
     switch (shape) {
     case 0: L_(32, 4, 2); break;
