@@ -122,6 +122,64 @@ __global__ void k_import(LevelDesc L, int ncomp, const TS* __restrict__ src, TD*
     for (int c = 0; c < ncomp; c++) dst[c * L.S + q] = (TD)(aos ? src[s * ncomp + c] : src[c * Nsrc + s]);
 }
 
+// The same for component planes (SoA) on both sides: a warp copies one row of
+// one component, COPY_UNROLL elements a lane in flight at once; bound by HBM.  The
+// node-per-thread kernel has three loads in flight and leaves the last warp of
+// a row of 2^k + 1 nodes nearly empty: 192 x 160 x 144
+// cells in FP32 (109 MB moved) 33 us against 16 in and 21 out; two sweeps through the
+// public call 431 against 389 us.
+constexpr int COPY_UNROLL = 8;
+template <typename TD, typename TS>
+__global__ void __launch_bounds__(256) k_import_rows(LevelDesc L, long long rows, const TS* __restrict__ src,
+                                                     TD* __restrict__ dst, int k0, int nk, long long Nsrc, int chunk)
+{
+    const int lane = threadIdx.x & 31;
+    const long long r = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (r >= rows) return;
+    const int j = (int)(r % L.nn[1]);
+    const long long t = r / L.nn[1];
+    const int k = k0 + (int)(t % nk), c = (int)(t / nk);
+    const TS* s = src + c * Nsrc + (long long)(L.n[0] + 1) * (j + (long long)(L.n[1] + 1) * (chunk ? k - k0 : k));
+    TD* d = dst + c * L.S + L.idx(0, j, k);
+    for (int i0 = lane; i0 < L.nn[0]; i0 += 32 * COPY_UNROLL) {
+        TS v[COPY_UNROLL];
+#pragma unroll
+        for (int u = 0; u < COPY_UNROLL; u++)
+            if (i0 + 32 * u < L.nn[0]) v[u] = __ldg(s + i0 + 32 * u);
+#pragma unroll
+        for (int u = 0; u < COPY_UNROLL; u++)
+            if (i0 + 32 * u < L.nn[0]) d[i0 + 32 * u] = (TD)v[u];
+    }
+}
+
+// and back, periodic images filled
+template <typename TD, typename TS>
+__global__ void __launch_bounds__(256) k_export_rows(LevelDesc L, long long rows, const TS* __restrict__ src,
+                                                     TD* __restrict__ dst, int k0, int nk, long long Ndst, int chunk)
+{
+    const int lane = threadIdx.x & 31;
+    const long long r = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (r >= rows) return;
+    const int n0 = L.n[0] + 1, n1 = L.n[1] + 1;
+    const int j = (int)(r % n1);
+    const long long t = r / n1;
+    const int k = k0 + (int)(t % nk), c = (int)(t / nk);
+    const TS* s = src + c * L.S + L.idx(0, L.per[1] && j == L.n[1] ? 0 : j, L.per[2] && k == L.n[2] ? 0 : k);
+    TD* d = dst + c * Ndst + (long long)n0 * (j + (long long)n1 * (chunk ? k - k0 : k));
+    const int wrap = L.per[0] ? L.n[0] : -1;   // this column is column 0
+    for (int i0 = lane; i0 < n0; i0 += 32 * COPY_UNROLL) {
+        TS v[COPY_UNROLL];
+#pragma unroll
+        for (int u = 0; u < COPY_UNROLL; u++) {
+            const int i = i0 + 32 * u;
+            if (i < n0) v[u] = __ldg(s + (i == wrap ? 0 : i));
+        }
+#pragma unroll
+        for (int u = 0; u < COPY_UNROLL; u++)
+            if (i0 + 32 * u < n0) d[i0 + 32 * u] = (TD)v[u];
+    }
+}
+
 // The same for interleaved (AoS) sources, through shared memory: a warp
 // copies the contiguous 32 x ncomp source values of 32 consecutive nodes of a
 // row into shared memory (coalesced), then writes each component's 32 values
@@ -342,6 +400,15 @@ void launch_import(cudaStream_t st, const LevelDesc& L, int ncomp, const TS* src
         count_launch();
         return;
     }
+    if (!aos || ncomp == 1) {
+        const int nk = std::min(kc, L.nn[2] - k0);
+        if (nk <= 0 || ncomp <= 0) return;
+        const long long rows = (long long)ncomp * nk * L.nn[1];
+        const long long Nsrc = (long long)(L.n[0] + 1) * (L.n[1] + 1) * (chunk ? kc : L.n[2] + 1);
+        k_import_rows<TD, TS><<<(unsigned)((rows + 7) / 8), 256, 0, st>>>(L, rows, src, dst, k0, nk, Nsrc, chunk ? 1 : 0);
+        count_launch();
+        return;
+    }
     dim3 blk(32, 4, 2);
     dim3 grd((L.nn[0] + blk.x - 1) / blk.x, (L.nn[1] + blk.y - 1) / blk.y, (kc + blk.z - 1) / blk.z);
     k_import<TD, TS><<<grd, blk, 0, st>>>(L, ncomp, src, dst, aos ? 1 : 0, k0, kc, chunk ? 1 : 0); count_launch();
@@ -351,6 +418,15 @@ template <typename TD, typename TS>
 void launch_export(cudaStream_t st, const LevelDesc& L, int ncomp, const TS* src, TD* dst, bool aos, int k0, int kc,
                    bool chunk)
 {
+    if (!aos || ncomp == 1) {
+        const int nk = std::min(kc, L.n[2] + 1 - k0);
+        if (nk <= 0 || ncomp <= 0) return;
+        const long long rows = (long long)ncomp * nk * (L.n[1] + 1);
+        const long long Ndst = (long long)(L.n[0] + 1) * (L.n[1] + 1) * (chunk ? kc : L.n[2] + 1);
+        k_export_rows<TD, TS><<<(unsigned)((rows + 7) / 8), 256, 0, st>>>(L, rows, src, dst, k0, nk, Ndst, chunk ? 1 : 0);
+        count_launch();
+        return;
+    }
     dim3 blk(32, 4, 2);
     dim3 grd((L.n[0] + 1 + blk.x - 1) / blk.x, (L.n[1] + 1 + blk.y - 1) / blk.y, (kc + blk.z - 1) / blk.z);
     k_export<TD, TS><<<grd, blk, 0, st>>>(L, ncomp, src, dst, aos ? 1 : 0, k0, kc, chunk ? 1 : 0); count_launch();
