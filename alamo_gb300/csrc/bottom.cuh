@@ -66,6 +66,11 @@ template <typename R> struct DenseRow {
 template <typename R> struct BlockRed {
     R* red;    // shared: 2 buffers x 3 values x 32 warps
     int buf;
+    static __device__ __forceinline__ R join(int op, R a, R b)
+    {
+        if (op == RED_SUM) return a + b;
+        return (b > a || b != b) ? b : a;
+    }
     template <int N>
     __device__ __forceinline__ void run(R (&v)[N], const int (&op)[N])
     {
@@ -74,22 +79,28 @@ template <typename R> struct BlockRed {
         for (int k = 0; k < N; k++) {
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) {
-                const R w = __shfl_xor_sync(0xffffffffu, v[k], o);
-                if (op[k] == RED_SUM) v[k] += w;
-                else v[k] = (w > v[k] || w != w) ? w : v[k];
+                v[k] = join(op[k], v[k], __shfl_xor_sync(0xffffffffu, v[k], o));
             }
             if (lane == 0) red[(buf * 3 + k) * 32 + warp] = v[k];
         }
         __syncthreads();
+        // few warps: every thread adds their partials in turn; more: each lane
+        // takes one and the warp adds them by shuffles (12 warps: four steps
+        // where the turn is twelve dependent reads)
+        if (nw <= 4) {
 #pragma unroll
-        for (int k = 0; k < N; k++) {
-            R t = red[(buf * 3 + k) * 32];
-            for (int w = 1; w < nw; w++) {
-                const R x = red[(buf * 3 + k) * 32 + w];
-                if (op[k] == RED_SUM) t += x;
-                else t = (x > t || x != x) ? x : t;
+            for (int k = 0; k < N; k++) {
+                R t = red[(buf * 3 + k) * 32];
+                for (int w = 1; w < nw; w++) t = join(op[k], t, red[(buf * 3 + k) * 32 + w]);
+                v[k] = t;
             }
-            v[k] = t;
+        } else {
+            const int span = nw <= 16 ? 16 : 32, l = lane & (span - 1);
+#pragma unroll
+            for (int k = 0; k < N; k++) v[k] = l < nw ? red[(buf * 3 + k) * 32 + l] : (R)0;   // 0: sums, and maxima of |.|
+            for (int o = span / 2; o > 0; o >>= 1)
+#pragma unroll
+                for (int k = 0; k < N; k++) v[k] = join(op[k], v[k], __shfl_xor_sync(0xffffffffu, v[k], o));
         }
         buf ^= 1;
     }

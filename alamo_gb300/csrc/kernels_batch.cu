@@ -967,7 +967,7 @@ __global__ void __launch_bounds__(BB_THREADS) k_batch_bottom(const BProb* __rest
 // and one barrier a reduction (dense_bottom_block).  k_batch_bottom evaluates
 // the row from the moduli in every product, with all vectors in global memory
 // and three barriers a sum: its time is a chain of latencies.  48 RVEs (8 to
-// 125 coarsest nodes): 92 and 182 us a call before, 47 now; the solve 119 to
+// 125 coarsest nodes): 92 and 182 us a call before, 43 now; the solve 119 to
 // 108 ms.
 // Above ROWS_MAX unknowns the registers of a CTA do not hold a row for each; FP64 cycles keep
 // k_batch_bottom: 57 FP64 multiply-adds an unknown cost more than the row.
@@ -1109,21 +1109,22 @@ __global__ void __launch_bounds__(256) k_batch_rhs(const BProb* __restrict__ pro
             for (int c = 0; c < 3; c++) E[a][c] = 0.0 - F0[tl.prob * 9 + a * 3 + c];
         double ret[3] = {0, 0, 0};
         for (int d = 0; d < 3; d++) {
-            double cpv[NCoef<SYM>::value], cmv[NCoef<SYM>::value], Dp[3][3], Dm[3][3];
-            for (int m = 0; m < NCoef<SYM>::value; m++) {
-                cpv[m] = ddw[P.co + m * L.S + nb.base + nb.o[d][2]];
-                cmv[m] = ddw[P.co + m * L.S + nb.base + nb.o[d][0]];
-            }
-            c_mul_mat<double, SYM>(cpv, E, Dp);
-            c_mul_mat<double, SYM>(cmv, E, Dm);
-            for (int r = 0; r < 3; r++) ret[r] += (Dp[r][d] - Dm[r][d]) * P.h1[d];
+            // (C+ - C-) : E, the difference of the moduli first
+            double dc[NCoef<SYM>::value], D[3][3];
+            for (int m = 0; m < NCoef<SYM>::value; m++)
+                dc[m] = ddw[P.co + m * L.S + nb.base + nb.o[d][2]] - ddw[P.co + m * L.S + nb.base + nb.o[d][0]];
+            c_mul_mat<double, SYM>(dc, E, D);
+            for (int r = 0; r < 3; r++) ret[r] += D[r][d] * P.h1[d];
         }
         for (int r = 0; r < 3; r++) rhs[P.vo + r * L.S + nb.base] = 0.0 - ret[r];
     }
 }
 
 // Per-problem sums of sigma = C : (grad u - F0) over the stored nodes
-// (central differences; fully periodic boxes), for the homogenized stress.
+// (central differences; fully periodic boxes), for the homogenized stress.  A
+// CTA takes a contiguous part of the list and a thread keeps its six sums while
+// the problem stays the same: reducing nine a tile by shuffles was most of its
+// FP64 work (17.3 M nodes 2.8 ms before, 1.2 now).
 template <int SYM>
 __global__ void __launch_bounds__(256) k_batch_mean_stress(const BProb* __restrict__ probs,
                                                            const BTile* __restrict__ tiles, int ntiles,
@@ -1131,38 +1132,47 @@ __global__ void __launch_bounds__(256) k_batch_mean_stress(const BProb* __restri
                                                            const double* __restrict__ F0,
                                                            const double* __restrict__ u, double* __restrict__ sums)
 {
-    __shared__ double red[9][8];
-    for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
+    __shared__ double red[6][8], tot[6];
+    double acc[6] = {0, 0, 0, 0, 0, 0};   // xx, xy, xz, yy, yz, zz
+    int prob = -1;
+    auto flush = [&]() {   // every thread of the CTA together
+        if (prob < 0) return;
+        seg_reduce<6>(acc, red, tot);
+        if (threadIdx.x < 9) {
+            const int r = threadIdx.x / 3, c = threadIdx.x % 3, lo = min(r, c), hi = max(r, c);
+            atomicAdd(&sums[prob * 9 + threadIdx.x], tot[lo == 0 ? hi : (lo == 1 ? 2 + hi : 5)]);
+        }
+        for (int q = 0; q < 6; q++) acc[q] = 0;
+    };
+    const int t0 = (int)((long long)ntiles * blockIdx.x / gridDim.x);
+    const int t1 = (int)((long long)ntiles * (blockIdx.x + 1) / gridDim.x);
+    for (int t = t0; t < t1; t++) {
         const BTile tl = tiles[t];
+        if (tl.prob != prob) {
+            flush();
+            prob = tl.prob;
+        }
         const BProb& P = probs[tl.prob];
         const LevelDesc& L = P.L;
         int i, j, k;
-        double S[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
-        if (tile_node<32, 4, 2>(tl, L, i, j, k)) {
-            const Nbr nb = make_nbr(L, i, j, k);
-            double G[3][3], c[NCoef<SYM>::value];
-            for (int p = 0; p < 3; p++)
-                for (int d = 0; d < 3; d++)
-                    G[p][d] = (u[P.vo + p * L.S + nb.base + nb.o[d][2]] - u[P.vo + p * L.S + nb.base + nb.o[d][0]]) *
-                                  P.h1[d] -
-                              F0[tl.prob * 9 + p * 3 + d];
-            for (int m = 0; m < NCoef<SYM>::value; m++) c[m] = ddw[P.co + m * L.S + nb.base];
-            c_mul_mat<double, SYM>(c, G, S);
-        }
-        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-        for (int a = 0; a < 9; a++) {
-            double v = S[a / 3][a % 3];
-            for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-            if (lane == 0) red[a][warp] = v;
-        }
-        __syncthreads();
-        if (threadIdx.x < 9) {
-            double v = 0;
-            for (int w = 0; w < 8; w++) v += red[threadIdx.x][w];
-            atomicAdd(&sums[tl.prob * 9 + threadIdx.x], v);
-        }
-        __syncthreads();
+        if (!tile_node<32, 4, 2>(tl, L, i, j, k)) continue;
+        const Nbr nb = make_nbr(L, i, j, k);
+        double G[3][3], S[3][3], c[NCoef<SYM>::value];
+        for (int p = 0; p < 3; p++)
+            for (int d = 0; d < 3; d++)
+                G[p][d] = (u[P.vo + p * L.S + nb.base + nb.o[d][2]] - u[P.vo + p * L.S + nb.base + nb.o[d][0]]) *
+                              P.h1[d] -
+                          F0[tl.prob * 9 + p * 3 + d];
+        for (int m = 0; m < NCoef<SYM>::value; m++) c[m] = ddw[P.co + m * L.S + nb.base];
+        c_mul_mat<double, SYM>(c, G, S);
+        acc[0] += S[0][0];
+        acc[1] += S[0][1];
+        acc[2] += S[0][2];
+        acc[3] += S[1][1];
+        acc[4] += S[1][2];
+        acc[5] += S[2][2];
     }
+    flush();
 }
 
 template <typename T>
