@@ -37,11 +37,10 @@ WORKLOAD = ("257^3-node cubic Voronoi polycrystal (64 grains, C11/C12/C44 = 1.68
             "uniaxial tension u_x=0.01, solve to 1e-8 relative FP64 residual")
 BYTES_PER_NODE = {"jacobi_f32_cubic": 132, "fapply_f32_cubic": 108, "jacobi_f64_cubic": 264,
                   "fapply_f64_cubic": 216}
-# FP64 operations of one interior node of the damped-Jacobi sweep on cubic
-# cells (an FMA counts 2), counted by ncu on the marching kernel (DFMA, DADD,
-# DMUL thread instructions over the interior nodes of one 65^3 launch:
-# 98 + 129 + 26)
-FLOPS_PER_NODE = {"jacobi_f64_cubic": 351, "fapply_f64_cubic": 339}   # Fapply: 95 + 126 + 23
+# FP64 operations of a node of the damped-Jacobi sweep on cubic cells (an FMA
+# counts 2), counted by ncu on k_column (DFMA, DADD, DMUL thread instructions
+# over the nodes of one 129^3 launch: 82 + 55 + 7)
+FLOPS_PER_NODE = {"jacobi_f64_cubic": 226, "fapply_f64_cubic": 215}   # Fapply: 76 + 56 + 7
 
 
 def parse():
@@ -642,7 +641,7 @@ def main():
                                 / 1e9, 1),
         "kernel_ms": res["kernels_ms"],
         "fp64_roofline": {
-            "kernel": "k_stencil_march<double,MajorMinor,Jacobi> + k_stencil_shell (finest level)", "bound": "fp64",
+            "kernel": "k_column<double,MajorMinor,Jacobi> (finest level)", "bound": "fp64",
             "flops_per_node": FLOPS_PER_NODE["jacobi_f64_cubic"],
             "achieved": round(FLOPS_PER_NODE["jacobi_f64_cubic"] * nodes / (res["kernels_ms"]["jacobi_f64"] * 1e-3)
                               / 1e12, 3),
