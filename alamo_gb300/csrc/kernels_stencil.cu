@@ -313,6 +313,7 @@ __global__ void __launch_bounds__(COL_X* COL_Y, COL_RESIDENT) k_column(LevelDesc
                                                          const T* __restrict__ b, const T* __restrict__ dinv,
                                                          T* __restrict__ out, T omega, void* norm_slot)
 {
+    pdl_entry();
     const int tx = threadIdx.x, ty = threadIdx.y;
     T nrm = 0;
     if ((int)blockIdx.z >= chunks) {
