@@ -17,6 +17,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdarg>
+#include <cstdint>
 #include <cstdio>
 #include <cstring>
 #include <new>
@@ -1643,15 +1644,22 @@ static double* device_view(agb_op op, double* p, int mem)
 }
 
 // u of the fields computed from a displacement: read in place in device
-// memory (*full), else imported into the operator's work buffer.
-static agb_status post_input(agb_op op, const double* u, int mem, const double** du, bool* full)
+// memory (*full), else imported into the operator's work buffer -- also where
+// one of the outputs (`nout` boxes of count[] doubles) overlaps u in device
+// memory, since a kernel that reads the neighbours of a node must not write over them.
+static agb_status post_input(agb_op op, const double* u, int mem, double* const* outs, const size_t* count, int nout,
+                             const double** du, bool* full)
 {
+    Level& v = op->lev[0];
     *full = mem == AGB_MEM_DEVICE;
+    const uintptr_t u0 = (uintptr_t)u;
+    const uintptr_t u1 = u0 + 3 * sizeof(double) * (size_t)(v.L.n[0] + 1) * (v.L.n[1] + 1) * (v.L.n[2] + 1);
+    for (int q = 0; q < nout; q++)
+        if (outs[q] && (uintptr_t)outs[q] < u1 && u0 < (uintptr_t)(outs[q] + count[q])) *full = false;
     if (*full) {
         *du = u;
         return caller_ready(mem);
     }
-    Level& v = op->lev[0];
     *du = v.hold64;
     return upload<double, double>(op, v.L, 3, false, u, mem, v.hold64);
 }
@@ -1671,12 +1679,12 @@ static agb_status post_fields(agb_op op, const double* F0, const double* u, doub
     const size_t N = (size_t)(v.L.n[0] + 1) * (v.L.n[1] + 1) * (v.L.n[2] + 1);
     double* dF0 = nullptr;
     TRY(load_F0(op, F0, mem, &dF0));
-    const double* du = nullptr;
-    bool full = false;
-    TRY(post_input(op, u, mem, &du, &full));
     double* want[3] = {sigma, eps, energy};
     double *dev[3] = {nullptr, nullptr, nullptr}, *tmp[3] = {nullptr, nullptr, nullptr};
     const size_t count[3] = {9 * N, 9 * N, N};
+    const double* du = nullptr;
+    bool full = false;
+    TRY(post_input(op, u, mem, want, count, 3, &du, &full));
     agb_status st = AGB_OK;
     for (int q = 0; q < 3 && st == AGB_OK; q++) {
         if (!want[q]) continue;
@@ -1717,7 +1725,7 @@ agb_status agb_traction_xhi(agb_op op, const double* F0, const double* u, double
     TRY(load_F0(op, F0, mem, &dF0));
     const double* du = nullptr;
     bool full = false;
-    TRY(post_input(op, u, mem, &du, &full));
+    TRY(post_input(op, u, mem, nullptr, nullptr, 0, &du, &full));
     // the bottom solve's work (8 x 3 x 64 doubles at least) is free outside a solve
     launch_traction_xhi(op->st, op->sym, v.L, v.ddw64, dF0, du, full, op->bottom_work, op->d_slots + 4);
     if (cudaGetLastError() != cudaSuccess ||

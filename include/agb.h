@@ -184,7 +184,8 @@ agb_status agb_traction_xhi(agb_op op, const double* F0, const double* u, double
  * Elastic::Energy(amrlev, energy, u), Elastic.cpp:552-597: energy = sig : eps
  * / 2 per node with sig = C : grad u (may be NULL; the reference adds this to
  * the values already in its output field, this call writes it).  Gradients
- * one-sided on the boundary as Numeric::GetStencil gives them. */
+ * one-sided on the boundary as Numeric::GetStencil gives them.  The outputs of
+ * agb_stress and agb_strain_energy may overlap u (and F0). */
 agb_status agb_strain_energy(agb_op op, const double* u, double* eps9, double* energy, int mem);
 
 /* Batched RVE homogenization: `nprob` independent boxes (sizes n_cells[3*q..],
