@@ -408,8 +408,13 @@ bool bottom_dense_fits(const LevelDesc& L) { return 3 * L.count() <= DENSE_MAX; 
 // Exact coarsest solve.  Once per solve the dense operator (FP64,
 // column-major) is inverted by Gauss-Jordan elimination with partial pivoting
 // in FP64 and stored row-major in FP64 (FP64 cycles) and FP32 (FP32 cycles).  A
-// fully periodic level (singular), or a pivot at or below 1e-13 of the largest
-// |entry|, clears *ok and the cycles keep the BiCGStab bottom.
+// displacement row is 1 and an interior row C/dx^2, so each row is first scaled
+// to a largest |entry| in [1, 2) by a power of two, which the columns of the
+// inverse take back: (S A)^-1 S = A^-1, exact, and the same pivots in any units.  A
+// fully periodic level (singular), or a pivot at or below 1e-13 of the scaled
+// rows, clears *ok and the cycles keep the BiCGStab bottom.  (Compared with the
+// largest entry of the whole matrix instead, a level of 2^3 cells has a smallest
+// pivot of 2e-2 with C = 1 on a unit box and 1e-17 with C = 2e11 on one of 1 cm.)
 //
 // BiCGStab runs in one CTA, whose SM has two FP64 lanes per clock and whose
 // reductions are barriers: 37 us (isotropic) to 248 us a call on 81 unknowns,
@@ -428,15 +433,25 @@ bool bottom_dense_fits(const LevelDesc& L) { return 3 * L.count() <= DENSE_MAX; 
 // new(r, c) = (r in panel ? 0 : old(perm r, c)) + sum_q T(r, q) old(perm(k + q), c),
 // from one copy of the matrix into another, so that its tiles are independent.
 // ---------------------------------------------------------------------------
+constexpr double PIVOT_MIN = 1e-13;
+
+// Power of two that brings a row whose largest |entry| is amax to [1, 2) (NaN
+// for an infinite entry, which no pivot passes).
+__device__ __forceinline__ double row_factor(double amax)
+{
+    if (amax == 0.0) return 1.0;
+    return isinf(amax) ? amax - amax : scalbn(1.0, min(-ilogb(amax), 1000));
+}
+
 __global__ void __launch_bounds__(1024) k_bottom_invert(LevelDesc L, const double* __restrict__ Ag,
                                                        double* __restrict__ inv64, float* __restrict__ inv32,
                                                        int* __restrict__ ok)
 {
     extern __shared__ __align__(16) unsigned char inv_raw[];
     double* M = reinterpret_cast<double*>(inv_raw);   // nu x nu, row-major
-    __shared__ double fcol[DENSE_MAX];
+    __shared__ double fcol[DENSE_MAX], scale[DENSE_MAX];
     __shared__ int piv[DENSE_MAX];
-    __shared__ double amax_s, pinv_s;
+    __shared__ double pinv_s;
     __shared__ int bad_s;
     const int nu = 3 * (int)L.count();
     const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31;
@@ -444,22 +459,17 @@ __global__ void __launch_bounds__(1024) k_bottom_invert(LevelDesc L, const doubl
         if (tid == 0) *ok = 0;
         return;
     }
-    double a = 0.0;
-    for (int t = tid; t < nu * nu; t += nt) {
-        const double v = Ag[t];
-        M[(t % nu) * nu + t / nu] = v;
-        a = fmax(a, fabs(v));
-    }
-    // block max of |A| (every warp's lane 0 folds into amax_s)
-    for (int o = 16; o > 0; o >>= 1) a = fmax(a, __shfl_xor_sync(0xffffffffu, a, o));
-    if (tid == 0) {
-        amax_s = 0.0;
-        bad_s = 0;
+    for (int t = tid; t < nu * nu; t += nt) M[(t % nu) * nu + t / nu] = Ag[t];
+    if (tid == 0) bad_s = 0;
+    __syncthreads();
+    for (int r = tid; r < nu; r += nt) {
+        double a = 0.0;
+        for (int c = 0; c < nu; c++) a = fmax(a, fabs(M[r * nu + c]));
+        scale[r] = row_factor(a);
     }
     __syncthreads();
-    if (lane == 0) atomicMax(reinterpret_cast<unsigned long long*>(&amax_s), (unsigned long long)__double_as_longlong(a));
+    for (int t = tid; t < nu * nu; t += nt) M[t] *= scale[t / nu];
     __syncthreads();
-    const double tol = 1e-13 * amax_s;
     for (int k = 0; k < nu; k++) {
         if (tid < 32) {
             // pivot: the largest |M(r, k)| for r >= k (ties to the lower row)
@@ -482,7 +492,7 @@ __global__ void __launch_bounds__(1024) k_bottom_invert(LevelDesc L, const doubl
             }
             if (lane == 0) {
                 piv[k] = br;
-                if (!(best > tol)) bad_s = 1;
+                if (!(best > PIVOT_MIN)) bad_s = 1;
             }
         }
         __syncthreads();
@@ -524,8 +534,9 @@ __global__ void __launch_bounds__(1024) k_bottom_invert(LevelDesc L, const doubl
         __syncthreads();
     }
     for (int t = tid; t < nu * nu; t += nt) {
-        if (inv64) inv64[t] = M[t];
-        if (inv32) inv32[t] = (float)M[t];
+        const double v = M[t] * scale[t % nu];
+        if (inv64) inv64[t] = v;
+        if (inv32) inv32[t] = (float)v;
     }
     if (tid == 0) *ok = 1;
 }
@@ -533,25 +544,36 @@ __global__ void __launch_bounds__(1024) k_bottom_invert(LevelDesc L, const doubl
 constexpr int INV_NB = 8;           // panel width
 constexpr int EXACT_MAX = 1536;     // unknowns
 
-// M = A row-major, perm state reset; the largest |entry| into *amax (bits)
-__global__ void __launch_bounds__(256) k_inv_begin(int nu, const double* __restrict__ A, double* __restrict__ M,
-                                                   unsigned long long* amax)
+// The factor of every row of A (column-major); a block takes 32 rows.
+__global__ void __launch_bounds__(256) k_inv_scale(int nu, const double* __restrict__ A, double* __restrict__ scale)
+{
+    __shared__ double m[8][32];
+    const int x = threadIdx.x & 31, y = threadIdx.x >> 5, r = blockIdx.x * 32 + x;
+    double a = 0.0;
+    if (r < nu) {
+#pragma unroll 8
+        for (int c = y; c < nu; c += 8) a = fmax(a, fabs(A[(long long)c * nu + r]));
+    }
+    m[y][x] = a;
+    __syncthreads();
+    if (y || r >= nu) return;
+    for (int q = 1; q < 8; q++) a = fmax(a, m[q][x]);
+    scale[r] = row_factor(a);
+}
+
+// M = A with scaled rows, row-major
+__global__ void __launch_bounds__(256) k_inv_begin(int nu, const double* __restrict__ A,
+                                                   const double* __restrict__ scale, double* __restrict__ M)
 {
     __shared__ double t[32][33];
     const int x = threadIdx.x & 31, y = threadIdx.x >> 5;
     const int r0 = blockIdx.x * 32, c0 = blockIdx.y * 32;
-    double a = 0;
+    const double f = r0 + x < nu ? scale[r0 + x] : 0.0;
     for (int q = y; q < 32; q += 8)   // column c0 + q, rows r0 + x
-        if (c0 + q < nu && r0 + x < nu) {
-            const double v = A[(long long)(c0 + q) * nu + r0 + x];
-            t[q][x] = v;
-            a = fmax(a, fabs(v));
-        }
+        if (c0 + q < nu && r0 + x < nu) t[q][x] = A[(long long)(c0 + q) * nu + r0 + x] * f;
     __syncthreads();
     for (int q = y; q < 32; q += 8)
         if (r0 + q < nu && c0 + x < nu) M[(long long)(r0 + q) * nu + c0 + x] = t[x][q];
-    for (int o = 16; o > 0; o >>= 1) a = fmax(a, __shfl_xor_sync(0xffffffffu, a, o));
-    if (x == 0) atomicMax(amax, (unsigned long long)__double_as_longlong(a));
 }
 
 // Gauss-Jordan on columns k .. k + w of M (w <= INV_NB): T (nu x INV_NB), the
@@ -559,14 +581,13 @@ __global__ void __launch_bounds__(256) k_inv_begin(int nu, const double* __restr
 template <int INV_ROWS>   // rows a thread holds: blocks of 1024 (one row) or 768 (two) threads at most
 __global__ void __launch_bounds__(INV_ROWS == 1 ? 1024 : 768) k_inv_panel(int nu, int k, const double* __restrict__ M,
                                                     double* __restrict__ T, int* __restrict__ perm,
-                                                    int* __restrict__ piv, const unsigned long long* amax, int* ok)
+                                                    int* __restrict__ piv, int* ok)
 {
     __shared__ double best_s[32], prow[INV_NB + 1], srow[INV_NB];
     __shared__ int row_s[32], src_s[2];
     if (!*ok) return;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
     const int w = min(INV_NB, nu - k);
-    const double tol = 1e-13 * __longlong_as_double((long long)*amax);
     double a[INV_ROWS][INV_NB];
     int src[INV_ROWS];
 #pragma unroll
@@ -614,7 +635,7 @@ __global__ void __launch_bounds__(INV_ROWS == 1 ? 1024 : 768) k_inv_panel(int nu
                 br = orow;
             }
         }
-        if (!(best > tol)) {   // uniform over the CTA
+        if (!(best > PIVOT_MIN)) {   // uniform over the CTA
             if (tid == 0) *ok = 0;
             return;
         }
@@ -698,9 +719,10 @@ __global__ void __launch_bounds__(256) k_inv_update(int nu, int k, const double*
 }
 
 // Undo the row interchanges (swap columns k <-> piv[k], last first) on the way
-// into the row-major inverses.
+// into the row-major inverses, and the rows' factors into their columns.
 __global__ void __launch_bounds__(256) k_inv_end(int nu, const double* __restrict__ M, const int* __restrict__ piv,
-                                                 double* __restrict__ inv64, float* __restrict__ inv32, const int* ok)
+                                                 const double* __restrict__ scale, double* __restrict__ inv64,
+                                                 float* __restrict__ inv32, const int* ok)
 {
     __shared__ int col[EXACT_MAX];
     __shared__ int pv[EXACT_MAX];
@@ -719,7 +741,7 @@ __global__ void __launch_bounds__(256) k_inv_end(int nu, const double* __restric
     __syncthreads();
     for (int r = blockIdx.x; r < nu; r += gridDim.x)
         for (int j = threadIdx.x; j < nu; j += blockDim.x) {
-            const double v = M[(long long)r * nu + col[j]];
+            const double v = M[(long long)r * nu + col[j]] * scale[j];
             if (inv64) inv64[(long long)r * nu + j] = v;
             if (inv32) inv32[(long long)r * nu + j] = (float)v;
         }
@@ -734,11 +756,11 @@ bool use_exact_bottom()
 
 bool bottom_exact_fits(const LevelDesc& L) { return !L.singular() && 3 * L.count() <= EXACT_MAX; }
 
-// Work of the panel elimination: two copies of the matrix, T, perm, piv, amax.
+// Work of the panel elimination: two copies of the matrix, T, scale, perm, piv.
 size_t bottom_invert_work_bytes(const LevelDesc& L)
 {
     const size_t nu = 3 * (size_t)L.count();
-    return bottom_dense_fits(L) ? 0 : (2 * nu * nu + nu * INV_NB + 1) * sizeof(double) + 2 * nu * sizeof(int);
+    return bottom_dense_fits(L) ? 0 : (2 * nu * nu + nu * INV_NB + nu) * sizeof(double) + 2 * nu * sizeof(int);
 }
 
 // *ok = 1 and the inverses of A, or *ok = 0 (a kernel of the chain that finds
@@ -754,17 +776,18 @@ void launch_bottom_invert(cudaStream_t st, const LevelDesc& L, const double* A, 
     }
     const size_t n2 = (size_t)nu * nu;
     double *M0 = work, *M1 = work + n2, *T = work + 2 * n2;
-    unsigned long long* amax = (unsigned long long*)(T + (size_t)nu * INV_NB);
-    int *perm = (int*)(amax + 1), *piv = perm + nu;
+    double* scale = T + (size_t)nu * INV_NB;
+    int *perm = (int*)(scale + nu), *piv = perm + nu;
     const dim3 tiles((nu + 31) / 32, (nu + 31) / 32);
     const int rows = nu <= 1024 ? 1 : 2, threads = ((nu + rows - 1) / rows + 31) / 32 * 32;
-    cudaMemsetAsync(amax, 0, sizeof(*amax), st);
     cudaMemsetAsync(ok, 1, sizeof(int), st);   // any value but 0
-    k_inv_begin<<<tiles, 256, 0, st>>>(nu, A, M0, amax);
+    k_inv_scale<<<(nu + 31) / 32, 256, 0, st>>>(nu, A, scale);
+    k_inv_begin<<<tiles, 256, 0, st>>>(nu, A, scale, M0);
+    count_launch();
     count_launch();
     for (int k = 0; k < nu; k += INV_NB) {
-        if (rows == 1) k_inv_panel<1><<<1, threads, 0, st>>>(nu, k, M0, T, perm, piv, amax, ok);
-        else k_inv_panel<2><<<1, threads, 0, st>>>(nu, k, M0, T, perm, piv, amax, ok);
+        if (rows == 1) k_inv_panel<1><<<1, threads, 0, st>>>(nu, k, M0, T, perm, piv, ok);
+        else k_inv_panel<2><<<1, threads, 0, st>>>(nu, k, M0, T, perm, piv, ok);
         k_inv_update<<<tiles, 256, 0, st>>>(nu, k, M0, M1, T, perm, ok);
         count_launch();
         count_launch();
@@ -772,7 +795,7 @@ void launch_bottom_invert(cudaStream_t st, const LevelDesc& L, const double* A, 
         M0 = M1;
         M1 = t;
     }
-    k_inv_end<<<64, 256, 0, st>>>(nu, M0, piv, inv64, inv32, ok);
+    k_inv_end<<<64, 256, 0, st>>>(nu, M0, piv, scale, inv64, inv32, ok);
     count_launch();
 }
 
