@@ -125,8 +125,8 @@ struct agb_op_s {
     double* bottom_work = nullptr;
     double* bottom_A = nullptr;   // dense coarsest-level operator (small bottom levels)
     bool bottom_exact = false;    // the cycles take the exact coarsest solve (AGB_BOTTOM_EXACT)
-    double* bottom_inv64 = nullptr;   // its inverse for the FP64 cycles
-    float* bottom_inv32 = nullptr;    // and for the FP32 cycles
+    double* bottom_inv64 = nullptr;   // its inverse
+    float* bottom_inv32 = nullptr;    // and for the FP32 cycles of a dense level
     double* bottom_iwork = nullptr;   // work of the panel elimination
     int* bottom_inv_ok = nullptr;     // device flag: the inverse exists
     int* d_ret = nullptr;
@@ -464,18 +464,18 @@ agb_status prepare_bottom(agb_solver s, bool fp32)
     if (!fp32 && s->p.fixed_iter > 0) return AGB_OK;
     if (op->lev.size() == 1 && !(fp32 && bottom_dense_fits(bl.L))) return AGB_OK;
     const size_t n2 = bottom_dense_bytes(bl.L) / sizeof(double), nw = bottom_invert_work_bytes(bl.L) / sizeof(double);
-    const bool dense = bottom_dense_fits(bl.L);
+    const bool dense = bottom_dense_fits(bl.L), inv32 = fp32 && dense;   // above the dense size both are FP64
     if ((!op->bottom_A && op->alloc(&op->bottom_A, n2) != AGB_OK) ||
         (!op->bottom_iwork && nw && op->alloc(&op->bottom_iwork, nw + 1) != AGB_OK) ||
         (!op->bottom_inv_ok && op->alloc(&op->bottom_inv_ok, 1) != AGB_OK) ||
-        (fp32 && !op->bottom_inv32 && op->alloc(&op->bottom_inv32, n2) != AGB_OK) ||
-        (!fp32 && !op->bottom_inv64 && op->alloc(&op->bottom_inv64, n2) != AGB_OK)) {
+        (inv32 && !op->bottom_inv32 && op->alloc(&op->bottom_inv32, n2) != AGB_OK) ||
+        (!inv32 && !op->bottom_inv64 && op->alloc(&op->bottom_inv64, n2) != AGB_OK)) {
         cudaGetLastError();
         return AGB_OK;
     }
     if (!dense) launch_bottom_assemble(op->st, op->sym, bl.L, op->bc, op->uniform, bl.ddw64, op->bottom_A);
-    launch_bottom_invert(op->st, bl.L, op->bottom_A, fp32 ? nullptr : op->bottom_inv64,
-                         fp32 ? op->bottom_inv32 : nullptr, op->bottom_iwork, op->bottom_inv_ok);
+    launch_bottom_invert(op->st, bl.L, op->bottom_A, inv32 ? nullptr : op->bottom_inv64,
+                         inv32 ? op->bottom_inv32 : nullptr, op->bottom_iwork, op->bottom_inv_ok);
     CK(cudaGetLastError());
     s->exact_bottom = true;
     return AGB_OK;
@@ -600,16 +600,16 @@ template <typename T> struct Engine {
     void bottom()
     {
         Level& v = lv(bot());
-        const T* inv = exact_bottom ? A::inv(op) : nullptr;
         if (bottom_dense_fits(v.L) && op->bottom_A) {
             launch_bottom_dense<T>(op->st, v.L, op->bottom_A, v.diag64, A::cor(v), A::res(v), p.bottom_max_iter,
                                    p.bottom_tol_rel, p.bottom_tol_abs, op->d_ret, p.bottom_smooth, p.final_smooth,
-                                   op->omega, inv, op->bottom_inv_ok);
+                                   op->omega, exact_bottom ? A::inv(op) : nullptr, op->bottom_inv_ok);
             return;
         }
         launch_bottom<T>(op->st, op->sym, v.L, op->bc, op->uniform, v.ddw64, v.diag64, A::cor(v), A::res(v),
                          op->bottom_work, p.bottom_max_iter, p.bottom_tol_rel, p.bottom_tol_abs, op->d_ret,
-                         p.bottom_smooth, p.final_smooth, op->omega, inv, op->bottom_inv_ok);
+                         p.bottom_smooth, p.final_smooth, op->omega, exact_bottom ? op->bottom_inv64 : nullptr,
+                         op->bottom_inv_ok);
     }
     // MLMG::mgVcycle(amrlev = 0, mglev_top)
     void vcycle(int top)

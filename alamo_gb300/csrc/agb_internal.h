@@ -334,7 +334,7 @@ template <typename T>
 void launch_bottom(cudaStream_t st, int sym, const LevelDesc& L, const BCTable& bc, bool uniform,
                    const double* ddw64, const double* diag64, T* cor, const T* res, double* work, int maxiter,
                    double tol_rel, double tol_abs, int* ret_slot, int nub, int nuf, double omega,
-                   const T* inv = nullptr, const int* inv_ok = nullptr);
+                   const double* inv = nullptr, const int* inv_ok = nullptr);
 
 void launch_newton_rhs(cudaStream_t st, int sym, const LevelDesc& L, const BCTable& bc, const double* ddw,
                        const double* F0, const double* u, const double* b, double* rhs, double* dw_work);

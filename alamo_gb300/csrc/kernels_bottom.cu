@@ -145,19 +145,20 @@ __device__ void cta_mean3(const LevelDesc& L, const double* v, double* red, doub
              c_ < 3; c_++)                                                                               \
             for (long long q = c_ * L.S + L.idx(i_, j_, k_), once_ = 0; once_ < 1; once_++)
 
-// cor = A^-1 res with the inverse row-major: one row a warp, the right-hand
-// side in shared memory.  Every CTA of the grid takes its rows.
-template <typename T>
-__device__ __forceinline__ void exact_product(const LevelDesc& L, const T* __restrict__ inv, T* __restrict__ cor,
-                                              const T* __restrict__ res, T* __restrict__ xs, int* ret_slot)
+// cor = A^-1 res with the inverse row-major, in the inverse's arithmetic I: one
+// row a warp, the right-hand side in shared memory.  Every CTA of the grid takes
+// its rows.
+template <typename T, typename I>
+__device__ __forceinline__ void exact_product(const LevelDesc& L, const I* __restrict__ inv, T* __restrict__ cor,
+                                              const T* __restrict__ res, I* __restrict__ xs, int* ret_slot)
 {
     const int cnt = (int)L.count(), nu = 3 * cnt;
-    for (int q = threadIdx.x; q < nu; q += blockDim.x) xs[q] = __ldcg(res + dense_to_padded(L, q, cnt));
+    for (int q = threadIdx.x; q < nu; q += blockDim.x) xs[q] = (I)__ldcg(res + dense_to_padded(L, q, cnt));
     __syncthreads();
     const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
     for (int row = blockIdx.x * nw + (threadIdx.x >> 5); row < nu; row += gridDim.x * nw) {
-        const T* a = inv + (long long)row * nu;
-        T y0 = 0, y1 = 0;
+        const I* a = inv + (long long)row * nu;
+        I y0 = 0, y1 = 0;
         int j = lane;
         for (; j + 32 < nu; j += 64) {
             y0 += a[j] * xs[j];
@@ -166,7 +167,7 @@ __device__ __forceinline__ void exact_product(const LevelDesc& L, const T* __res
         if (j < nu) y0 += a[j] * xs[j];
         y0 += y1;
         for (int o = 16; o > 0; o >>= 1) y0 += __shfl_xor_sync(0xffffffffu, y0, o);
-        if (lane == 0) cor[dense_to_padded(L, row, cnt)] = y0;
+        if (lane == 0) cor[dense_to_padded(L, row, cnt)] = (T)y0;
     }
     if (blockIdx.x == 0 && threadIdx.x == 0 && ret_slot) *ret_slot = 0;
 }
@@ -178,12 +179,12 @@ __global__ void __launch_bounds__(BOT_THREADS) k_bottom(LevelDesc L, BCTable bc,
                                                         const T* __restrict__ res, double* __restrict__ work,
                                                         int maxiter, double eps_rel, double eps_abs, int nub,
                                                         int nuf, double omega, int* ret_slot,
-                                                        const T* __restrict__ inv, const int* __restrict__ inv_ok)
+                                                        const double* __restrict__ inv, const int* __restrict__ inv_ok)
 {
     __shared__ double red[33];
     if (inv && *inv_ok) {
         extern __shared__ __align__(16) unsigned char bsm_raw[];
-        exact_product<T>(L, inv, cor, res, reinterpret_cast<T*>(bsm_raw), ret_slot);
+        exact_product(L, inv, cor, res, reinterpret_cast<double*>(bsm_raw), ret_slot);
         return;
     }
     if (blockIdx.x) return;   // the BiCGStab solve is one CTA's
@@ -390,7 +391,7 @@ __global__ void __launch_bounds__(DENSE_MAX) k_bottom_dense(LevelDesc L, const d
     __shared__ R red[2 * 3 * 32];
     const int nu = 3 * (int)L.count();
     if (inv && *inv_ok) {
-        exact_product<T>(L, inv, cor, res, reinterpret_cast<T*>(dsm_raw), ret_slot);
+        exact_product(L, inv, cor, res, reinterpret_cast<T*>(dsm_raw), ret_slot);
         return;
     }
     if (blockIdx.x) return;   // the BiCGStab solve is one CTA's
@@ -407,7 +408,10 @@ bool bottom_dense_fits(const LevelDesc& L) { return 3 * L.count() <= DENSE_MAX; 
 // ---------------------------------------------------------------------------
 // Exact coarsest solve.  Once per solve the dense operator (FP64,
 // column-major) is inverted by Gauss-Jordan elimination with partial pivoting
-// in FP64 and stored row-major in FP64 (FP64 cycles) and FP32 (FP32 cycles).  A
+// in FP64 and stored row-major in FP64, or in FP32 for the FP32 cycles of a level
+// of up to DENSE_MAX unknowns, whose BiCGStab is in FP32 as well.  (Above, the
+// BiCGStab of both is FP64, and so is the product: an inverse in 24 bits is off
+// by the level's condition times 6e-8, which grows with the level.)  A
 // displacement row is 1 and an interior row C/dx^2, so each row is first scaled
 // to a largest |entry| in [1, 2) by a power of two, which the columns of the
 // inverse take back: (S A)^-1 S = A^-1, exact, and the same pivots in any units.  A
@@ -859,12 +863,13 @@ template void launch_bottom_dense<float>(cudaStream_t, const LevelDesc&, const d
 template <typename T>
 void launch_bottom(cudaStream_t st, int sym, const LevelDesc& L, const BCTable& bc, bool uniform, const double* ddw64,
                    const double* diag64, T* cor, const T* res, double* work, int maxiter, double tol_rel,
-                   double tol_abs, int* ret_slot, int nub, int nuf, double omega, const T* inv, const int* inv_ok)
+                   double tol_abs, int* ret_slot, int nub, int nuf, double omega, const double* inv,
+                   const int* inv_ok)
 {
     const Geo<double> g = make_geo<double>(L);
     const size_t nu = 3 * (size_t)L.count();
     const unsigned grid = inv ? (unsigned)((nu + BOT_THREADS / 32 - 1) / (BOT_THREADS / 32)) : 1u;
-    const size_t smem = inv ? nu * sizeof(T) : 0;
+    const size_t smem = inv ? nu * sizeof(double) : 0;
     if (sym == SYM_ISO)
         k_bottom<T, SYM_ISO><<<grid, BOT_THREADS, smem, st>>>(L, bc, g, uniform ? 1 : 0, ddw64, diag64, cor, res, work,
                                                               maxiter, tol_rel, tol_abs, nub, nuf, omega, ret_slot,
@@ -881,7 +886,7 @@ template void launch_bottom<double>(cudaStream_t, int, const LevelDesc&, const B
                                     int, double, const double*, const int*);
 template void launch_bottom<float>(cudaStream_t, int, const LevelDesc&, const BCTable&, bool, const double*,
                                    const double*, float*, const float*, double*, int, double, double, int*, int, int,
-                                   double, const float*, const int*);
+                                   double, const double*, const int*);
 
 }  // namespace agb
 
