@@ -42,6 +42,9 @@ def _ptr(a, dtype=np.float64):
             raise TypeError("expected a C-contiguous %s array" % np.dtype(dtype).name)
         return a.ctypes.data_as(ctypes.c_void_p), _lib.AGB_MEM_HOST
     if hasattr(a, "data_ptr"):
+        # the kernels read sizeof(dtype) bytes an entry, whatever the tensor holds
+        if str(getattr(a, "dtype", dtype)).rsplit(".", 1)[-1] != str(np.dtype(dtype)):
+            raise TypeError("expected a %s tensor, got %s" % (np.dtype(dtype).name, a.dtype))
         if not a.is_contiguous():
             raise TypeError("expected a contiguous tensor")
         mem = _lib.AGB_MEM_DEVICE if getattr(a, "is_cuda", False) else _lib.AGB_MEM_HOST
