@@ -729,6 +729,18 @@ agb_status gcr_setup(agb_batch b, int m)
     return AGB_OK;
 }
 
+// No graph may be running: every call that replays one ends with a synchronisation.
+void drop_graphs(agb_batch b)
+{
+    if (b->g64) cudaGraphExecDestroy(b->g64);
+    if (b->g32) cudaGraphExecDestroy(b->g32);
+    b->g64 = b->g32 = nullptr;
+    for (cudaGraphExec_t& g : b->gk) {
+        if (g) cudaGraphExecDestroy(g);
+        g = nullptr;
+    }
+}
+
 }  // namespace
 
 extern "C" {
@@ -785,10 +797,7 @@ agb_status agb_batch_destroy(agb_batch b)
 {
     if (!b) return AGB_OK;
     if (b->st) cudaStreamSynchronize(b->st);
-    if (b->g64) cudaGraphExecDestroy(b->g64);
-    if (b->g32) cudaGraphExecDestroy(b->g32);
-    for (cudaGraphExec_t g : b->gk)
-        if (g) cudaGraphExecDestroy(g);
+    drop_graphs(b);
     for (void* v : b->allocs) cudaFree(v);
     if (b->h_norms) cudaFreeHost(b->h_norms);
     if (b->e0) cudaEventDestroy(b->e0);
@@ -801,12 +810,15 @@ agb_status agb_batch_destroy(agb_batch b)
 agb_status agb_batch_set_bc(agb_batch b, const agb_bc* bc)
 {
     if (!b || !bc) return bfail(AGB_BADARG, "null argument");
+    bool same = true;
     for (int f = 0; f < AGB_NFACES; f++)
         for (int c = 0; c < 3; c++) {
             if (bc->type[f][c] < AGB_BC_DISP || bc->type[f][c] > AGB_BC_NONE) return bfail(AGB_BADARG, "bad BC type");
+            same = same && b->bc.type[f][c] == (int8_t)bc->type[f][c];
             b->bc.type[f][c] = (int8_t)bc->type[f][c];
             b->bc.val[f][c] = bc->val[f][c];
         }
+    if (!same) drop_graphs(b);   // the captured kernels hold the types of the rows
     b->prepared = false;
     return AGB_OK;
 }
@@ -858,7 +870,8 @@ agb_status agb_batch_solve(agb_batch b, double tol_rel, double tol_abs, agb_solv
     long long replayed = 0;
     BCK(cudaEventRecord(b->e0, b->st));
     // right-hand side of the Newton step at u = 0 and x = 0
-    launch_batch_rhs(b->st, b->sym, b->grid, v0.d_probs, v0.d_t32_full, (int)v0.t32_full.size(), v0.ddw64, b->F0, b->b64);
+    launch_batch_rhs(b->st, b->sym, b->grid, v0.d_probs, v0.d_t32_full, (int)v0.t32_full.size(), b->bc, v0.ddw64, b->F0,
+                     b->b64);
     if (b->per[0] && b->per[1] && b->per[2]) project<double>(b, nullptr, b->b64, false);
     BCK(cudaMemsetAsync(b->x64, 0, sizeof(double) * v0.nvec, b->st));
     b->active.assign(np, 1);

@@ -185,7 +185,7 @@ void launch_batch_bottom_rows(cudaStream_t st, const BProb* probs, const int* pl
                               const int* active, const float* rows, const double* diag, float* cor, const float* res,
                               int maxiter, double tol_rel, double tol_abs, int nub, int nuf, double omega);
 void launch_batch_rhs(cudaStream_t st, int sym, int grid, const BProb* probs, const BTile* tiles, int ntiles,
-                      const double* ddw, const double* F0, double* rhs);
+                      const BCTable& bc, const double* ddw, const double* F0, double* rhs);
 void launch_batch_mean_stress(cudaStream_t st, int sym, int grid, const BProb* probs, const BTile* tiles, int ntiles,
                               const double* ddw, const double* F0, const double* u, double* sums);
 // per-problem component sums of y over the stored nodes into sums (3 per

@@ -1113,12 +1113,28 @@ __global__ void __launch_bounds__(ROWS_MAX) k_batch_bottom_rows(const BProb* __r
                                      eps_abs, nub, nuf, omega, nullptr);
 }
 
-// rhs = -div(C : (0 - F0)) with a uniform eigenstrain F0 per problem: the
-// Newton right-hand side at u = 0 of an affine model (Newton.H:199-231,
-// Model/Solid/Affine/Isotropic.H:42-45) on a fully periodic box.
+// Faces a node lies on: the directions that are not periodic.
+__device__ __forceinline__ bool node_faces(const LevelDesc& L, int i, int j, int k, int mn[3], int mx[3])
+{
+    const int pos[3] = {i, j, k};
+    bool bnd = false;
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+        mn[d] = !L.per[d] && pos[d] == 0;
+        mx[d] = !L.per[d] && pos[d] == L.n[d];
+        bnd = bnd || mn[d] || mx[d];
+    }
+    return bnd;
+}
+
+// rhs = b - div(C : (0 - F0)) with a uniform eigenstrain F0 per problem: the
+// Newton right-hand side at u = 0 of an affine model (Newton.H:144-231,
+// Model/Solid/Affine/Isotropic.H:42-45).  On the faces of a box that is not
+// periodic in every direction the boundary condition's value less its row of the
+// same stress (a node there has no neighbour on one side); b is 0 elsewhere.
 template <int SYM>
 __global__ void __launch_bounds__(256) k_batch_rhs(const BProb* __restrict__ probs, const BTile* __restrict__ tiles,
-                                                   int ntiles, const double* __restrict__ ddw,
+                                                   int ntiles, BCTable bc, const double* __restrict__ ddw,
                                                    const double* __restrict__ F0, double* __restrict__ rhs)
 {
     for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
@@ -1128,24 +1144,34 @@ __global__ void __launch_bounds__(256) k_batch_rhs(const BProb* __restrict__ pro
         int i, j, k;
         if (!tile_node<32, 4, 2>(tl, L, i, j, k)) continue;
         const Nbr nb = make_nbr(L, i, j, k);
-        double E[3][3];
+        double E[3][3], b[3] = {0, 0, 0}, ret[3] = {0, 0, 0};
         for (int a = 0; a < 3; a++)
             for (int c = 0; c < 3; c++) E[a][c] = 0.0 - F0[tl.prob * 9 + a * 3 + c];
-        double ret[3] = {0, 0, 0};
-        for (int d = 0; d < 3; d++) {
-            // (C+ - C-) : E, the difference of the moduli first
-            double dc[NCoef<SYM>::value], D[3][3];
-            for (int m = 0; m < NCoef<SYM>::value; m++)
-                dc[m] = ddw[P.co + m * L.S + nb.base + nb.o[d][2]] - ddw[P.co + m * L.S + nb.base + nb.o[d][0]];
-            c_mul_mat<double, SYM>(dc, E, D);
-            for (int r = 0; r < 3; r++) ret[r] += D[r][d] * P.h1[d];
+        int mn[3], mx[3];
+        if (node_faces(L, i, j, k, mn, mx)) {
+            double c[NCoef<SYM>::value], S[3][3], nrm[3];
+            const double zero[3] = {0, 0, 0}, G[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
+            for (int m = 0; m < NCoef<SYM>::value; m++) c[m] = ddw[P.co + m * L.S + nb.base];
+            c_mul_mat<double, SYM>(c, E, S);
+            const int face = face_of(mn, mx, nrm);
+            bc_set<double>(bc.type[face], zero, G, S, nrm, ret);
+            for (int r = 0; r < 3; r++) b[r] = bc.val[face][r];
+        } else {
+            for (int d = 0; d < 3; d++) {
+                // (C+ - C-) : E, the difference of the moduli first
+                double dc[NCoef<SYM>::value], D[3][3];
+                for (int m = 0; m < NCoef<SYM>::value; m++)
+                    dc[m] = ddw[P.co + m * L.S + nb.base + nb.o[d][2]] - ddw[P.co + m * L.S + nb.base + nb.o[d][0]];
+                c_mul_mat<double, SYM>(dc, E, D);
+                for (int r = 0; r < 3; r++) ret[r] += D[r][d] * P.h1[d];
+            }
         }
-        for (int r = 0; r < 3; r++) rhs[P.vo + r * L.S + nb.base] = 0.0 - ret[r];
+        for (int r = 0; r < 3; r++) rhs[P.vo + r * L.S + nb.base] = b[r] - ret[r];
     }
 }
 
 // Per-problem sums of sigma = C : (grad u - F0) over the stored nodes
-// (central differences; fully periodic boxes), for the homogenized stress.  A
+// (central differences, one-sided on faces), for the homogenized stress.  A
 // CTA takes a contiguous part of the list and a thread keeps its six sums while
 // the problem stays the same: reducing nine a tile by shuffles was most of its
 // FP64 work (17.3 M nodes 2.8 ms before, 1.2 now).
@@ -1182,11 +1208,15 @@ __global__ void __launch_bounds__(256) k_batch_mean_stress(const BProb* __restri
         if (!tile_node<32, 4, 2>(tl, L, i, j, k)) continue;
         const Nbr nb = make_nbr(L, i, j, k);
         double G[3][3], S[3][3], c[NCoef<SYM>::value];
-        for (int p = 0; p < 3; p++)
-            for (int d = 0; d < 3; d++)
-                G[p][d] = (u[P.vo + p * L.S + nb.base + nb.o[d][2]] - u[P.vo + p * L.S + nb.base + nb.o[d][0]]) *
-                              P.h1[d] -
+        int mn[3], mx[3];
+        node_faces(L, i, j, k, mn, mx);
+        for (int d = 0; d < 3; d++) {
+            const long long hi = mx[d] ? 0 : nb.o[d][2], lo = mn[d] ? 0 : nb.o[d][0];
+            const double h = mn[d] || mx[d] ? P.i1[d] : P.h1[d];
+            for (int p = 0; p < 3; p++)
+                G[p][d] = (u[P.vo + p * L.S + nb.base + hi] - u[P.vo + p * L.S + nb.base + lo]) * h -
                           F0[tl.prob * 9 + p * 3 + d];
+        }
         for (int m = 0; m < NCoef<SYM>::value; m++) c[m] = ddw[P.co + m * L.S + nb.base];
         c_mul_mat<double, SYM>(c, G, S);
         acc[0] += S[0][0];
@@ -1566,10 +1596,10 @@ void launch_batch_bottom_rows(cudaStream_t st, const BProb* probs, const int* pl
 }
 
 void launch_batch_rhs(cudaStream_t st, int sym, int grid, const BProb* probs, const BTile* tiles, int ntiles,
-                      const double* ddw, const double* F0, double* rhs)
+                      const BCTable& bc, const double* ddw, const double* F0, double* rhs)
 {
-    if (sym == SYM_ISO) k_batch_rhs<SYM_ISO><<<grid, 256, 0, st>>>(probs, tiles, ntiles, ddw, F0, rhs);
-    else k_batch_rhs<SYM_MM><<<grid, 256, 0, st>>>(probs, tiles, ntiles, ddw, F0, rhs);
+    if (sym == SYM_ISO) k_batch_rhs<SYM_ISO><<<grid, 256, 0, st>>>(probs, tiles, ntiles, bc, ddw, F0, rhs);
+    else k_batch_rhs<SYM_MM><<<grid, 256, 0, st>>>(probs, tiles, ntiles, bc, ddw, F0, rhs);
     count_launch();
 }
 

@@ -195,10 +195,11 @@ agb_status agb_strain_energy(agb_op op, const double* u, double* eps9, double* e
  * by timing on the batch at the first solve.  Each problem's right-hand side is
  * the Newton step at u = 0 of an affine model with a uniform eigenstrain F0
  * (9 doubles per problem; F0 = -macroscopic strain), the setting of
- * Model/Solid/Affine with Newton.H:199-231.  Per problem the algorithm is the
- * single-box solver's, V-cycles; params.precision selects plain FP64 or FP32
- * cycles in FP64 refinement.  For fully periodic boxes the solution is returned
- * modulo rigid translation (zero mean). */
+ * Model/Solid/Affine with Newton.H:199-231; on faces that are not periodic it
+ * holds the values of agb_batch_set_bc (displacement 0 unless set).  Per problem
+ * the algorithm is the single-box solver's, V-cycles; params.precision selects
+ * plain FP64 or FP32 cycles in FP64 refinement.  For fully periodic boxes the
+ * solution is returned modulo rigid translation (zero mean). */
 typedef struct agb_batch_s* agb_batch;
 agb_status agb_batch_create(int nprob, const int* n_cells, const double* dx, const int periodic[3], int sym,
                             const agb_solver_params* params, agb_batch* out);
