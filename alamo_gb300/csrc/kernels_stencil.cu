@@ -716,10 +716,12 @@ static void rows_dispatch(cudaStream_t st, const LevelDesc& L, const BCTable& bc
             const int chunks = (L.n[2] - 1 + kz - 1) / kz;
             const long long per_z = (long long)gx * gy * COL_X * COL_Y;
             const int shell_z = (int)((shell_count(L, 1) + per_z - 1) / per_z);
-            pdl_launch(k_column<T, SYM, MODE, CUBE>, dim3(gx, gy, chunks + shell_z), dim3(COL_X, COL_Y), 0, st, L, bc,
-                       g, uniform ? 1 : 0, kz, chunks, ddw, div, x, b, diag, out, omega, norm_slot);
-            count_launch();
-            return;
+            if (gy <= 65535 && chunks + shell_z <= 65535) {   // the most blocks a grid has in y and z
+                pdl_launch(k_column<T, SYM, MODE, CUBE>, dim3(gx, gy, chunks + shell_z), dim3(COL_X, COL_Y), 0, st, L,
+                           bc, g, uniform ? 1 : 0, kz, chunks, ddw, div, x, b, diag, out, omega, norm_slot);
+                count_launch();
+                return;
+            }
         }
     }
     long long threads = L.count();

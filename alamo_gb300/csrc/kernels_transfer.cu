@@ -20,8 +20,8 @@ static inline dim3 grid_for(const LevelDesc& L, dim3 blk)
     return dim3((L.nn[0] + blk.x - 1) / blk.x, (L.nn[1] + blk.y - 1) / blk.y, (L.nn[2] + blk.z - 1) / blk.z);
 }
 
-// One coarse node and component a thread (blockIdx.z counts planes and
-// components): on the coarse levels the three components side by side are
+// One coarse node and component a thread (blockIdx.x counts blocks of a
+// row and components: the other two have only 65535): on the coarse levels the three components side by side are
 // three times the threads, and the FP64 sums a third as long.  257^3 -> 129^3
 // nodes, FP32: 103 us (27 reads and a loop over the components: 135); 9^3 -> 5^3,
 // FP64: 5.3 us (10.5).
@@ -30,9 +30,9 @@ __global__ void __launch_bounds__(256) k_restrict(LevelDesc Lf, LevelDesc Lc, co
                                                   T* __restrict__ crse, int ncomp)
 {
     pdl_entry();
-    const int I = blockIdx.x * blockDim.x + threadIdx.x;
+    const int c = blockIdx.x % ncomp, I = (blockIdx.x / ncomp) * blockDim.x + threadIdx.x;
     const int J = blockIdx.y * blockDim.y + threadIdx.y;
-    const int c = blockIdx.z % ncomp, K = (blockIdx.z / ncomp) * blockDim.z + threadIdx.z;
+    const int K = blockIdx.z * blockDim.z + threadIdx.z;
     if (I >= Lc.nn[0] || J >= Lc.nn[1] || K >= Lc.nn[2]) return;
     const RestrictNode<T> r(Lf, Lc, I, J, K);
     crse[c * Lc.S + Lc.idx(I, J, K)] = r(fine + c * Lf.S);
@@ -45,9 +45,9 @@ __global__ void __launch_bounds__(256) k_interp(LevelDesc Lf, LevelDesc Lc, T* _
                                                 const T* __restrict__ crse, int assign)
 {
     pdl_entry();
-    const int I = blockIdx.x * blockDim.x + threadIdx.x;
+    const int c = blockIdx.x % 3, I = (blockIdx.x / 3) * blockDim.x + threadIdx.x;
     const int J = blockIdx.y * blockDim.y + threadIdx.y;
-    const int c = blockIdx.z % 3, K = (blockIdx.z / 3) * blockDim.z + threadIdx.z;
+    const int K = blockIdx.z * blockDim.z + threadIdx.z;
     if (I >= Lc.nn[0] || J >= Lc.nn[1] || K >= Lc.nn[2]) return;
     const InterpCell<T> cell(Lf, Lc, I, J, K);
     cell(crse + c * Lc.S, fine + c * Lf.S, assign != 0);
@@ -332,7 +332,7 @@ void launch_restriction(cudaStream_t st, const LevelDesc& Lf, const LevelDesc& L
 {
     const dim3 blk = transfer_block(Lc);
     dim3 grd = grid_for(Lc, blk);
-    grd.z *= ncomp;
+    grd.x *= ncomp;
     pdl_launch(k_restrict<T>, grd, blk, 0, st, Lf, Lc, fine, crse, ncomp); count_launch();
 }
 
@@ -342,7 +342,7 @@ void launch_interpolation(cudaStream_t st, const LevelDesc& Lf, const LevelDesc&
 {
     const dim3 blk = transfer_block(Lc);
     dim3 grd = grid_for(Lc, blk);
-    grd.z *= 3;
+    grd.x *= 3;
     pdl_launch(k_interp<T>, grd, blk, 0, st, Lf, Lc, fine, crse, assign ? 1 : 0); count_launch();
 }
 
