@@ -19,6 +19,7 @@
 #include <cstdarg>
 #include <cstdint>
 #include <cstdio>
+#include <cstdlib>
 #include <cstring>
 #include <new>
 #include <string>
@@ -136,18 +137,69 @@ struct agb_op_s {
     size_t dma_bytes = 0;
     double *nw_dw = nullptr, *nw_u0 = nullptr, *nw_F0 = nullptr;   // Newton work fields, kept across calls
     int pageable_ok = 0;         // device can read pageable host memory directly
-    std::vector<void*> allocs;
+    // Device memory.  The divergence fields (make_div) only save time, so an
+    // allocation that finds no memory takes theirs and they are not made again.
+    // epoch counts what makes captured cycles stale: this, and agb_op_set_uniform.
+    std::vector<std::pair<void*, size_t>> allocs;
+    size_t held = 0, held_max = 0;   // bytes; held_max: most it may hold, 0 = no limit (AGB_OP_BYTES_MAX)
+    bool use_div = true;             // AGB_DIV=0: without divergence fields
+    int epoch = 0;
 
+    // AGB_NOMEM (without a message) or memory set to zero
+    agb_status grab(void** out, size_t bytes)
+    {
+        cudaError_t e = held_max && held + bytes > held_max ? cudaErrorMemoryAllocation : cudaMalloc(out, bytes);
+        if (e != cudaSuccess) {
+            cudaGetLastError();
+            return AGB_NOMEM;
+        }
+        allocs.push_back({*out, bytes});
+        held += bytes;
+        e = cudaMemsetAsync(*out, 0, bytes, st);
+        return e == cudaSuccess ? AGB_OK : fail(AGB_CUDA, "cudaMemsetAsync: %s", cudaGetErrorString(e));
+    }
+    void drop(void* p)
+    {
+        for (size_t i = 0; i < allocs.size(); i++)
+            if (allocs[i].first == p) {
+                cudaFree(p);
+                held -= allocs[i].second;
+                allocs.erase(allocs.begin() + i);
+                return;
+            }
+    }
+    bool give_back_div()
+    {
+        use_div = false;
+        bool any = false;
+        for (auto& lv : lev) any = any || lv.div64 || lv.div32;
+        if (!any || cudaStreamSynchronize(st) != cudaSuccess) return false;
+        for (auto& lv : lev) {
+            if (lv.div64) drop(lv.div64);
+            if (lv.div32) drop(lv.div32);
+            lv.div64 = nullptr;
+            lv.div32 = nullptr;
+        }
+        epoch++;
+        return true;
+    }
     template <typename T> agb_status alloc(T** p, size_t count)
     {
+        const size_t bytes = std::max<size_t>(count, 1) * sizeof(T);
         void* q = nullptr;
-        cudaError_t e = cudaMalloc(&q, std::max<size_t>(count, 1) * sizeof(T));
-        if (e != cudaSuccess) return fail(AGB_NOMEM, "cudaMalloc(%zu bytes): %s", count * sizeof(T), cudaGetErrorString(e));
-        e = cudaMemsetAsync(q, 0, std::max<size_t>(count, 1) * sizeof(T), st);
-        if (e != cudaSuccess) return fail(AGB_CUDA, "cudaMemsetAsync: %s", cudaGetErrorString(e));
-        allocs.push_back(q);
+        agb_status s = grab(&q, bytes);
+        if (s == AGB_NOMEM && give_back_div()) s = grab(&q, bytes);
+        if (s == AGB_NOMEM) return fail(s, "cudaMalloc(%zu bytes): out of memory", bytes);
+        if (s == AGB_OK) *p = (T*)q;
+        return s;
+    }
+    // for what a call can do without: no message, and nothing is given back for it
+    template <typename T> bool try_alloc(T** p, size_t count)
+    {
+        void* q = nullptr;
+        if (grab(&q, std::max<size_t>(count, 1) * sizeof(T)) != AGB_OK) return false;
         *p = (T*)q;
-        return AGB_OK;
+        return true;
     }
 };
 
@@ -159,6 +211,7 @@ struct agb_solver_s {
     cudaGraphExec_t g64 = nullptr, g32 = nullptr;
     int g64_fcycle = -1, g32_fcycle = -1;   // cycle kind each graph holds
     long long g64_kernels = 0, g32_kernels = 0;
+    int epoch = 0;                           // of the operator, when they were captured
     long long replayed = 0;                  // kernels executed through graph replays
     // inner FP32 GCR of the mixed solve (params.krylov > 0): directions, their
     // images, the inner residual, device scalars, the preconditioner's graph
@@ -229,8 +282,11 @@ agb_status dma_buffer(agb_op op, size_t bytes, char** out)
             op->dma = nullptr;
             op->dma_bytes = 0;
         }
-        if (cudaMalloc(&op->dma, bytes) != cudaSuccess) {
+        cudaError_t e = cudaMalloc(&op->dma, bytes);
+        if (e != cudaSuccess && op->give_back_div()) e = cudaMalloc(&op->dma, bytes);
+        if (e != cudaSuccess) {
             cudaGetLastError();
+            op->dma = nullptr;
             return fail(AGB_NOMEM, "cudaMalloc(%zu bytes) for the host copy", bytes);
         }
         op->dma_bytes = bytes;
@@ -365,15 +421,12 @@ agb_status check_level(agb_op op, int level)
 }
 
 // A level's divergence field, made from its moduli.  A field that finds no
-// memory is left out: the rows then read the moduli of the neighbours.
+// memory is left out: the rows then read the moduli of the neighbours.  Rows of
+// moduli declared uniform read neither.
 template <typename T> void make_div(agb_op op, Level& lv, const T* ddw, T** div)
 {
-    if (!stencil_uses_div(op->sym, sizeof(T) == 4, lv.L)) return;
-    if (!*div && op->alloc(div, 18 * (size_t)lv.L.S) != AGB_OK) {
-        cudaGetLastError();
-        *div = nullptr;
-        return;
-    }
+    if (op->uniform || !op->use_div || !stencil_uses_div(op->sym, sizeof(T) == 4, lv.L)) return;
+    if (!*div && !op->try_alloc(div, 18 * (size_t)lv.L.S)) return;
     launch_div_moduli<T>(op->st, lv.L, ddw, *div);
 }
 
@@ -465,14 +518,12 @@ agb_status prepare_bottom(agb_solver s, bool fp32)
     if (op->lev.size() == 1 && !(fp32 && bottom_dense_fits(bl.L))) return AGB_OK;
     const size_t n2 = bottom_dense_bytes(bl.L) / sizeof(double), nw = bottom_invert_work_bytes(bl.L) / sizeof(double);
     const bool dense = bottom_dense_fits(bl.L), inv32 = fp32 && dense;   // above the dense size both are FP64
-    if ((!op->bottom_A && op->alloc(&op->bottom_A, n2) != AGB_OK) ||
-        (!op->bottom_iwork && nw && op->alloc(&op->bottom_iwork, nw + 1) != AGB_OK) ||
-        (!op->bottom_inv_ok && op->alloc(&op->bottom_inv_ok, 1) != AGB_OK) ||
-        (inv32 && !op->bottom_inv32 && op->alloc(&op->bottom_inv32, n2) != AGB_OK) ||
-        (!inv32 && !op->bottom_inv64 && op->alloc(&op->bottom_inv64, n2) != AGB_OK)) {
-        cudaGetLastError();
+    if ((!op->bottom_A && !op->try_alloc(&op->bottom_A, n2)) ||
+        (!op->bottom_iwork && nw && !op->try_alloc(&op->bottom_iwork, nw + 1)) ||
+        (!op->bottom_inv_ok && !op->try_alloc(&op->bottom_inv_ok, 1)) ||
+        (inv32 && !op->bottom_inv32 && !op->try_alloc(&op->bottom_inv32, n2)) ||
+        (!inv32 && !op->bottom_inv64 && !op->try_alloc(&op->bottom_inv64, n2)))
         return AGB_OK;
-    }
     if (!dense) launch_bottom_assemble(op->st, op->sym, bl.L, op->bc, op->uniform, bl.ddw64, op->bottom_A);
     launch_bottom_invert(op->st, bl.L, op->bottom_A, inv32 ? nullptr : op->bottom_inv64,
                          inv32 ? op->bottom_inv32 : nullptr, op->bottom_iwork, op->bottom_inv_ok);
@@ -716,9 +767,22 @@ template <class Fn> agb_status capture(agb_op op, cudaGraphExec_t* out, Fn fn)
     return AGB_OK;
 }
 
+// Drops the captured cycles of an earlier epoch of the operator.  No graph is
+// running (every replay is followed by a wait).
+void refresh_graphs(agb_solver s)
+{
+    if (s->epoch == s->op->epoch) return;
+    for (cudaGraphExec_t* g : {&s->g64, &s->g32, &s->gpre}) {
+        if (*g) cudaGraphExecDestroy(*g);
+        *g = nullptr;
+    }
+    s->epoch = s->op->epoch;
+}
+
 agb_status run_iter64(agb_solver s, int iter)
 {
     agb_op op = s->op;
+    refresh_graphs(s);
     const bool fc = iter < s->p.max_fmg_iter;
     if (s->p.use_graph) {
         // F-cycle and V-cycle iterations have different kernel sequences; the
@@ -746,6 +810,7 @@ agb_status run_iter64(agb_solver s, int iter)
 agb_status run_iter32(agb_solver s, int iter)
 {
     agb_op op = s->op;
+    refresh_graphs(s);
     const bool fc = iter < s->p.max_fmg_iter;
     if (s->p.use_graph) {
         if (s->g32 && s->g32_fcycle != (int)fc) {
@@ -856,6 +921,7 @@ void precond32_body(agb_solver s)
 agb_status run_precond32(agb_solver s)
 {
     agb_op op = s->op;
+    refresh_graphs(s);
     if (!s->p.use_graph) {
         precond32_body(s);
         CK(cudaGetLastError());
@@ -947,7 +1013,9 @@ agb_status inner_gcr32(agb_solver s, double inner_tol, double* inorm_out, int* c
             if (k == m) k = 0;
             float* zl = s->kZ[k];
             float* wl = s->kW[k];
-            TRY(learned_direction(s->net, st, op->sym, L, s->kr, v0.ddw32, zl));
+            agb_status ls = learned_direction(s->net, st, op->sym, L, s->kr, v0.ddw32, zl);
+            if (ls == AGB_NOMEM && op->give_back_div()) ls = learned_direction(s->net, st, op->sym, L, s->kr, v0.ddw32, zl);
+            TRY(ls);
             launch_stencil<float>(st, op->sym, MODE_APPLY, L, op->bc, op->uniform, v0.ddw32, v0.div32, zl, nullptr, nullptr, wl,
                                   0.0f, nullptr);
             CK(cudaMemsetAsync(s->kdots, 0, sizeof(double) * (GCR_MAX + 4), st));
@@ -1120,6 +1188,8 @@ agb_status agb_op_create(const int n_cells[3], const double dx[3], const int per
         op->dx[d] = dx[d];
     }
     memset(&op->bc, 0, sizeof(op->bc));
+    if (const char* e = getenv("AGB_DIV")) op->use_div = e[0] != '0';
+    if (const char* e = getenv("AGB_OP_BYTES_MAX")) op->held_max = (size_t)strtoull(e, nullptr, 10);
     auto bail = [&](agb_status s) {
         agb_op_destroy(op);
         return s;
@@ -1183,7 +1253,7 @@ agb_status agb_op_destroy(agb_op op)
 {
     if (!op) return AGB_OK;
     if (op->st) cudaStreamSynchronize(op->st);
-    for (void* p : op->allocs) cudaFree(p);
+    for (auto& a : op->allocs) cudaFree(a.first);
     if (op->dma) cudaFree(op->dma);
     if (op->h_slots) cudaFreeHost(op->h_slots);
     if (op->e0) cudaEventDestroy(op->e0);
@@ -1223,7 +1293,10 @@ agb_status agb_op_set_model(agb_op op, const double* ddw, int layout, int mem)
 agb_status agb_op_set_uniform(agb_op op, int uniform)
 {
     if (!op) return fail(AGB_BADARG, "null operator");
+    if (op->uniform == (uniform != 0)) return AGB_OK;
     op->uniform = uniform != 0;
+    op->prepared = op->f32_ready = false;   // the divergence fields are made for moduli that are not uniform
+    op->epoch++;                            // and the captured cycles hold the flag
     return AGB_OK;
 }
 
@@ -1555,8 +1628,7 @@ static void release(agb_op op, void* p)
 {
     if (!p) return;
     cudaStreamSynchronize(op->st);
-    cudaFree(p);
-    op->allocs.erase(std::remove(op->allocs.begin(), op->allocs.end(), p), op->allocs.end());
+    op->drop(p);
 }
 
 agb_status agb_newton_rhs(agb_op op, const double* F0, const double* u, const double* b, double* rhs, int mem)

@@ -253,11 +253,13 @@ static agb_status ensure_workspace(agb_learned net, const int g0[3])
     for (int a = 0; a < NA; a++)
         if (cudaMalloc(&net->act[a], act_elems(g0, a) * sizeof(__nv_bfloat16)) != cudaSuccess) {
             net->release();
+            cudaGetLastError();
             return AGB_NOMEM;
         }
     const size_t V = (size_t)g0[0] * g0[1] * g0[2];
     if (cudaMalloc(&net->out, V * FEAT * sizeof(float)) != cudaSuccess) {
         net->release();
+        cudaGetLastError();
         return AGB_NOMEM;
     }
     for (int d = 0; d < 3; d++) net->g0[d] = g0[d];
