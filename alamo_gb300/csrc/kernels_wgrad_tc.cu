@@ -12,7 +12,10 @@
 // line y-1 of x on, the lines y-1, y and y+1 (all three dy taps) of a block of
 // CB input channels, the N side the line y of CO output channels, and the
 // three dx taps are three MMAs whose M operand starts one voxel (16 bytes)
-// further.  Rows of the 128 beyond 3 CB are whatever follows in shared memory;
+// further.  A line that ends inside its last 16 voxels is filled up with zeros:
+// behind it for the taps 0 and +1, before it for the tap -1 (both operands start
+// `pad` voxels earlier), so that dy's zeros meet zeros of x and a NaN or infinity
+// in x reaches the taps that use it only.  Rows of the 128 beyond 3 CB are whatever follows in shared memory;
 // they are never read back.  CTAs are (dz, channel blocks, run of batches); the
 // accumulators are read out, added in FP32 registers and started again after
 // every batch: tensor cores do not round their FP32 sums to nearest, and a
@@ -29,9 +32,11 @@
 //
 // What bounds it: issuing the copies (33 a thread and batch of four 80-voxel
 // lines, 2500 clocks) beside the MMAs (60 a batch, 2900 clocks).  65^3 voxels, 32
-// x 32 channels: 61 us; with TMA boxes and MMAs issued from one thread's branch
-// 82 us; the scalar kernel below 3080 us.  The bias gradient reads 8 channels
-// a thread: 7 against 21 us.
+// x 32 channels: 63.5 us (60.7 with the zeros of all taps behind the line: the
+// shifted dy operand of the tap -1 starts inside a core matrix); 64^3, which has
+// none, 51; with TMA boxes and MMAs issued from one thread's branch 82 us at 65^3;
+// the scalar kernel below 3080 us.  The bias gradient reads 8 channels a thread:
+// 7 against 21 us.
 //
 // The scalar kernel stays for slices and pointers that are not 16-byte aligned.
 #include <cuda_bf16.h>
@@ -62,6 +67,7 @@ struct WtArgs {
     int x_cs, dy_cs;
     int cin, cout;
     int T, chunks, stages;     // lines of a batch, CTAs along the batches, stages of shared memory (2 to 4)
+    int lead;                  // voxels of zeros before each line: 16 where lines end inside their last 16
     float* dw;
     int* err;
 };
@@ -69,16 +75,16 @@ struct WtArgs {
 // Bytes from one 8-channel group of a line to the next.  The copying threads
 // write the groups of a voxel side by side; the odd multiples of 32 (16 for 8
 // groups) bytes put them in different banks.
-__host__ __device__ inline int x_pitch(int kx) { return (kx + 2) * 16; }
-__host__ __device__ inline int dy_pitch(int kx, int co) { return kx * 16 + (co == 64 ? 16 : 32); }
-__host__ __device__ inline int stage_bytes(int kx, int cb, int co, int T)
+__host__ __device__ inline int x_pitch(int kx, int lead) { return (lead + kx + 2) * 16; }
+__host__ __device__ inline int dy_pitch(int kx, int lead, int co) { return (lead + kx) * 16 + (co == 64 ? 16 : 32); }
+__host__ __device__ inline int stage_bytes(int kx, int lead, int cb, int co, int T)
 {
-    return (T + 2) * (cb / 8) * x_pitch(kx) + T * (co / 8) * dy_pitch(kx, co);
+    return (T + 2) * (cb / 8) * x_pitch(kx, lead) + T * (co / 8) * dy_pitch(kx, lead, co);
 }
 // the 16 M groups of the last line reach past the x lines: room behind the stages
-__host__ __device__ inline int smem_bytes(int kx, int cb, int co, int T, int stages)
+__host__ __device__ inline int smem_bytes(int kx, int lead, int cb, int co, int T, int stages)
 {
-    return 128 + stages * stage_bytes(kx, cb, co, T) + 16 * x_pitch(kx) + 128;
+    return 128 + stages * stage_bytes(kx, lead, cb, co, T) + 16 * x_pitch(kx, lead) + 128;
 }
 
 // `lines` lines from (x0, y0, z) of GROUPS x 8 channels into dst, `len` voxels each
@@ -120,8 +126,8 @@ __global__ void __launch_bounds__(WtThreads<CO>::all, 1) k_wgrad_tc(WtArgs a)
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t full = smem_u32(&bars[0]), done = smem_u32(&bars[4]), accfree = smem_u32(&bars[8]);
     const int NS = a.stages;
-    const int xp = x_pitch(a.kx), dp = dy_pitch(a.kx, CO);
-    const int xbytes = (a.T + 2) * (CB / 8) * xp, stage = stage_bytes(a.kx, CB, CO, a.T);
+    const int xp = x_pitch(a.kx, a.lead), dp = dy_pitch(a.kx, a.lead, CO);
+    const int xbytes = (a.T + 2) * (CB / 8) * xp, stage = stage_bytes(a.kx, a.lead, CB, CO, a.T);
     const int dz = blockIdx.y;
     const int nci = a.cin / CB;
     const int ci0 = (blockIdx.z % nci) * CB, co0 = (blockIdx.z / nci) * CO;
@@ -146,6 +152,15 @@ __global__ void __launch_bounds__(WtThreads<CO>::all, 1) k_wgrad_tc(WtArgs a)
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         bad = 0;
     }
+    // the zeros before the lines: written once, the copies leave them alone
+    const int xlines = (a.T + 2) * (CB / 8), lines_all = xlines + a.T * (CO / 8);
+    if (a.lead)
+        for (int s = 0; s < NS; s++)
+            for (int l = tid >> 4; l < lines_all; l += WtThreads<CO>::all / 16) {
+                unsigned char* line = sm + s * stage + (l < xlines ? l * xp : xbytes + (l - xlines) * dp);
+                *reinterpret_cast<uint4*>(line + 16 * (tid & 15)) = make_uint4(0, 0, 0, 0);
+            }
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     umma_fence_before();
     __syncthreads();
     umma_fence_after();
@@ -167,7 +182,7 @@ __global__ void __launch_bounds__(WtThreads<CO>::all, 1) k_wgrad_tc(WtArgs a)
                 ok = false;
                 break;
             }
-            const uint32_t dst = smem_u32(sm + s * stage);
+            const uint32_t dst = smem_u32(sm + s * stage) + 16 * a.lead;
             copy_lines<CB / 8, COPY>(dst, xp, a.T + 2, a.kx + 2, a.x + ci0, a.x_cs, x0 - 1, y0 - 1, z + dz - 1, a, t);
             copy_lines<CO / 8, COPY>(dst + xbytes, dp, a.T, a.kx, a.dy + co0, a.dy_cs, x0, y0, z, a, t);
             // the thread's arrival, once its copies so far have landed
@@ -189,16 +204,19 @@ __global__ void __launch_bounds__(WtThreads<CO>::all, 1) k_wgrad_tc(WtArgs a)
             // the copies were generic writes; the MMAs read through the async proxy
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             umma_fence_after();
-            const uint32_t xs = smem_u32(sm) + s * stage, d = tmem + (uint32_t)((n & 1) * COLS);
+            const uint32_t xs = smem_u32(sm) + s * stage + 16 * a.lead, d = tmem + (uint32_t)((n & 1) * COLS);
             const uint64_t ax = umma_desc(xs, 128, xp), bd = umma_desc(xs + xbytes, 128, dp);
             const int lines = min(a.T, a.ny - y0), steps = min(a.kx, (a.nx - x0 + 15) / 16 * 16) / 16;
+            const int pad = max(16 * steps - (a.nx - x0), 0);
+            const uint64_t ap = umma_advance(ax, -pad), bp = umma_advance(bd, -pad);
             uint32_t more = 0;   // the first step of a batch starts the accumulators
             for (int l = 0; l < lines; l++)
 #pragma unroll 2
                 for (int k = 0; k < steps; k++) {
                     const uint64_t ak = umma_advance(ax, l * la + 16 * k), bk = umma_advance(bd, l * lb + 16 * k);
+                    umma_bf16(d, umma_advance(ap, l * la + 16 * k), umma_advance(bp, l * lb + 16 * k), idesc, more);
 #pragma unroll
-                    for (int dx = 0; dx < 3; dx++)
+                    for (int dx = 1; dx < 3; dx++)
                         umma_bf16(d + (uint32_t)(dx * CO), umma_advance(ak, dx), bk, idesc, more);
                     more = 1;
                 }
@@ -363,15 +381,16 @@ bool launch_wt(cudaStream_t st, WtArgs a)
                                                   WT_SMEM) == cudaSuccess;
     if (!attr) return false;
     a.T = 4;
-    while (a.T > 1 && smem_bytes(a.kx, CB, CO, a.T, 2) > WT_SMEM) a.T--;
+    a.lead = a.nx % 16 ? 16 : 0;
+    while (a.T > 1 && smem_bytes(a.kx, a.lead, CB, CO, a.T, 2) > WT_SMEM) a.T--;
     a.stages = 4;
-    while (a.stages > 2 && smem_bytes(a.kx, CB, CO, a.T, a.stages) > WT_SMEM) a.stages--;
+    while (a.stages > 2 && smem_bytes(a.kx, a.lead, CB, CO, a.T, a.stages) > WT_SMEM) a.stages--;
     const int blocks = 3 * (a.cin / CB) * (a.cout / CO);
     const long long total = (long long)a.nz * ((a.ny + a.T - 1) / a.T) * a.ntx;
     // one CTA a SM over all channel blocks and dz
     a.chunks = (int)std::min<long long>(std::max(1, sm_count() / blocks), total);
     k_wgrad_tc<CB, CO><<<dim3(a.chunks, 3, (a.cin / CB) * (a.cout / CO)), WtThreads<CO>::all,
-                         smem_bytes(a.kx, CB, CO, a.T, a.stages), st>>>(a);
+                         smem_bytes(a.kx, a.lead, CB, CO, a.T, a.stages), st>>>(a);
     return true;
 }
 
