@@ -41,6 +41,15 @@ def _i3(g):
     return (ctypes.c_int * 3)(*[int(v) for v in g])
 
 
+def check_waits():
+    """Raises AgbError if a bounded wait of a convolution or weight gradient ran
+    out since the last call: its output, or its part of a gradient, is missing."""
+    flag = ctypes.c_int()
+    check(lib().agb_conv3_tc_error(ctypes.byref(flag)))
+    if flag.value:
+        raise _lib.AgbError(_lib.AGB_CUDA, "a wait of a tensor-core convolution or weight gradient ran out")
+
+
 def topology():
     L = lib()
     nl, na = 11, 13
@@ -340,7 +349,8 @@ def cosine_loss(out, target):
 
 def train(net, samples, n, steps=1000, lr=1e-3, warmup=50, log=None):
     """Adam on the cosine loss, one sample per step (cycling), the learning
-    rate ramped up over the first `warmup` steps.  Returns the loss history."""
+    rate ramped up over the first `warmup` steps.  Returns the loss history;
+    raises AgbError once a step's kernels have not finished (check_waits)."""
     g0 = (n + 1,) * 3
     hist = []
     for it in range(steps):
@@ -348,10 +358,12 @@ def train(net, samples, n, steps=1000, lr=1e-3, warmup=50, log=None):
         out = net.forward(g0, smp["feat"])
         loss, dout = cosine_loss(out, smp["target"])
         hist.append(loss)
+        check_waits()   # the loss was read: everything before it has run
         gw, gb = net.backward(g0, dout)
         net.adam(gw, gb, lr=lr * min(1.0, (it + 1) / float(warmup)))
         if log and (it + 1) % max(1, steps // 5) == 0:
             log("step %d: mean loss over the last %d steps %.4f" % (it + 1, min(it + 1, 50), float(np.mean(hist[-50:]))))
+    check_waits()
     return hist
 
 
@@ -494,6 +506,7 @@ def train_gain(net, problems, n, steps=600, lr=1e-3, warmup=50, log=None):
         gain = a * a / ((y * y * W).sum() * (rp * rp * W).sum())
         (1.0 - gain).backward()
         hist.append(float(gain.detach()))
+        check_waits()
         gaz = az.grad if az.grad is not None else torch.zeros_like(az)
         gz = p["At"] @ torch.nan_to_num(gaz)
         dout = torch.zeros(V, FEAT, dtype=torch.float32, device="cuda")
@@ -502,4 +515,5 @@ def train_gain(net, problems, n, steps=600, lr=1e-3, warmup=50, log=None):
         net.adam(gw, gb, lr=lr * min(1.0, (step + 1) / float(warmup)))
         if log and (step + 1) % max(1, steps // 10) == 0:
             log("step %d: mean gain over the last 50 steps %.4f" % (step + 1, float(np.mean(hist[-50:]))))
+    check_waits()
     return hist

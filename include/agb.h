@@ -285,8 +285,11 @@ agb_status agb_gen_sphere(const int n_cells[3], double radius, double lam_m, dou
  * elements: rows w_co0 .. w_co0 + cout of a [27][w_cout][cin] array, so a wide
  * layer runs as several convolutions); bias (FP32, cout) may be NULL; out FP32 when out_f32; ReLU when
  * relu.  Device pointers, 16-byte aligned; queued on `stream`.
- * agb_conv3_tc_error reports (and clears) a bounded wait of the kernel that
- * ran out since the last call. */
+ * A bounded wait (about 1 s) of this kernel or of agb_conv3_wgrad0's that runs
+ * out sets a flag, although the call returned AGB_OK: the convolution's output is
+ * then incomplete, and the weight gradient lacks the parts of the blocks that
+ * stopped.  agb_conv3_tc_error reports (and clears) it, after everything queued on
+ * the device's streams that it should cover has been waited for. */
 agb_status agb_conv3_tc_pack(int cin, int cout, const void* w, int w_cout, int w_co0, void* wp, void* stream);
 agb_status agb_conv3_tc(const int n[3], int cin, int cout, const void* in, int in_cs, int in_c0, const void* wp,
                         const float* bias, void* out, int out_cs, int out_c0, int out_f32, int relu, void* stream);
@@ -338,6 +341,7 @@ agb_status agb_solver_learned_stats(agb_solver s, int* tried, int* kept, int* ac
  * buffers with channel stride cs; device pointers, queued on `stream`.
  *   wgrad0: dw[tap][co][ci] += sum_v dy[v][co] x[v + off(tap)][ci], zero
  *     padding (FP32, accumulated); db[co] += sum_v dy[v][co] (db may be NULL).
+ *     A wait that runs out is reported by agb_conv3_tc_error.
  *   flip: wt[26 - tap][ci][co] = w[tap][co][ci]; the data gradient of a layer
  *     is the forward convolution of dy with wt.
  *   grid_prolong: fine = beta fine + s P coarse (trilinear, fine = 2 (coarse
