@@ -72,7 +72,7 @@ struct Level {
     float *cor32 = nullptr, *res32 = nullptr, *rescor32 = nullptr, *hold32 = nullptr, *tmp32 = nullptr;
 };
 
-bool g_attr_done = false;
+DeviceOnce g_attributes;
 
 }  // namespace
 
@@ -91,14 +91,18 @@ bool pdl_enabled()
     }();
     return v;
 }
+int current_device()
+{
+    int dev = -1;
+    if (cudaGetDevice(&dev) == cudaSuccess) return dev;
+    cudaGetLastError();
+    return -1;
+}
 int sm_count()
 {
-    static int cache[64] = {0};
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) {
-        cudaGetLastError();
-        return 1;
-    }
+    static int cache[MAX_DEVICES] = {0};
+    const int dev = current_device();
+    if (dev < 0 || dev >= MAX_DEVICES) return 1;
     int v = __atomic_load_n(&cache[dev], __ATOMIC_RELAXED);
     if (v > 0) return v;
     if (cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || v < 1) {
@@ -1198,12 +1202,12 @@ agb_status agb_op_create(const int n_cells[3], const double dx[3], const int per
         return bail(fail(AGB_CUDA, "cudaStreamCreate failed"));
     cudaEventCreate(&op->e0);
     cudaEventCreate(&op->e1);
-    if (!g_attr_done) {
+    g_attributes.run(current_device(), [] {
         init_kernel_attributes();
         init_bottom_attributes();
         init_tma_attributes();
-        g_attr_done = true;
-    }
+        return true;
+    });
     int dev = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&op->pageable_ok, cudaDevAttrPageableMemoryAccess, dev);

@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 
 #include "agb.h"
+#include "device_once.h"
 
 // Truncated unit normals of BC/Operator/Elastic/Elastic.H:79-80 (kept as the
 // reference writes them: the edge/corner traction rows depend on these digits).
@@ -79,6 +80,18 @@ inline void count_launch() { ++launch_counter(); }
 // Streaming multiprocessors of the current device (queried once per device;
 // 1 if the query fails, which only shrinks grid-stride grids).
 int sm_count();
+// The current device (-1 without one).
+int current_device();
+// Allows `kernel` `bytes` of dynamic shared memory on the current device (asked
+// once a device); false, without a pending error, if it cannot have them.
+template <typename... Args> inline bool allow_smem(DeviceOnce& once, void (*kernel)(Args...), int bytes)
+{
+    return once.run(current_device(), [&] {
+        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess) return true;
+        cudaGetLastError();   // the caller's fallback must not find it
+        return false;
+    });
+}
 // Sets the thread-local message agb_last_error() returns.
 void set_error(const char* msg);
 

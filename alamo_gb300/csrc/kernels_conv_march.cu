@@ -273,9 +273,8 @@ __global__ void __launch_bounds__(MC_THREADS, 1) k_conv3_march(McArgs a)
 
 template <int CO> bool launch_march(cudaStream_t st, const McArgs& a, int smem)
 {
-    static const bool attr = cudaFuncSetAttribute(k_conv3_march<CO>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                  MC_SMEM) == cudaSuccess;
-    if (!attr) return false;
+    static DeviceOnce once;
+    if (!allow_smem(once, k_conv3_march<CO>, MC_SMEM)) return false;
     const int tiles = (a.ny * a.px + a.mt * 128 - 1) / (a.mt * 128);
     k_conv3_march<CO><<<dim3(tiles, (a.nz + a.zc - 1) / a.zc, a.cout / CO), MC_THREADS, smem, st>>>(a);
     return true;

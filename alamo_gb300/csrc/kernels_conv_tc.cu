@@ -266,15 +266,16 @@ void init_conv_tc_attributes()
     tc_attr<64>();
 }
 
-// Device address of the error flag of the tensor-core kernels (null without one).
+// Address of the current device's error flag of the tensor-core kernels (null without one).
 int* conv_tc_error_address()
 {
-    static int* err = [] {
+    static DevicePointer<int> err;
+    return err.get(current_device(), [] {
         int* p = nullptr;
-        if (cudaGetSymbolAddress((void**)&p, g_tc_error) != cudaSuccess) p = nullptr;
-        return p;
-    }();
-    return err;
+        if (cudaGetSymbolAddress((void**)&p, g_tc_error) == cudaSuccess) return p;
+        cudaGetLastError();
+        return (int*)nullptr;
+    });
 }
 
 // Reads and clears the error flag the tensor-core convolution sets when a
@@ -331,11 +332,11 @@ extern "C" agb_status agb_conv3_tc(const int n[3], int cin, int cout, const void
         return AGB_BADARG;
     }
     int* err = conv_tc_error_address();
-    static bool attr = [] {
+    static DeviceOnce attributes;
+    attributes.run(current_device(), [] {
         init_conv_tc_attributes();
         return true;
-    }();
-    (void)attr;
+    });
     if (err && launch_conv3_march((cudaStream_t)stream, n, cin, cout, in, in_cs, in_c0, wp, bias, out, out_cs, out_c0,
                                   out_f32, relu, err)) {
         count_launch();

@@ -377,9 +377,8 @@ constexpr int WT_SMEM = 220 * 1024;
 template <int CB, int CO>
 bool launch_wt(cudaStream_t st, WtArgs a)
 {
-    static const bool attr = cudaFuncSetAttribute(k_wgrad_tc<CB, CO>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                  WT_SMEM) == cudaSuccess;
-    if (!attr) return false;
+    static DeviceOnce once;
+    if (!allow_smem(once, k_wgrad_tc<CB, CO>, WT_SMEM)) return false;
     a.T = 4;
     a.lead = a.nx % 16 ? 16 : 0;
     while (a.T > 1 && smem_bytes(a.kx, a.lead, CB, CO, a.T, 2) > WT_SMEM) a.T--;
