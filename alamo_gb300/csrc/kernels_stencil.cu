@@ -106,13 +106,13 @@ __device__ __forceinline__ void epilogue(const T f[3], const T* __restrict__ x, 
 }
 
 // ---------------------------------------------------------------------------
-// one thread per node
+// one thread per node: general moduli without their divergence
 // ---------------------------------------------------------------------------
-template <typename T, int SYM, int MODE>
-__global__ void __launch_bounds__(256) k_stencil_node(LevelDesc L, BCTable bc, Geo<T> g, int uniform,
-                                                      const T* __restrict__ ddw, const T* __restrict__ x,
-                                                      const T* __restrict__ b, const T* __restrict__ dinv,
-                                                      T* __restrict__ out, T omega, void* norm_slot)
+template <typename T, int MODE>
+__global__ void __launch_bounds__(256) k_stencil_node(LevelDesc L, BCTable bc, Geo<T> g, const T* __restrict__ ddw,
+                                                      const T* __restrict__ x, const T* __restrict__ b,
+                                                      const T* __restrict__ dinv, T* __restrict__ out, T omega,
+                                                      void* norm_slot)
 {
     pdl_entry();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -131,8 +131,8 @@ __global__ void __launch_bounds__(256) k_stencil_node(LevelDesc L, BCTable bc, G
         }
         GlobalAcc<T> acc{x, ddw, L.S, make_nbr(L, i, j, k)};
         T f[3];
-        if (bnd) boundary_row<T, SYM>(acc, g, bc, mn, mx, f);
-        else interior_row<T, SYM>(acc, g, uniform != 0, f);
+        if (bnd) boundary_row<T, SYM_MM>(acc, g, bc, mn, mx, f);
+        else interior_row<T, SYM_MM>(acc, g, false, f);
         epilogue<T, MODE>(f, x, b, dinv, out, L.S, acc.nb.base, omega, nrm);
     }
     if (MODE == MODE_RESID && norm_slot) block_max_to_slot<T>(nrm, norm_slot);
@@ -764,13 +764,15 @@ static void stencil_dispatch(cudaStream_t st, const LevelDesc& L, const BCTable&
             return;
         }
     }
-    if (SYM == SYM_MM && !div && !uniform) {
-        dim3 b2(32, 4, 2);
-        if (L.nn[0] <= 40) b2 = dim3(8, 8, 4);   // fewer idle lanes on short rows
-        pdl_launch(k_stencil_node<T, SYM, MODE>, node_grid(L, b2), b2, 0, st, L, bc, g, uniform ? 1 : 0, ddw, x, b,
-                   diag, out, omega, norm_slot);
-        count_launch();
-        return;
+    if constexpr (SYM == SYM_MM) {
+        if (!div && !uniform) {
+            dim3 b2(32, 4, 2);
+            if (L.nn[0] <= 40) b2 = dim3(8, 8, 4);   // fewer idle lanes on short rows
+            pdl_launch(k_stencil_node<T, MODE>, node_grid(L, b2), b2, 0, st, L, bc, g, ddw, x, b, diag, out, omega,
+                       norm_slot);
+            count_launch();
+            return;
+        }
     }
     if (g.cube)
         rows_dispatch<T, SYM, MODE, true>(st, L, bc, g, uniform, ddw, div, x, b, diag, out, omega, norm_slot);

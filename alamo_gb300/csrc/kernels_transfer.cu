@@ -105,29 +105,12 @@ __global__ void k_norm_inf(long long n, const T* __restrict__ x, void* slot)
 }
 
 // Reference nodal box (n+1 nodes per direction) -> padded storage, for the
-// k-planes [k0, k0+kc).  With `chunk`, src holds only those planes (a staging
-// slab); otherwise src is the whole box.
-template <typename TD, typename TS>
-__global__ void k_import(LevelDesc L, int ncomp, const TS* __restrict__ src, TD* __restrict__ dst, int aos, int k0,
-                         int kc, int chunk)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = blockIdx.y * blockDim.y + threadIdx.y;
-    const int k = k0 + blockIdx.z * blockDim.z + threadIdx.z;
-    if (i >= L.nn[0] || j >= L.nn[1] || k >= L.nn[2] || k >= k0 + kc) return;
-    const long long planeN = (long long)(L.n[0] + 1) * (L.n[1] + 1);
-    const long long Nsrc = chunk ? planeN * kc : planeN * (L.n[2] + 1);
-    const long long s = (long long)i + (long long)(L.n[0] + 1) * j + planeN * (chunk ? k - k0 : k);
-    const long long q = L.idx(i, j, k);
-    for (int c = 0; c < ncomp; c++) dst[c * L.S + q] = (TD)(aos ? src[s * ncomp + c] : src[c * Nsrc + s]);
-}
-
-// The same for component planes (SoA) on both sides: a warp copies one row of
-// one component, COPY_UNROLL elements a lane in flight at once; bound by HBM.  The
-// node-per-thread kernel has three loads in flight and leaves the last warp of
-// a row of 2^k + 1 nodes nearly empty: 192 x 160 x 144
-// cells in FP32 (109 MB moved) 33 us against 16 in and 21 out; two sweeps through the
-// public call 431 against 389 us.
+// k-planes [k0, k0+nk).  With `chunk`, src holds only those planes (a staging
+// slab); otherwise src is the whole box.  Component planes (SoA): a warp copies one row of
+// one component, COPY_UNROLL elements a lane in flight at once; bound by HBM.  A
+// thread for each node has three loads in flight and leaves the last warp of a row
+// of 2^k + 1 nodes nearly empty: 192 x 160 x 144 cells in FP32 (109 MB moved) 33 us
+// against 16 in and 21 out; two sweeps through the public call 431 against 389 us.
 constexpr int COPY_UNROLL = 8;
 template <typename TD, typename TS>
 __global__ void __launch_bounds__(256) k_import_rows(LevelDesc L, long long rows, const TS* __restrict__ src,
@@ -207,27 +190,22 @@ __global__ void __launch_bounds__(256) k_import_aos(LevelDesc L, int ncomp, cons
     }
 }
 
-// padded storage -> reference nodal box for planes [k0, k0+kc) (periodic images filled)
+// and back to interleaved fields, periodic images filled
 template <typename TD, typename TS>
-__global__ void k_export(LevelDesc L, int ncomp, const TS* __restrict__ src, TD* __restrict__ dst, int aos, int k0,
-                         int kc, int chunk)
+__global__ void k_export_aos(LevelDesc L, int ncomp, const TS* __restrict__ src, TD* __restrict__ dst, int k0, int kc,
+                             int chunk)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y * blockDim.y + threadIdx.y;
     const int k = k0 + blockIdx.z * blockDim.z + threadIdx.z;
     if (i > L.n[0] || j > L.n[1] || k > L.n[2] || k >= k0 + kc) return;
     const long long planeN = (long long)(L.n[0] + 1) * (L.n[1] + 1);
-    const long long Ndst = chunk ? planeN * kc : planeN * (L.n[2] + 1);
     const long long s = (long long)i + (long long)(L.n[0] + 1) * j + planeN * (chunk ? k - k0 : k);
     const int ii = (L.per[0] && i == L.n[0]) ? 0 : i;
     const int jj = (L.per[1] && j == L.n[1]) ? 0 : j;
     const int kk = (L.per[2] && k == L.n[2]) ? 0 : k;
     const long long q = L.idx(ii, jj, kk);
-    for (int c = 0; c < ncomp; c++) {
-        const TD v = (TD)src[c * L.S + q];
-        if (aos) dst[s * ncomp + c] = v;
-        else dst[c * Ndst + s] = v;
-    }
+    for (int c = 0; c < ncomp; c++) dst[s * ncomp + c] = (TD)src[c * L.S + q];
 }
 
 // The first damped-Jacobi sweep from x = 0: A 0 = 0 in every row (interior,
@@ -391,27 +369,19 @@ template <typename TD, typename TS>
 void launch_import(cudaStream_t st, const LevelDesc& L, int ncomp, const TS* src, TD* dst, bool aos, int k0, int kc,
                    bool chunk)
 {
-    if (aos && ncomp > 1 && ncomp <= 21) {
-        const dim3 blk(32, 8);
-        const long long rows = (long long)L.nn[1] * std::min(kc, L.nn[2] - k0);
+    const int nk = std::min(kc, L.nn[2] - k0);
+    if (nk <= 0 || ncomp <= 0) return;
+    const long long rows = (long long)nk * L.nn[1];
+    if (aos && ncomp > 1) {   // 21 components at most: 43 KB of shared memory
         const dim3 grd((L.nn[0] + 31) / 32, (unsigned)((rows + 7) / 8));
         const size_t smem = 8 * 32 * (size_t)ncomp * sizeof(TS);
-        k_import_aos<TD, TS><<<grd, blk, smem, st>>>(L, ncomp, src, dst, k0, kc, chunk ? 1 : 0);
-        count_launch();
-        return;
-    }
-    if (!aos || ncomp == 1) {
-        const int nk = std::min(kc, L.nn[2] - k0);
-        if (nk <= 0 || ncomp <= 0) return;
-        const long long rows = (long long)ncomp * nk * L.nn[1];
+        k_import_aos<TD, TS><<<grd, dim3(32, 8), smem, st>>>(L, ncomp, src, dst, k0, kc, chunk ? 1 : 0);
+    } else {
         const long long Nsrc = (long long)(L.n[0] + 1) * (L.n[1] + 1) * (chunk ? kc : L.n[2] + 1);
-        k_import_rows<TD, TS><<<(unsigned)((rows + 7) / 8), 256, 0, st>>>(L, rows, src, dst, k0, nk, Nsrc, chunk ? 1 : 0);
-        count_launch();
-        return;
+        k_import_rows<TD, TS><<<(unsigned)((rows * ncomp + 7) / 8), 256, 0, st>>>(L, rows * ncomp, src, dst, k0, nk, Nsrc,
+                                                                                  chunk ? 1 : 0);
     }
-    dim3 blk(32, 4, 2);
-    dim3 grd((L.nn[0] + blk.x - 1) / blk.x, (L.nn[1] + blk.y - 1) / blk.y, (kc + blk.z - 1) / blk.z);
-    k_import<TD, TS><<<grd, blk, 0, st>>>(L, ncomp, src, dst, aos ? 1 : 0, k0, kc, chunk ? 1 : 0); count_launch();
+    count_launch();
 }
 
 template <typename TD, typename TS>
@@ -429,7 +399,7 @@ void launch_export(cudaStream_t st, const LevelDesc& L, int ncomp, const TS* src
     }
     dim3 blk(32, 4, 2);
     dim3 grd((L.n[0] + 1 + blk.x - 1) / blk.x, (L.n[1] + 1 + blk.y - 1) / blk.y, (kc + blk.z - 1) / blk.z);
-    k_export<TD, TS><<<grd, blk, 0, st>>>(L, ncomp, src, dst, aos ? 1 : 0, k0, kc, chunk ? 1 : 0); count_launch();
+    k_export_aos<TD, TS><<<grd, blk, 0, st>>>(L, ncomp, src, dst, k0, kc, chunk ? 1 : 0); count_launch();
 }
 
 template <typename T>
