@@ -167,6 +167,7 @@ __global__ void __launch_bounds__(MC_THREADS, 1) k_conv3_march(McArgs a)
         constexpr uint32_t idesc = umma_idesc_bf16(128, 3 * CO, false);
         const uint64_t wd = umma_desc(sw, 5 * CO * 16, 128);
         ok = __all_sync(0xffffffffu, mbar_wait(wbar, 0));
+        if (!ok) mbar_wait(wbar, 0);   // bounded: the weights' copies must not outlive the shared memory
         int u = 0;
         for (int n = 0; n < planes && ok; n++) {
             const int r = (z0 - 1 + n + 3) % 3;
