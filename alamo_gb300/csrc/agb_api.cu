@@ -143,7 +143,8 @@ struct agb_op_s {
     int pageable_ok = 0;         // device can read pageable host memory directly
     // Device memory.  The divergence fields (make_div) only save time, so an
     // allocation that finds no memory takes theirs and they are not made again.
-    // epoch counts what makes captured cycles stale: this, and agb_op_set_uniform.
+    // epoch counts what makes captured cycles stale: this, and other types of
+    // boundary conditions, another uniform flag or omega.
     std::vector<std::pair<void*, size_t>> allocs;
     size_t held = 0, held_max = 0;   // bytes; held_max: most it may hold, 0 = no limit (AGB_OP_BYTES_MAX)
     bool use_div = true;             // AGB_DIV=0: without divergence fields
@@ -171,6 +172,11 @@ struct agb_op_s {
                 allocs.erase(allocs.begin() + i);
                 return;
             }
+    }
+    void set_omega(double w)
+    {
+        if (w != omega) epoch++;
+        omega = w;
     }
     bool give_back_div()
     {
@@ -1270,13 +1276,16 @@ agb_status agb_op_destroy(agb_op op)
 agb_status agb_op_set_bc(agb_op op, const agb_bc* bc)
 {
     if (!op || !bc) return fail(AGB_BADARG, "null argument");
+    bool stale = false;   // the rows of the captured cycles hold the types (not the values)
     for (int f = 0; f < AGB_NFACES; f++)
         for (int c = 0; c < 3; c++) {
             const int t = bc->type[f][c];
             if (t < AGB_BC_DISP || t > AGB_BC_NONE) return fail(AGB_BADARG, "bad BC type %d at face %d comp %d", t, f, c);
+            if (op->bc.type[f][c] != (int8_t)t) stale = true;
             op->bc.type[f][c] = (int8_t)t;
             op->bc.val[f][c] = bc->val[f][c];
         }
+    if (stale) op->epoch++;
     op->bc_set = true;
     op->prepared = false;
     return AGB_OK;
@@ -1308,7 +1317,7 @@ agb_status agb_op_set_omega(agb_op op, double omega)
 {
     if (!op) return fail(AGB_BADARG, "null operator");
     if (!(omega > 0 && omega < 2)) return fail(AGB_BADARG, "omega must be in (0,2)");
-    op->omega = omega;
+    op->set_omega(omega);
     return AGB_OK;
 }
 
@@ -1479,7 +1488,7 @@ agb_status agb_solver_create(agb_op op, const agb_solver_params* params, agb_sol
         delete s;
         return fail(AGB_BADARG, "krylov must be in 0..%d", GCR_MAX);
     }
-    if (s->p.omega > 0) op->omega = s->p.omega;   // Linear::PrepareMLMG -> SetOmega
+    if (s->p.omega > 0) op->set_omega(s->p.omega);   // Linear::PrepareMLMG -> SetOmega
     const size_t n3 = 3 * (size_t)op->lev[0].L.S;
     agb_status st;
     if ((st = op->alloc(&s->x64, n3)) != AGB_OK || (st = op->alloc(&s->b64, n3)) != AGB_OK) {
