@@ -548,7 +548,7 @@ __global__ void __launch_bounds__(256) k_batch_diag(const BProb* __restrict__ pr
 // and divisions in every thread; here one thread makes them once a problem.
 // Bound by HBM.  48 RVEs (17.3 M nodes), finest level, us before and now: GCR
 // step 872 and 175, the sums and the subtraction of the FP32 zero-mean
-// projection 305 and 37, 305 and 75; the solve 160 to 128 ms with the copies
+// projection 305 and 37, 305 and 75; the solve 160 to 124 ms with the copies
 // around the cycle gone.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ void seg_range(const BSegList& list, int& s0, int& s1)

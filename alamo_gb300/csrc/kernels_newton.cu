@@ -90,8 +90,9 @@ __global__ void k_dw(LevelDesc L, Geo<double> g, const double* __restrict__ ddw,
 // (periodic images included) and passes its 9 values a node through shared
 // memory, so the interleaved output is written in whole lines; the moduli are
 // read once, coalesced, and u in place in the caller's layout when it is device
-// memory (U: the strides of u).  Bound by the FP64 pipe, 57 operations a node
-// for the stress and 71 for strain and energy: 518 us together at 129^3 nodes
+// memory (U: the strides of u; the host imports u where an output overlaps it).
+// Bound by the FP64 pipe, 57 operations a node for the stress and 70 for strain
+// and energy: 520 us together at 129^3 nodes
 // with general moduli (430 us of FP64 work; with padded intermediate fields, their
 // export, FP64 divisions and three forms of every difference evaluated, 1690 us
 // besides two allocations a call).

@@ -210,12 +210,12 @@ __global__ void __launch_bounds__(256) k_stencil_shell(LevelDesc L, BCTable bc, 
 // is read once, coalesced, by the thread that uses it, and the displacement's
 // neighbours come through L1.
 //
-// What bounds it: in FP64 the FP64 pipe (two lanes per clock and SM on GB300;
-// 144 operations a node here against 253 with the moduli of the neighbours,
-// and the extra 144 bytes a node of the divergence cost a tenth of that time);
+// What bounds it: in FP64 the FP64 pipe (two lanes per clock and SM on GB300; a
+// Jacobi sweep is 146 operations a node in k_rows and 144 in k_column, counted by
+// ncu, against 262 with the moduli of the neighbours, and the extra 144 bytes a node of the divergence cost a tenth of that time);
 // in FP32, on the levels that fit in L2, latency.  A Jacobi sweep with general
-// moduli went from 10.10 to 4.37 ms at 257^3 nodes in FP64 (0.87 of the FP64
-// peak at 138 operations a node), 338 to 88 us at 65^3, 34.8 to 14.4 us at
+// moduli went from 10.10 to 4.37 ms at 257^3 nodes in FP64 (0.89 of what the
+// pipe issues at 144 operations a node), 338 to 88 us at 65^3, 34.8 to 14.4 us at
 // 33^3, 27.7 to 10.3 us at 9^3; isotropic 671 to 433 us at 129^3; FP32 general
 // moduli 18.4 to 10.3 us at 49^3.
 //
@@ -225,9 +225,9 @@ __global__ void __launch_bounds__(256) k_stencil_shell(LevelDesc L, BCTable bc, 
 //             threads a block, so that the 9^3- to 33^3-node levels spread over all SMs.
 //   k_column  FP64 on large levels: a thread marches up a column, carrying the
 //             x and y differences of three planes in registers, from which the
-//             mixed xz and yz differences cost one subtraction each (132
-//             operations a node) and 27 instead of 57 displacement loads; the
-//             boundary shell is done by the last blocks of the same launch.
+//             mixed xz and yz differences cost one subtraction each and a node
+//             27 instead of 57 displacement loads; the boundary shell is done by
+//             the last blocks of the same launch.
 // ---------------------------------------------------------------------------
 constexpr int ROW_THREADS = 64;
 
